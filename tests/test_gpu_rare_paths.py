@@ -1,0 +1,62 @@
+"""The rare paths and edges of the register-row, tensor-core, triangular-solve and
+emulated-format kernels: pivots that need the exact comparison, divisions outside the
+shared-reciprocal range, zero pivots over columns that are not plain zeros, ragged
+orders, partial passes of right-hand sides, binary16 storage."""
+import numpy as np
+import pytest
+
+from conftest import load_pkg
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+tsdx = load_pkg()
+capi = load_pkg("capi")
+device = load_pkg("device")
+M = load_pkg("matrices")
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def same(a, b):
+    """Bit-identical, NaN where the other has NaN."""
+    iv = {2: np.uint16, 4: np.uint32, 8: np.uint64}[a.dtype.itemsize]
+    a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
+    return bool(((a.view(iv) == b.view(iv)) | (np.isnan(a) & np.isnan(b))).all())
+
+
+def odd_matrices(n, dtype, seed):
+    r = np.random.default_rng(seed)
+    f32 = dtype == np.float32
+    A = r.standard_normal((14, n, n)).astype(dtype)
+    c = n // 2
+    A[0] *= dtype(1e-30 if f32 else 1e-200)                     # pivots below the range
+    A[1] *= dtype(1e33 if f32 else 1e200)                       # and above it
+    A[2, ::2] *= dtype(1e-25 if f32 else 1e-190)                # tiny multipliers
+    A[3, :, c] = -0.0                                           # a zero pivot over -0
+    A[4, :, c] = 0.0
+    A[4, -1, c] = np.nan                                        # and over a NaN
+    A[5, 0, 0] = np.nan
+    A[6, -1, 0] = np.inf
+    A[7] = r.integers(-1, 2, (n, n))                            # ties and zeros
+    A[8] = np.eye(n)[r.permutation(n)]
+    A[9, 0, 0] = np.nextafter(dtype(4), dtype(0))               # an all-ones significand
+    A[10, 0, 0] = -np.nextafter(dtype(4), dtype(0))
+    A[11] = np.where(r.random((n, n)) < 0.6, 0.0, A[11])
+    A[12] = 0.0
+    for i in (9, 10):
+        A[i, 1:, 0] = (r.integers(1, 16, n - 1) / 8.0).astype(dtype)
+    return A
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [2, 4, 7, 8, 16, 21, 24, 29, 32, 40, 45, 48, 61, 64])
+def test_odd_pivots_bit_exact(oracle, n, dtype):
+    A = odd_matrices(n, dtype, 900 + n)
+    LU, piv, info = (t.cpu().numpy() for t in (lambda a: (a, *device.getrf(a)))(dev(A)))
+    LUo, pivo, infoo = oracle.lu(A, "scalar")
+    assert np.array_equal(info, infoo) and np.array_equal(piv, pivo)
+    for i in range(len(A)):
+        assert same(LU[i], LUo[i]), i

@@ -1,33 +1,26 @@
-// Blocked batched LU with partial pivoting (getrf/gesv) and Cholesky (potrf/posv):
-// one G-lane segment per matrix (G = 32 for n > 16; 32/G matrices per warp below),
-// the matrix plus its right-hand sides (appended as columns) in shared memory,
-// factored in panels of PB columns:
-//   1. panel factorization in registers (lane l owns rows l + G*s): LU pivot
-//      search by segment reduction with implicit row swaps, or the Cholesky
-//      diagonal; multipliers; rank-1 update of the panel only;
-//   2. LU: U12, the panel's pivot rows brought up to date on the trailing
-//      columns by a unit-lower triangular solve (one lane per column);
-//      Cholesky: forward substitution of the panel rows' right-hand sides;
-//   3. trailing update A22 -= L21 U12 (Cholesky: the lower triangle, L21 L21^T)
-//      for the rows still active, column chunk by column chunk, from shared memory
-//      with the panel multipliers kept in registers.
+// Shared pieces of the kernels that keep a matrix in shared memory (layout, staging,
+// copies), and the general LU body: one G-lane segment per matrix, the matrix plus its
+// right-hand sides (appended as columns) in shared memory, factored in panels of PB
+// columns:
+//   1. panel factorization in registers (lane l owns rows l + G*s): pivot search by
+//      segment reduction with implicit row swaps, multipliers, rank-1 update of the
+//      panel only;
+//   2. U12, the panel's pivot rows brought up to date on the trailing columns by a
+//      unit-lower triangular solve (one lane per column);
+//   3. trailing update A22 -= L21 U12 for the rows still active, column chunk by column
+//      chunk, from shared memory with the panel multipliers kept in registers.
 // Every element receives exactly the reference's chain of operations, so factors,
-// pivots and info are bit-identical to TinySolverDx's CPU backends:
-//   LU (kernels.hpp:91-119): a_ij <- fma(-l_ik, u_kj, a_ij) in increasing k,
-//     l_ik = a_ik / u_kk correctly rounded, a zero pivot skips the column; ties go
-//     to the first maximum and NaN never wins unless on the diagonal position.
-//   Cholesky as the default simd backend compiles kernels.hpp:57-87: the products
-//     subtracted in increasing k, fused for n <= 16 and separately rounded for
-//     n >= 17 (NP <= 16 <=> n <= 16); a pivot that is not > 0 records info, is
-//     replaced by 1 and the factorization completes; the upper triangle is zeroed.
-// Rows never move: ord[k] records the physical row retired at step k and the
-// factor is written in that order, which is where the reference's full-row swaps
-// leave each row. The forward substitution rides along as extra columns (the
-// reference's chain, kernels.hpp:184-193 / 214-218); the backward substitution is
-// column-oriented with reciprocal diagonals, so X agrees to rounding.
+// pivots and info are bit-identical to TinySolverDx's CPU backends (kernels.hpp:91-119):
+//   a_ij <- fma(-l_ik, u_kj, a_ij) in increasing k, l_ik = a_ik / u_kk correctly rounded,
+//   a zero pivot skips the column; ties go to the first maximum and NaN never wins unless
+//   on the diagonal position.
+// Rows never move: ord[k] records the physical row retired at step k and the factor is
+// written in that order, which is where the reference's full-row swaps leave each row.
+// The forward substitution rides along as extra columns (the reference's chain,
+// kernels.hpp:184-193 / 214-218); the backward substitution is column-oriented with
+// reciprocal diagonals, so X agrees to rounding.
 //
-// The per-matrix body is a device function over a MatJob (base pointers, sizes),
-// shared by the dense-batch kernel below and the uneven-stream kernel.
+// This body covers every input; rows.cuh holds the faster ones and falls back on it.
 #pragma once
 #include "common.cuh"
 
@@ -78,6 +71,7 @@ struct MatJob {
 struct Seg {
   int lane, lsl, segbase;
   unsigned segmask;
+  unsigned zrow;  // shared address of a row of zeros (rows.cuh)
 };
 
 // Widest copy chunk that keeps every row start aligned.
@@ -172,25 +166,23 @@ __device__ __forceinline__ void seg_load(unsigned char* M, const MatJob<T>& j, c
   __syncwarp();
 }
 
-// Column-oriented back substitution with reciprocal diagonals. LU: U(i,k) sits in
-// shared row ord[i]; Cholesky: L^T(i,k) = L(k,i).
-template <class T, int NP, int NRHS, bool CHOL, int GO>
+// Column-oriented back substitution with reciprocal diagonals; U(i,k) sits in shared row
+// ord[i].
+template <class T, int NP, int NRHS, int GO>
 __device__ __forceinline__ void seg_backsolve(unsigned char* M, const int* ord, const MatJob<T>& j, const Seg& g) {
   using C = BlkCfg<T, NP, NRHS, GO>;
   constexpr int G = C::G, MR = C::MR, RS = C::RS;
   auto at = [&](int r, int c) -> T& { return *reinterpret_cast<T*>(M + r * RS + c * int(sizeof(T))); };
   T yv[MR][NRHS], dv[MR];
-  // U(i, k) of this lane's rows at ubase[t] + k * ustride (LU: row ord[i], column k;
-  // Cholesky: row k, column i)
-  const unsigned char* ubase[MR];
-  constexpr int ustride = CHOL ? RS : int(sizeof(T));
+  const unsigned char* ubase[MR];  // this lane's rows of U
+  constexpr int ustride = int(sizeof(T));
 #pragma unroll
   for (int t = 0; t < MR; ++t) {
     const int i = g.lsl + G * t;
     const int ii = i < NP ? i : 0;
-    const int pr = CHOL ? ii : ord[ii];
+    const int pr = ord[ii];
     dv[t] = rcp_(at(pr, ii));
-    ubase[t] = CHOL ? M + ii * int(sizeof(T)) : M + pr * RS;
+    ubase[t] = M + pr * RS;
 #pragma unroll
     for (int c = 0; c < NRHS; ++c) yv[t][c] = at(pr, NP + c);
   }
@@ -409,7 +401,7 @@ __device__ __forceinline__ void lu_matrix(unsigned char* M, const MatJob<T>& j, 
     __syncwarp();
   }
 
-  if constexpr (NRHS > 0) seg_backsolve<T, NP, NRHS, false, GO>(M, ord, j, g);
+  if constexpr (NRHS > 0) seg_backsolve<T, NP, NRHS, GO>(M, ord, j, g);
   if (j.live) {
     if (j.piv) {
 #pragma unroll
@@ -423,233 +415,6 @@ __device__ __forceinline__ void lu_matrix(unsigned char* M, const MatJob<T>& j, 
   __syncwarp();
   if (j.live && j.Aout) seg_copy_out<T, G, RS>(M, j.Aout, j.n, lsl, ord);
   __syncwarp();
-}
-
-// ------------------------------------------------------------------- Cholesky
-template <class T, int NP, int NRHS, int GO>
-__device__ __forceinline__ void chol_matrix(unsigned char* M, const MatJob<T>& j, const Seg& g) {
-  using C = BlkCfg<T, NP, NRHS, GO>;
-  using V = Vec16<T>;
-  using VT = typename V::type;
-  constexpr int G = C::G, MR = C::MR, PB = C::PB, NC = C::NC, CH = C::CH, RS = C::RS;
-  constexpr int VN = V::n, TS = int(sizeof(T));
-  constexpr bool FUSED = NP <= 16;
-  const int lsl = g.lsl, segbase = g.segbase;
-  auto at = [&](int r, int c) -> T& { return *reinterpret_cast<T*>(M + r * RS + c * TS); };
-  auto vat = [&](int r, int c) -> VT& { return *reinterpret_cast<VT*>(M + r * RS + c * TS); };
-  auto sub = [](T s, T x, T y) -> T { return FUSED ? fma_(-x, y, s) : sub_mul(s, x, y); };
-
-  seg_load<T, NP, NRHS, GO>(M, j, g);
-  int info = 0;
-  for (int k0 = 0; k0 < NP; k0 += PB) {
-    T pan[MR][PB];
-#pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lsl + G * s;
-      const int rr = r < NP ? r : 0;
-#pragma unroll
-      for (int i0 = 0; i0 < PB; i0 += VN) {
-        const VT v = vat(rr, k0 + i0);
-#pragma unroll
-        for (int q = 0; q < VN; ++q) pan[s][i0 + q] = V::get(v, q);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < PB; ++i) {
-      const int k = k0 + i;
-      const int dl = segbase + (k & (G - 1)), ds = k / G;
-      T dv = pan[0][i];
-#pragma unroll
-      for (int t = 1; t < MR; ++t) dv = (ds == t) ? pan[t][i] : dv;
-      const T d = __shfl_sync(kFull, dv, dl);
-      const bool bad = !(d > T(0));
-      info = (bad && info == 0) ? k + 1 : info;
-      const T lkk = sqrt_(bad ? T(1) : d);
-      const T ry = rcp_(lkk);
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const int r = lsl + G * s;
-        if (r == k) pan[s][i] = lkk;
-        else if (r > k && r < NP) pan[s][i] = div_by(pan[s][i], lkk, ry);
-      }
-#pragma unroll
-      for (int jj = i + 1; jj < PB; ++jj) {
-        const int rj = k0 + jj;
-        T v = pan[0][i];
-#pragma unroll
-        for (int t = 1; t < MR; ++t) v = ((rj / G) == t) ? pan[t][i] : v;
-        const T lj = __shfl_sync(kFull, v, segbase + (rj & (G - 1)));
-#pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = lsl + G * s;
-          if (r >= rj && r < NP) pan[s][jj] = sub(pan[s][jj], pan[s][i], lj);
-        }
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lsl + G * s;
-      if (r >= NP || r < k0) continue;
-#pragma unroll
-      for (int i0 = 0; i0 < PB; i0 += VN) {
-        VT v;
-#pragma unroll
-        for (int q = 0; q < VN; ++q) V::set(v, q, pan[s][i0 + q]);
-        vat(r, k0 + i0) = v;
-      }
-    }
-    __syncwarp();
-    const int j1 = k0 + PB;
-    if (j1 >= NC) continue;
-    if constexpr (NRHS > 0) {
-      // forward substitution of the panel rows' right-hand sides (fused, then / l_ii)
-      for (int cc = lsl; cc < NRHS; cc += G) {
-        const int c = NP + cc;
-        T y[PB];
-#pragma unroll
-        for (int i = 0; i < PB; ++i) {
-          const int r = k0 + i;
-          T acc = at(r, c);
-#pragma unroll
-          for (int i2 = 0; i2 < i; ++i2) acc = fma_(-at(r, k0 + i2), y[i2], acc);
-          y[i] = div_(acc, at(r, r));
-          at(r, c) = y[i];
-        }
-      }
-      __syncwarp();
-    }
-    for (int jc = j1; jc < NC; jc += CH) {
-      T acc[MR][CH];
-      const bool bcols = jc >= NP;  // NP % CH == 0: a chunk is all-matrix or all-RHS
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const int r = lsl + G * s;
-        const int rr = (r >= j1 && r < NP) ? r : 0;
-#pragma unroll
-        for (int c0 = 0; c0 < CH; c0 += VN) {
-          const VT v = vat(rr, jc + c0);
-#pragma unroll
-          for (int q = 0; q < VN; ++q) acc[s][c0 + q] = V::get(v, q);
-        }
-      }
-      if (!bcols) {
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          const int jcol = jc + c;
-#pragma unroll
-          for (int i0 = 0; i0 < PB; i0 += VN) {
-            const VT v = vat(jcol, k0 + i0);
-#pragma unroll
-            for (int q = 0; q < VN; ++q) {
-              const T lj = V::get(v, q);
-#pragma unroll
-              for (int s = 0; s < MR; ++s) {
-                const int r = lsl + G * s;
-                if (jcol <= r) acc[s][c] = sub(acc[s][c], pan[s][i0 + q], lj);
-              }
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < PB; ++i) {
-          const int pr = k0 + i;
-#pragma unroll
-          for (int c0 = 0; c0 < CH; c0 += VN) {
-            const VT v = vat(pr, jc + c0);
-#pragma unroll
-            for (int q = 0; q < VN; ++q) {
-              const T u = V::get(v, q);
-#pragma unroll
-              for (int s = 0; s < MR; ++s) acc[s][c0 + q] = fma_(-pan[s][i], u, acc[s][c0 + q]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const int r = lsl + G * s;
-        if (r < j1 || r >= NP) continue;
-#pragma unroll
-        for (int c0 = 0; c0 < CH; c0 += VN) {
-          VT v;
-#pragma unroll
-          for (int q = 0; q < VN; ++q) V::set(v, q, acc[s][c0 + q]);
-          vat(r, jc + c0) = v;
-        }
-      }
-    }
-    __syncwarp();
-  }
-
-  if constexpr (NRHS > 0) seg_backsolve<T, NP, NRHS, true, GO>(M, nullptr, j, g);
-  if (j.live && lsl == 0 && j.info) *j.info = info;
-  // no early return: every lane of the warp must reach each __syncwarp
-  const bool out = j.live && j.Aout;
-  __syncwarp();
-  if (out) {
-#pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lsl + G * s;
-      if (r >= NP) continue;
-      for (int c = r + 1; c < j.n; ++c) at(r, c) = T(0);
-    }
-  }
-  __syncwarp();
-  if (out) seg_copy_out<T, G, RS>(M, j.Aout, j.n, lsl, nullptr);
-  __syncwarp();
-}
-
-template <class T, int NP, int NRHS, bool CHOL, int GO = 0>
-__device__ __forceinline__ void blk_matrix(unsigned char* M, const MatJob<T>& j, const Seg& g) {
-  if constexpr (CHOL) chol_matrix<T, NP, NRHS, GO>(M, j, g);
-  else lu_matrix<T, NP, NRHS, GO>(M, j, g);
-}
-
-// Dense batch: one persistent CTA of WPC warps per SM slot; every round each
-// segment takes the next matrix and the CTA walks the code together, so the
-// instruction stream fetched for one warp serves all of them.
-template <class T, int NP, int NRHS, int WPC, bool CHOL, int GO = 0>
-__global__ void __launch_bounds__(WPC * 32, 1) blk_kernel(SolveArgs<T> p) {
-  using C = BlkCfg<T, NP, NRHS, GO>;
-  constexpr int G = C::G, S = C::S;
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Seg g;
-  g.lane = lane;
-  g.lsl = lane & (G - 1);
-  g.segbase = (lane / G) * G;
-  g.segmask = (G == 32) ? kFull : (((1u << G) - 1u) << g.segbase);
-  unsigned char* M = smem + warp * C::WARPB + (lane / G) * C::SEGB;
-  const long long nn = (long long)p.n * p.n;
-  const long long per_round = (long long)gridDim.x * WPC * S;
-  // warps own disjoint shared memory, so they run their rounds without a block barrier
-  for (long long base = (long long)blockIdx.x * WPC * S; base < p.batch; base += per_round) {
-    const long long m = base + (long long)warp * S + lane / G;
-    {
-      // this warp's next unit heads for L2 while this one is solved
-      const long long nxt = base + per_round + (long long)warp * S;
-      if (lane == 0 && nxt < p.batch) {
-        const long long cnt = (p.batch - nxt) < S ? (p.batch - nxt) : S;
-        prefetch_l2(p.A + nxt * nn, cnt * nn * (long long)sizeof(T));
-        if (p.B) prefetch_l2(p.B + nxt * (long long)p.n * p.ldb, cnt * (long long)p.n * p.ldb * (long long)sizeof(T));
-      }
-    }
-    MatJob<T> j;
-    j.live = m < p.batch && !(p.status && p.status[m] >= 0);
-    if (!__any_sync(kFull, j.live)) continue;
-    const long long mm = j.live ? m : 0;
-    j.A = p.A + mm * nn;
-    j.Aout = p.wf ? p.A + mm * nn : nullptr;
-    j.B = p.B ? p.B + mm * (long long)p.n * p.ldb : nullptr;
-    j.piv = (p.piv && p.wf) ? p.piv + mm * p.n : nullptr;
-    j.info = p.info ? p.info + mm : nullptr;
-    j.n = p.n;
-    j.ldb = p.ldb;
-    j.b0 = p.b0;
-    j.nrhs = p.nrhs;
-    blk_matrix<T, NP, NRHS, CHOL, GO>(M, j, g);
-  }
 }
 
 }  // namespace dev

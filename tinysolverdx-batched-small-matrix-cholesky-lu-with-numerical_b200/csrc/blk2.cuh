@@ -217,7 +217,7 @@ __device__ __forceinline__ void lu2_matrix(unsigned char* M, const MatJob<T>& j,
       g0.lsl = lane;
       g0.segbase = 0;
       g0.segmask = kFull;
-      seg_backsolve<T, NP, NRHS, false, 32>(M, ord, j, g0);
+      seg_backsolve<T, NP, NRHS, 32>(M, ord, j, g0);
     }
   } else if (j.live) {
     if (j.piv)

@@ -7,9 +7,9 @@
 #include <cstdint>
 #include <string>
 
-#include "blk.cuh"
-#include "solve.cuh"
 #include "blk3.cuh"
+#include "rows.cuh"
+#include "solve.cuh"
 #include "blk_tc.cuh"
 
 namespace tsdx {
@@ -59,41 +59,45 @@ int grid_for(Kern kern, int smem, long long ctas_needed, int threads = 128) {
 
 template <class Kern>
 int prepare(Kern kern, int smem) {
-  // the attribute is per function and per device; setting it is idempotent
-  if (smem > 48 * 1024) {
+  // the attribute is per function and per device; setting it is idempotent (the 48 KB
+  // that need none hold a kernel's static shared memory as well)
+  if (smem > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute"); return -5; }
   }
   return 0;
 }
 
-// Blocked LU / Cholesky (blk.cuh): a persistent CTA per SM with as many warps as
-// shared memory holds (at most 16).
+// LU / Cholesky with rows in registers (rows.cuh): a persistent CTA per SM with as many
+// warps as shared memory holds, at most 16. Between 12 and 16 it stays at 12: warps are
+// dealt to four schedulers, so 13 to 15 cost the registers of 16 (128 a thread instead of
+// 168) without its parallelism (float32 LU, order 56, 65,536 matrices: 1547 us with 12,
+// 1568 with 14; Cholesky 1398 and 1476).
 template <class T, int NP, int NRHS, int GO = 0>
 constexpr int blk_wpc() {
-  constexpr int FIT = (227 * 1024) / dev::BlkCfg<T, NP, NRHS, GO>::WARPB;
-  return FIT < 1 ? 1 : (FIT > 16 ? 16 : FIT);
+  constexpr int FIT = (227 * 1024 - dev::kRowConst) / dev::BlkCfg<T, NP, NRHS, GO>::WARPB;
+  return FIT < 1 ? 1 : (FIT >= 16 ? 16 : FIT >= 12 ? 12 : FIT);
 }
 
-// Lanes per matrix: two matrices share a warp (16 lanes each, two rows per lane)
-// where that still leaves 16 warps per SM (orders 17..32 in float32, 17..24 in
-// float64) and for float32 LU at order 40. Measured on B200 against one matrix
-// per warp at batch 262,144: +12..43 % there, slower wherever it costs warps.
-// Orders 9..16 pack four matrices per warp.
-template <class T, int NP, int NRHS, bool CHOL>
+// Lanes per matrix (0: the layout's own choice; the matrices that share a warp run its
+// steps together, so small orders spend fewer instructions each). Measured on B200 at
+// 65,536 to 262,144 matrices against the next choice, best warps each: order 8, 4 lanes
+// 117 us against 118 with 8 (float32 LU), 102 against 113 (float64 Cholesky); order 16, 8
+// lanes 180 against 247 with 16 (float32 Cholesky), 325 against 429 (float64); order 24,
+// float32 8 lanes 595 against 691 with 16, float64 16 lanes 650 against 681 with 8;
+// order 32, float32 16 lanes 1114 against 1132 with 32, float64 32 lanes 1105 against
+// 1226 with 16; order 40, float32 16 lanes 1214 against 1371 with 32, float64 32 lanes
+// (within 2 % of 16). Above that, one matrix per warp.
+template <class T, int NP>
 constexpr int blk_lanes() {
-  // order 9..16: four matrices per warp (8 lanes, two rows per lane): +22..50 % over
-  // two per warp on B200 at 262,144 matrices (posv fp64 303 -> 405 M solves/s)
-  if (NP == 16) return 8;
-  // order 5..8 Cholesky: eight per warp (4 lanes): posv 1177 -> 1560 M solves/s (fp64);
-  // LU keeps four per warp (the 4-lane LU form is not used)
-  if (NP == 8) return CHOL ? 4 : 0;
-  // float32 order 17..24: four per warp (8 lanes, three rows per lane): +18 % (posv),
-  // +39 % (gesv); float64 keeps two per warp
-  if (NP == 24 && sizeof(T) == 4) return 8;
-  if (NP <= 16 || NP > 40) return 0;
-  if (NP == 40) return (sizeof(T) == 4 && !CHOL) ? 16 : 0;
-  return blk_wpc<T, NP, NRHS, 16>() == 16 ? 16 : 0;
+  constexpr bool F32 = sizeof(T) == 4;
+  switch (NP) {
+    case 8: return 4;
+    case 16: return 8;
+    case 24: return F32 ? 8 : 16;
+    case 32: case 40: return F32 ? 16 : 32;
+    default: return 0;
+  }
 }
 
 // Two warps per matrix (blk2.cuh) for float64 LU of padded order 48..56: measured on
@@ -139,7 +143,7 @@ int launch_blk3(const SolveArgs<T>& a, cudaStream_t st) {
 }
 
 // LU kernel family: 0 = by order (the default), 1 = shared-memory blocked kernels
-// with CUDA-core updates everywhere (blk.cuh / blk2.cuh / blk3.cuh), 3 = the float64
+// with CUDA-core updates everywhere (rows.cuh / blk2.cuh / blk3.cuh), 3 = the float64
 // tensor-core trailing update (blk_tc.cuh) at every padded order 32..64. Read once
 // from TSDX_LU_KERNEL ("smem" or "tc"); all give bit-identical results.
 int lu_kernel_family();
@@ -179,7 +183,7 @@ int launch_blk(const SolveArgs<T>& a, cudaStream_t st) {
   }
   if constexpr (!CHOL && sizeof(T) == 8 && NP == 64) return launch_blk3<T, NP, NRHS>(a, st);
   if constexpr (!CHOL && sizeof(T) == 8 && NP >= 48) return launch_blk2<T, NP, NRHS>(a, st);
-  constexpr int GO = blk_lanes<T, NP, NRHS, CHOL>();
+  constexpr int GO = blk_lanes<T, NP>();
   using C = dev::BlkCfg<T, NP, NRHS, GO>;
   constexpr int WPC = blk_wpc<T, NP, NRHS, GO>();
   constexpr int SMEM = WPC * C::WARPB;

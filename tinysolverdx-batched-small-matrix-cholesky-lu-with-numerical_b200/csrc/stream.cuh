@@ -23,7 +23,7 @@
 // bit-identical to them. The launches are capturable in a CUDA graph (no host
 // synchronisation; scratch passed in by the caller).
 #pragma once
-#include "blk.cuh"
+#include "rows.cuh"
 
 namespace tsdx {
 namespace dev {
@@ -60,18 +60,21 @@ __device__ __forceinline__ int bucket_of(int kind, int n, int nrhs) {
 }
 __device__ __forceinline__ int bucket_class(int b) { return kStreamClasses - 1 - (b >> 2); }
 // matrices per work unit for a bucket (the dense kernels' measured packings): order
-// <= 8: 8 (Cholesky, 4 lanes each) or 4 (LU); order 9..16: 4; order 17..24: 4 in
-// float32, 2 in float64; order 25..32: 2; above: 1. Sched bit c (order class c =
-// 0..3) asks for one matrix per warp instead.
+// <= 8: 8; order 9..16: 4; order 17..24: 4 in float32, 2 in float64; order 25..40: 2 in
+// float32, else 1. Sched bit c (order class c = 0..3) asks for one matrix per warp
+// instead.
 template <class T>
 __device__ __forceinline__ int unit_size(int b, unsigned sched) {
   const int c = bucket_class(b);
-  const bool lu = (b >> 1) & 1;
-  if (c >= 4 || ((sched >> c) & 1u)) return 1;
-  if (c == 0) return lu ? 4 : 8;
-  if (c == 1) return 4;
-  if (c == 2) return sizeof(T) == 4 ? 4 : 2;
-  return 2;
+  constexpr bool F32 = sizeof(T) == 4;
+  if (c < 4 && ((sched >> c) & 1u)) return 1;
+  switch (c) {
+    case 0: return 8;
+    case 1: return 4;
+    case 2: return F32 ? 4 : 2;
+    case 3: case 4: return F32 ? 2 : 1;
+    default: return 1;
+  }
 }
 
 template <class T>
@@ -129,12 +132,13 @@ __global__ void stream_scatter_kernel(StreamArgs<T> a) {
 
 template <class T, int NP, int NRHS, bool CHOL, int G>
 __device__ __forceinline__ void stream_unit(unsigned char* M, const StreamArgs<T>& a, const int* perm, int first,
-                                            int last, int lane) {
+                                            int last, int lane, unsigned zrow) {
   Seg g;
   g.lane = lane;
   g.lsl = lane & (G - 1);
   g.segbase = (lane / G) * G;
-  g.segmask = (G == 32) ? kFull : (((1u << G) - 1u) << g.segbase);
+  g.segmask = (G == 32) ? kFull : (((1u << (G & 31)) - 1u) << g.segbase);
+  g.zrow = zrow;
   const int idx = first + lane / G;
   MatJob<T> j;
   j.live = idx < last;
@@ -171,14 +175,15 @@ __global__ void __launch_bounds__(WPC * 32, 1) stream_kernel(StreamArgs<T> a) {
   constexpr int B_LO = (kStreamClasses - 1 - CHI) * 4, B_HI = (kStreamClasses - CLO) * 4;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int ustart_s[kStreamBuckets + 1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ __align__(16) unsigned char consts[kRowConst];
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int* start = a.scratch + kStreamBuckets;
   const int* cnt = a.scratch;
   const int* ustart = a.scratch + 3 * kStreamBuckets;
   int* head = a.scratch + 2 * kStreamBuckets + CLO;
   const int* perm = a.scratch + 4 * kStreamBuckets + 2;
   if (threadIdx.x <= kStreamBuckets) ustart_s[threadIdx.x] = ustart[threadIdx.x];
-  __syncthreads();
+  const unsigned zrow = rows_constants(consts);  // a block barrier
   const int u0 = ustart_s[B_LO], total = ustart_s[B_HI];
   unsigned char* M = smem + warp * WARPB;
   for (;;) {
@@ -194,7 +199,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) stream_kernel(StreamArgs<T> a) {
     const bool one = us == 1;
     const int c = bucket_class(b);
     const bool lu = (b >> 1) & 1, wide = b & 1;
-#define TSDX_SU(NP_, R_, CH_, G_) stream_unit<T, NP_, R_, CH_, G_>(M, a, perm, first, last, lane)
+#define TSDX_SU(NP_, R_, CH_, G_) stream_unit<T, NP_, R_, CH_, G_>(M, a, perm, first, last, lane, zrow)
 #define TSDX_SU_KIND(NP_, R_, G_) \
   if (lu) TSDX_SU(NP_, R_, false, G_); \
   else TSDX_SU(NP_, R_, true, G_)
@@ -203,15 +208,8 @@ __global__ void __launch_bounds__(WPC * 32, 1) stream_kernel(StreamArgs<T> a) {
   else { TSDX_SU_KIND(NP_, 2, G_); }
     switch (c) {
       case 0:
-        if constexpr (CLO > 0) {
-        } else if (one) {
-          TSDX_SU_RHS(8, 32)
-        } else if (wide) {
-          if (lu) TSDX_SU(8, 8, false, 8);
-          else TSDX_SU(8, 8, true, 4);
-        } else {
-          if (lu) TSDX_SU(8, 2, false, 8);
-          else TSDX_SU(8, 2, true, 4);
+        if constexpr (CLO <= 0) {
+          if (one) { TSDX_SU_RHS(8, 32) } else { TSDX_SU_RHS(8, 4) }
         }
         break;
       case 1:
@@ -220,22 +218,17 @@ __global__ void __launch_bounds__(WPC * 32, 1) stream_kernel(StreamArgs<T> a) {
         }
         break;
       case 2:
-        if constexpr (CLO > 2 || CHI < 2) {
-        } else if (one) {
-          TSDX_SU_RHS(24, 32)
-        } else if constexpr (sizeof(T) == 4) {
-          TSDX_SU_RHS(24, 8)
-        } else {
-          TSDX_SU_RHS(24, 16)
+        if constexpr (CLO <= 2 && CHI >= 2) {
+          if (one) { TSDX_SU_RHS(24, 32) } else { TSDX_SU_RHS(24, (sizeof(T) == 4 ? 8 : 16)) }
         }
         break;
       case 3:
         if constexpr (CLO <= 3 && CHI >= 3) {
-          if (one) { TSDX_SU_RHS(32, 32) } else { TSDX_SU_RHS(32, 16) }
+          if (sizeof(T) == 8 || one) { TSDX_SU_RHS(32, 32) } else { TSDX_SU_RHS(32, (sizeof(T) == 4 ? 16 : 32)) }
         }
         break;
       case 4:
-        if constexpr (CLO <= 4 && CHI >= 4) { TSDX_SU_RHS(40, 32) }
+        if constexpr (CLO <= 4 && CHI >= 4) { TSDX_SU_RHS(40, (sizeof(T) == 4 ? 16 : 32)) }
         break;
       case 5:
         if constexpr (CLO <= 5 && CHI >= 5) { TSDX_SU_RHS(48, 32) }

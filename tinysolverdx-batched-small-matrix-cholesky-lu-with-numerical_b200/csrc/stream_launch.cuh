@@ -18,11 +18,11 @@ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 template <class T> constexpr int class_warpb(int c) {
   using dev::BlkCfg;
   switch (c) {
-    case 0: return cmax(BlkCfg<T, 8, 8, 32>::WARPB, cmax(BlkCfg<T, 8, 8, 8>::WARPB, BlkCfg<T, 8, 8, 4>::WARPB));
+    case 0: return cmax(BlkCfg<T, 8, 8, 32>::WARPB, BlkCfg<T, 8, 8, 4>::WARPB);
     case 1: return cmax(BlkCfg<T, 16, 8, 32>::WARPB, BlkCfg<T, 16, 8, 8>::WARPB);
     case 2: return cmax(BlkCfg<T, 24, 8, 32>::WARPB, BlkCfg<T, 24, 8, sizeof(T) == 4 ? 8 : 16>::WARPB);
-    case 3: return cmax(BlkCfg<T, 32, 8, 32>::WARPB, BlkCfg<T, 32, 8, 16>::WARPB);
-    case 4: return BlkCfg<T, 40, 8, 32>::WARPB;
+    case 3: return cmax(BlkCfg<T, 32, 8, 32>::WARPB, BlkCfg<T, 32, 8, sizeof(T) == 4 ? 16 : 32>::WARPB);
+    case 4: return BlkCfg<T, 40, 8, sizeof(T) == 4 ? 16 : 32>::WARPB;
     case 5: return BlkCfg<T, 48, 8, 32>::WARPB;
     case 6: return BlkCfg<T, 56, 8, 32>::WARPB;
     default: return BlkCfg<T, 64, 8, 32>::WARPB;
@@ -39,8 +39,9 @@ template <class T> constexpr int stream_warpb(int lo, int hi) {
 template <class T, int CLO, int CHI>
 int launch_drain(const dev::StreamArgs<T>& a, cudaStream_t st) {
   constexpr int WARPB = stream_warpb<T>(CLO, CHI);
-  constexpr int FIT = (227 * 1024) / WARPB;
-  constexpr int WPC = FIT < 1 ? 1 : (FIT > 16 ? 16 : FIT);
+  // as blk_wpc; the static shared memory holds the unit table and the rows' constants
+  constexpr int FIT = (227 * 1024 - dev::kRowConst - 256) / WARPB;
+  constexpr int WPC = FIT < 1 ? 1 : (FIT >= 16 ? 16 : FIT >= 12 ? 12 : FIT);
   constexpr int SMEM = WPC * WARPB;
   auto kern = dev::stream_kernel<T, WARPB, WPC, CLO, CHI>;
   if (int rc = prepare(kern, SMEM)) return rc;
