@@ -60,3 +60,25 @@ def test_odd_pivots_bit_exact(oracle, n, dtype):
     assert np.array_equal(info, infoo) and np.array_equal(piv, pivo)
     for i in range(len(A)):
         assert same(LU[i], LUo[i]), i
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 47, 49, 64])
+@pytest.mark.parametrize("nrhs", [2, 4, 5, 8, 16, 17])
+def test_solves_from_factor(oracle, n, nrhs, dtype):
+    r = np.random.default_rng(n * 31 + nrhs)
+    A = M.general(r, 9, n, 1e2).astype(dtype)
+    S = M.spd(r, 9, n, 1e2).astype(dtype)
+    B = r.standard_normal((9, n, nrhs)).astype(dtype)
+    LU, piv, _ = oracle.lu(A, "scalar")
+    L, _ = oracle.cholesky(S, "simd")
+    bad = piv.astype(np.int32).copy()
+    bad[0, -1] = n            # a pivot that names no row is ignored: the last swap is a no-op anyway
+    bad[1, -1] = -1
+    for mats, run in ((A, lambda b: device.getrs(dev(LU), dev(bad), b)), (S, lambda b: device.potrs(dev(L), b))):
+        b = dev(B)
+        run(b)
+        X, M64, B64 = b.cpu().numpy().astype(np.float64), mats.astype(np.float64), B.astype(np.float64)
+        num = np.linalg.norm(B64 - M64 @ X, axis=1)
+        den = np.linalg.norm(M64, axis=(1, 2))[:, None] * np.linalg.norm(X, axis=1) + np.linalg.norm(B64, axis=1)
+        assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2

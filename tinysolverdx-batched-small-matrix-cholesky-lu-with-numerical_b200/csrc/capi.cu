@@ -101,17 +101,17 @@ int run_device(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, i
     a.nrhs = std::min(nrhs, 8);
     const int rc = (kind == POTRF || kind == POSV) ? run_chol<T>(a, st) : run_lu<T>(a, st);
     if (rc) return rc;
-    for (int b0 = 8; b0 < nrhs; b0 += 8) {  // remaining right-hand sides from the factor
+    for (int b0 = 8; b0 < nrhs; b0 += kTrsRhs) {  // remaining right-hand sides from the factor
       a.b0 = b0;
-      a.nrhs = std::min(8, nrhs - b0);
+      a.nrhs = std::min(kTrsRhs, nrhs - b0);
       const int r2 = (kind == POSV) ? run_potrs<T>(a, st) : run_getrs<T>(a, st);
       if (r2) return r2;
     }
     return TSDX_OK;
   }
-  for (int b0 = 0; b0 < nrhs; b0 += 8) {
+  for (int b0 = 0; b0 < nrhs; b0 += kTrsRhs) {
     a.b0 = b0;
-    a.nrhs = std::min(8, nrhs - b0);
+    a.nrhs = std::min(kTrsRhs, nrhs - b0);
     const int rc = (kind == POTRS) ? run_potrs<T>(a, st) : run_getrs<T>(a, st);
     if (rc) return rc;
   }

@@ -199,14 +199,22 @@ int launch_blk(const SolveArgs<T>& a, cudaStream_t st) {
   return 0;
 }
 
-template <class T, int NP, int NRHS, bool LU>
-int launch_trs(const SolveArgs<T>& a, int vec, cudaStream_t st) {
-  constexpr int SMEM = dev::SolveSmem<T, NP>::CTA;
-  auto kern = dev::trs_kernel<T, NP, NRHS, LU>;
+// Triangular solves (solve.cuh): one warp per matrix, as many warps as shared memory and
+// 128 registers a thread allow. W: tiles of 8 right-hand sides (float64) or columns
+// (float32).
+template <class T, int NP, int W, bool LU>
+int launch_trs(const SolveArgs<T>& a, cudaStream_t st) {
+  using C = dev::TrsCfg<T, NP>;
+  constexpr int FIT = (227 * 1024) / C::WARPB;
+  constexpr int WPC = FIT > 16 ? 16 : FIT;
+  constexpr int SMEM = WPC * C::WARPB;
+  auto kern = [] {
+    if constexpr (sizeof(T) == 8) return dev::trs_f64_kernel<NP, W, LU, WPC>;
+    else return dev::trs_f32_kernel<NP, W, LU, WPC>;
+  }();
   if (int rc = prepare(kern, SMEM)) return rc;
-  const long long ctas = (a.batch + 3) / 4;
-  const int grid = grid_for(kern, SMEM, ctas);
-  kern<<<grid, 128, SMEM, st>>>(a, FastDiv((unsigned)a.n), vec);
+  const int grid = grid_for(kern, SMEM, (a.batch + WPC - 1) / WPC, WPC * 32);
+  kern<<<grid, WPC * 32, SMEM, st>>>(a);
   launch_counter().fetch_add(1);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_cuda_error(e, "kernel launch"); return -5; }
@@ -241,18 +249,23 @@ int run_blk(const SolveArgs<T>& a, cudaStream_t st) {
   return 0;
 }
 
-// One solve pass from a factor (nrhs <= 8).
+// One solve pass from a factor (nrhs <= kTrsRhs). Orders run in the next multiple of 16.
+constexpr int kTrsRhs = 16;
+template <class T, bool LU, int W>
+int run_trs_np(const SolveArgs<T>& a, cudaStream_t st) {
+  switch ((a.n + 15) / 16) {
+    case 1: return launch_trs<T, 16, W, LU>(a, st);
+    case 2: return launch_trs<T, 32, W, LU>(a, st);
+    case 3: return launch_trs<T, 48, W, LU>(a, st);
+    default: return launch_trs<T, 64, W, LU>(a, st);
+  }
+}
 template <class T, bool LU>
 int run_trs(const SolveArgs<T>& a, cudaStream_t st) {
-  const int vec = vec_for<T>(a.A, a.n);
-  SolveArgs<T> b = a;
-  b.rowdiv = FastDiv((unsigned)(a.n * int(sizeof(T)) / vec));
-  const int np = np_of(a.n) <= 32 ? 32 : 64, rb = nrhs_bucket(a.nrhs);
-  if (np == 32) {
-    TSDX_RHS_SWITCH(rb == 0 ? 1 : rb, return (launch_trs<T, 32, (R_ > 0 ? R_ : 1), LU>(b, vec, st)));
-  }
-  TSDX_RHS_SWITCH(rb == 0 ? 1 : rb, return (launch_trs<T, 64, (R_ > 0 ? R_ : 1), LU>(b, vec, st)));
-  return 0;
+  if constexpr (sizeof(T) == 8) return a.nrhs > 8 ? run_trs_np<T, LU, 2>(a, st) : run_trs_np<T, LU, 1>(a, st);
+  else
+    return a.nrhs > 8 ? run_trs_np<T, LU, 16>(a, st) : a.nrhs > 4 ? run_trs_np<T, LU, 8>(a, st)
+         : a.nrhs > 1 ? run_trs_np<T, LU, 4>(a, st) : run_trs_np<T, LU, 1>(a, st);
 }
 
 // Explicitly instantiated in the per-type translation units.

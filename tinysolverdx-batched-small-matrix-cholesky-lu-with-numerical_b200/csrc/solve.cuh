@@ -2,104 +2,410 @@
 // (P L U x = b) — TinySolverDx kernels.hpp:184-227 driven by batched.hpp:248-268
 // (which the reference always runs on the CPU; here they run on the GPU).
 //
-// One warp per matrix: the factor is staged to shared memory with cp.async, the
-// right-hand sides live in registers (lane l owns rows l and l + 32). The forward
-// substitution keeps the reference's chain (increasing k, fused multiply-add, and
-// for Cholesky the division by l_ii); the backward substitution is column-oriented
-// and multiplies by the reciprocal of the diagonal, so X agrees with the
+// One warp per matrix, up to 16 right-hand sides at a time: the factor is staged to
+// shared memory with cp.async, the right-hand sides live in registers. The forward
+// substitution keeps the reference's chain (increasing k, fused multiply-add, and for
+// Cholesky the division by l_ii); the backward substitution is column-oriented
+// (decreasing k) and multiplies by the reciprocal of the diagonal, so X agrees with the
 // reference to rounding.
+//
+//   float64: the right-hand sides are 8 x 8 accumulator tiles of the FP64 tensor cores.
+//     Blocks of 8 rows are solved by shuffles among the 8 lanes of a column pair; the
+//     rows below (above) take the block by one tile product per 8 rows, which
+//     accumulates its four products in fragment order as fused multiply-adds (see
+//     blk_tc.cuh); the backward pass numbers the fragments downwards. So every element
+//     keeps its chain of operations.
+//   float32: lane l owns rows l and l + 32; the solved row goes through shared memory
+//     (which keeps it as the result) and every lane updates its rows, two columns to an
+//     instruction.
 #pragma once
-#include "common.cuh"
+#include "blk_tc.cuh"
+#include "rows.cuh"
 
 namespace tsdx {
 namespace dev {
 
 template <class T, int NP>
-struct SolveSmem {
-  static constexpr int RS = NP * int(sizeof(T)) + 16;
-  static constexpr int WARP = NP * RS + 64 * 4;  // staged factor + permutation
-  static constexpr int CTA = 4 * WARP;
+struct TrsCfg {
+  static constexpr int RS = NP * int(sizeof(T)) + 16;  // an odd number of 16-byte units
+  static constexpr int MAT = NP * RS;
+  static constexpr int XB = 16 * int(sizeof(T));       // one solved row (float32)
+  static constexpr int OFF_X = MAT, OFF_PERM = MAT + (sizeof(T) == 4 ? NP * XB : 0);
+  static constexpr int WARPB = (OFF_PERM + 2 * NP * 4 + 127) / 128 * 128;
+  static_assert(NP % 16 == 0, "row stride in an odd number of 16-byte units");
 };
 
-// LU == true: getrs with pivots; LU == false: potrs.
-template <class T, int NP, int NRHS, bool LU>
-__global__ void __launch_bounds__(128) trs_kernel(SolveArgs<T> p, FastDiv ndiv, int vec) {
-  using SM = SolveSmem<T, NP>;
-  constexpr int MR = (NP + 31) / 32;
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* stage = smem + warp * SM::WARP;
-  int* perm = reinterpret_cast<int*>(stage + NP * SM::RS);
-  const int n = p.n;
-  const long long nn = (long long)n * n;
-  const int rc = n * int(sizeof(T)) / vec;
-  const long long nw = (long long)gridDim.x * 4;
-
-  for (long long m = (long long)blockIdx.x * 4 + warp; m < p.batch; m += nw) {
-    const char* g = reinterpret_cast<const char*>(p.A + m * nn);
-    if (vec == 16) stage_in<T, 16, SM::RS, SM::WARP>(stage, g, n, n, rc, p.rowdiv, ndiv, lane, 32);
-    else if (vec == 8) stage_in<T, 8, SM::RS, SM::WARP>(stage, g, n, n, rc, p.rowdiv, ndiv, lane, 32);
-    else stage_in<T, 4, SM::RS, SM::WARP>(stage, g, n, n, rc, p.rowdiv, ndiv, lane, 32);
-    if (LU) {
-      for (int i = lane; i < n; i += 32) perm[i] = i;
-      __syncwarp();
-      if (lane == 0)
-        for (int k = 0; k < n; ++k) {  // kernels.hpp:207-213: swaps applied in k order
-          int q = p.piv[m * n + k];
-          q = (q < 0 || q >= n) ? k : q;  // out-of-range pivots are ignored, never dereferenced
-          const int t = perm[k]; perm[k] = perm[q]; perm[q] = t;
-        }
-    }
-    cp_async_wait<0>();
-    __syncwarp();
-    auto at = [&](int r, int c) -> T { return *reinterpret_cast<const T*>(stage + r * SM::RS + c * int(sizeof(T))); };
-
-    T b[MR][NRHS];
-    const long long bbase = m * (long long)n * p.ldb + p.b0;
+// Stages the factor, identity-padded to NP, and for LU the row that the pivots bring to
+// each position: kernels.hpp:207-213 swaps rows j and piv[j] in increasing j, so a
+// position's origin is found by following it backwards through the swaps. All positions
+// are traced at once, one swap at a time; a pivot outside [0, n) is ignored.
+template <class T, int NP, bool LU>
+__device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const int* piv, int n, int lane) {
+  using C = TrsCfg<T, NP>;
+  constexpr int RS = C::RS, TS = int(sizeof(T)), MR = (NP + 31) / 32;
+  const int vec = vec_of<T>(A, n), rowb = n * TS;
+  const char* src = reinterpret_cast<const char*>(A);
+  if (vec == 16) walk_chunks<T, NP, 32, 16>(n, lane, [&](int r, int c) { cp_async<16>(M + r * RS + c * 16, src + r * rowb + c * 16); });
+  else if (vec == 8) walk_chunks<T, NP, 32, 8>(n, lane, [&](int r, int c) { cp_async<8>(M + r * RS + c * 8, src + r * rowb + c * 8); });
+  else if constexpr (sizeof(T) == 4) walk_chunks<T, NP, 32, 4>(n, lane, [&](int r, int c) { cp_async<4>(M + r * RS + c * 4, src + r * rowb + c * 4); });
+  cp_async_commit();
+  if (n < NP) {
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
       const int r = lane + 32 * s;
-      const int src = (r < n) ? (LU ? perm[r] : r) : 0;
-#pragma unroll
-      for (int c = 0; c < NRHS; ++c) b[s][c] = (r < n && c < p.nrhs) ? p.B[bbase + (long long)src * p.ldb + c] : T(0);
+      T* row = reinterpret_cast<T*>(M + r * RS);
+      if (r < n) {
+        for (int c = n; c < NP; ++c) row[c] = T(0);
+      } else if (r < NP) {
+        for (int c = 0; c < NP * TS / 16; ++c) reinterpret_cast<uint4*>(row)[c] = make_uint4(0, 0, 0, 0);
+        row[r] = T(1);
+      }
     }
+  }
+  if constexpr (LU) {
+    int* pv = reinterpret_cast<int*>(M + C::OFF_PERM);
+    int* perm = pv + NP;
+    int q[MR];
+#pragma unroll
+    for (int s = 0; s < MR; ++s) {
+      const int k = lane + 32 * s;
+      q[s] = k;
+      if (k < n) {
+        const int v = piv[k];
+        if (v >= 0 && v < n) q[s] = v;
+      }
+      if (k < NP) pv[k] = q[s];
+      q[s] = k;
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int j0 = NP - 4; j0 >= 0; j0 -= 4) {
+      const int4 pj = *reinterpret_cast<const int4*>(pv + j0);
+      const int pp[4] = {pj.x, pj.y, pj.z, pj.w};
+#pragma unroll
+      for (int j = 3; j >= 0; --j)
+#pragma unroll
+        for (int s = 0; s < MR; ++s) q[s] = q[s] == j0 + j ? pp[j] : (q[s] == pp[j] ? j0 + j : q[s]);
+    }
+#pragma unroll
+    for (int s = 0; s < MR; ++s)
+      if (lane + 32 * s < NP) perm[lane + 32 * s] = q[s];
+  }
+}
+
+// ---------------------------------------------------------------- float64
+// NT tiles of 8 right-hand sides. Accumulator fragment: lane (fr, fq) holds columns 2 fq
+// and 2 fq + 1 of row fr of each tile.
+template <int NP, int NT, bool LU, int WPC>
+__global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> p) {
+  using C = TrsCfg<double, NP>;
+  constexpr int RS = C::RS, NB = NP / 8;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int fr = lane >> 2, fq = lane & 3;
+  unsigned char* M = smem + warp * C::WARPB;
+  const int* perm = reinterpret_cast<const int*>(M + C::OFF_PERM) + NP;
+  auto at = [&](int r, int c) -> double { return *reinterpret_cast<const double*>(M + r * RS + c * 8); };
+  const int n = p.n;
+  const long long nn = (long long)n * n, step = (long long)gridDim.x * WPC;
+
+  for (long long m = (long long)blockIdx.x * WPC + warp; m < p.batch; m += step) {
+    if (lane == 0 && m + step < p.batch) {
+      prefetch_l2(p.A + (m + step) * nn, nn * 8);
+      prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 8);
+    }
+    trs_stage<double, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, lane);
+    if (LU) __syncwarp();
+    double* Bm = p.B + m * (long long)n * p.ldb + p.b0;
+    double2 c[NB][NT];
+#pragma unroll
+    for (int I = 0; I < NB; ++I) {
+      const int r = 8 * I + fr;
+      const double* row = Bm + (long long)(LU ? perm[r] : r) * p.ldb;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int col = 8 * t + 2 * fq;
+        c[I][t].x = (r < n && col < p.nrhs) ? row[col] : 0.0;
+        c[I][t].y = (r < n && col + 1 < p.nrhs) ? row[col + 1] : 0.0;
+      }
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+
+    // B fragment (k = 4 h + fq, or counted down from 7 with DOWN; column fr) of the solved
+    // block: its value stands on lane 4 k + fr / 2
+    auto bfrag = [&](const double2& v, int k) -> double {
+      const int src = 4 * k + (fr >> 1);
+      const double x = __shfl_sync(kFull, v.x, src), y = __shfl_sync(kFull, v.y, src);
+      return (fr & 1) ? y : x;
+    };
     // forward: L y = P b
-    for (int k = 0; k < n; ++k) {
-      const int ks = k >> 5, kl = k & 31;
-      const T lkk = LU ? T(1) : at(k, k);
 #pragma unroll
-      for (int c = 0; c < NRHS; ++c) {
-        T v = b[0][c];
-        if (MR > 1 && ks == 1) v = b[MR - 1][c];
-        T y = __shfl_sync(kFull, v, kl);
-        if (!LU) y = div_(y, lkk);
+    for (int K = 0; K < NB; ++K) {
+      double l[8];
+      {
+        const double2* lr = reinterpret_cast<const double2*>(M + (8 * K + fr) * RS + 64 * K);
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = lane + 32 * s;
-          const T lrk = (r > k && r < n) ? at(r, k) : T(0);
-          b[s][c] = (r == k) ? y : ((r > k && r < n) ? fma_(-lrk, y, b[s][c]) : b[s][c]);
+        for (int j = 0; j < 4; ++j) {
+          l[2 * j] = lr[j].x;
+          l[2 * j + 1] = lr[j].y;
+        }
+      }
+      const double dkk = LU ? 1.0 : at(8 * K + fr, 8 * K + fr);
+      const double dinv = LU ? 1.0 : rcp_(dkk);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (!LU && fr == j) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) c[K][t] = make_double2(div_by(c[K][t].x, dkk, dinv), div_by(c[K][t].y, dkk, dinv));
+        }
+        if (!LU) __syncwarp();
+        if (j == 7) break;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const double yx = __shfl_sync(kFull, c[K][t].x, 4 * j + fq), yy = __shfl_sync(kFull, c[K][t].y, 4 * j + fq);
+          c[K][t].x = fr > j ? fma_(-l[j], yx, c[K][t].x) : c[K][t].x;
+          c[K][t].y = fr > j ? fma_(-l[j], yy, c[K][t].y) : c[K][t].y;
+        }
+      }
+      double b0[NT], b1[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        b0[t] = bfrag(c[K][t], fq);
+        b1[t] = bfrag(c[K][t], 4 + fq);
+      }
+#pragma unroll
+      for (int I = K + 1; I < NB; ++I) {
+        const double a0 = -at(8 * I + fr, 8 * K + fq), a1 = -at(8 * I + fr, 8 * K + 4 + fq);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          dmma_m8n8k4(c[I][t], a0, b0[t]);
+          dmma_m8n8k4(c[I][t], a1, b1[t]);
         }
       }
     }
-    // backward: U x = y (LU) or L^T x = y (Cholesky)
-    for (int k = n - 1; k >= 0; --k) {
-      const int ks = k >> 5, kl = k & 31;
-      const T rinv = rcp_(at(k, k));
-      T ck[MR];
+    // backward: U x = y (LU) or L^T x = y (Cholesky), columns in decreasing order
 #pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const int r = lane + 32 * s;
-        ck[s] = (r < k) ? (LU ? at(r, k) : at(k, r)) : T(0);
+    for (int K = NB - 1; K >= 0; --K) {
+      double u[8];
+      if constexpr (LU) {
+        const double2* ur = reinterpret_cast<const double2*>(M + (8 * K + fr) * RS + 64 * K);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          u[2 * j] = ur[j].x;
+          u[2 * j + 1] = ur[j].y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[j] = at(8 * K + j, 8 * K + fr);
+      }
+      const double dinv = rcp_(at(8 * K + fr, 8 * K + fr));
+#pragma unroll
+      for (int j = 7; j >= 0; --j) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          c[K][t].x = fr == j ? c[K][t].x * dinv : c[K][t].x;
+          c[K][t].y = fr == j ? c[K][t].y * dinv : c[K][t].y;
+          if (j == 0) continue;
+          const double xx = __shfl_sync(kFull, c[K][t].x, 4 * j + fq), xy = __shfl_sync(kFull, c[K][t].y, 4 * j + fq);
+          c[K][t].x = fr < j ? fma_(-u[j], xx, c[K][t].x) : c[K][t].x;
+          c[K][t].y = fr < j ? fma_(-u[j], xy, c[K][t].y) : c[K][t].y;
+        }
+      }
+      double b0[NT], b1[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        b0[t] = bfrag(c[K][t], 7 - fq);
+        b1[t] = bfrag(c[K][t], 3 - fq);
       }
 #pragma unroll
-      for (int c = 0; c < NRHS; ++c) {
-        T v = b[0][c];
-        if (MR > 1 && ks == 1) v = b[MR - 1][c];
-        const T x = __shfl_sync(kFull, v * rinv, kl);
+      for (int I = 0; I < K; ++I) {
+        const double a0 = LU ? -at(8 * I + fr, 8 * K + 7 - fq) : -at(8 * K + 7 - fq, 8 * I + fr);
+        const double a1 = LU ? -at(8 * I + fr, 8 * K + 3 - fq) : -at(8 * K + 3 - fq, 8 * I + fr);
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = lane + 32 * s;
-          b[s][c] = (r == k) ? x : ((r < k) ? fma_(-ck[s], x, b[s][c]) : b[s][c]);
+        for (int t = 0; t < NT; ++t) {
+          dmma_m8n8k4(c[I][t], a0, b0[t]);
+          dmma_m8n8k4(c[I][t], a1, b1[t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int I = 0; I < NB; ++I) {
+      const int r = 8 * I + fr;
+      if (r >= n) continue;
+      double* row = Bm + (long long)r * p.ldb;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int col = 8 * t + 2 * fq;
+        if (col < p.nrhs) row[col] = c[I][t].x;
+        if (col + 1 < p.nrhs) row[col + 1] = c[I][t].y;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------- float32
+// NRHS columns in units of two (one: a single scalar column, exchanged by shuffle).
+template <int NP, int NRHS, bool LU, int WPC>
+__global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p) {
+  using C = TrsCfg<float, NP>;
+  using U = Unit<float>;
+  using E = U::E;
+  constexpr int RS = C::RS, XB = C::XB, MR = (NP + 31) / 32, NU = NRHS > 1 ? NRHS / 2 : 1;
+  static_assert(NRHS == 1 || NRHS % 4 == 0, "whole 16-byte vectors");
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  unsigned char* M = smem + warp * C::WARPB;
+  const unsigned Mu = (unsigned)__cvta_generic_to_shared(M), Xu = Mu + C::OFF_X;
+  const int* perm = reinterpret_cast<const int*>(M + C::OFF_PERM) + NP;
+  const int n = p.n;
+  const long long nn = (long long)n * n, step = (long long)gridDim.x * WPC;
+
+  for (long long m = (long long)blockIdx.x * WPC + warp; m < p.batch; m += step) {
+    if (lane == 0 && m + step < p.batch) {
+      prefetch_l2(p.A + (m + step) * nn, nn * 4);
+      prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 4);
+    }
+    trs_stage<float, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, lane);
+    if (LU) __syncwarp();
+    float* Bm = p.B + m * (long long)n * p.ldb + p.b0;
+    E b[MR][NU];
+    float b1[MR];
+#pragma unroll
+    for (int s = 0; s < MR; ++s) {
+      const int r = lane + 32 * s;
+      const float* row = Bm + (long long)(LU && r < n ? perm[r] : r) * p.ldb;
+      float v[NRHS > 1 ? NRHS : 2];
+#pragma unroll
+      for (int c = 0; c < NRHS; ++c) v[c] = (r < n && c < p.nrhs) ? row[c] : 0.f;
+      b1[s] = v[0];
+      if constexpr (NRHS > 1) {
+#pragma unroll
+        for (int c = 0; c < NU; ++c) b[s][c] = U::pack(v[2 * c], v[2 * c + 1]);
+      }
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    float dg[MR], dinv[MR];
+    unsigned own[MR], xown[MR];
+#pragma unroll
+    for (int s = 0; s < MR; ++s) {
+      const int r = lane + 32 * s < NP ? lane + 32 * s : NP - 1;
+      own[s] = Mu + r * RS;
+      xown[s] = Xu + r * XB;
+      dg[s] = *reinterpret_cast<const float*>(M + r * RS + r * 4);
+      dinv[s] = rcp_(dg[s]);
+    }
+    // forward: L y = P b; a row's y is final after its own step, where it is published
+#pragma unroll
+    for (int t = 0; t < MR; ++t) {
+      const int top = 32 * (t + 1) < NP ? 32 * (t + 1) : NP;
+#pragma unroll 1
+      for (int k0 = 32 * t; k0 < top; k0 += 4) {
+        Unit2<E> lv[MR];
+#pragma unroll
+        for (int s = t; s < MR; ++s) lv[s] = lds16(own[s] + k0 * 4, E());
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int kl = k0 + i - 32 * t;
+          if constexpr (NRHS == 1) {
+            const float y = __shfl_sync(kFull, LU ? b1[t] : div_by(b1[t], dg[t], dinv[t]), kl);
+            if (!LU) b1[t] = lane == kl ? y : b1[t];
+#pragma unroll
+            for (int s = t; s < MR; ++s) {
+              const float v = fma_(-U::get(i / 2 ? lv[s].y : lv[s].x, i % 2), y, b1[s]);
+              b1[s] = (s > t || lane > kl) ? v : b1[s];
+            }
+          } else {
+            if (lane == kl) {
+#pragma unroll
+              for (int c = 0; c < NU; c += 2) {
+                E v0 = b[t][c], v1 = b[t][c + 1];
+                if (!LU) {
+                  v0 = U::pack(div_by(U::get(v0, 0), dg[t], dinv[t]), div_by(U::get(v0, 1), dg[t], dinv[t]));
+                  v1 = U::pack(div_by(U::get(v1, 0), dg[t], dinv[t]), div_by(U::get(v1, 1), dg[t], dinv[t]));
+                }
+                sts16(xown[t] + c * 8, v0, v1);
+              }
+            }
+            __syncwarp();
+            E nl[MR];
+#pragma unroll
+            for (int s = t; s < MR; ++s) nl[s] = U::dup(-U::get(i / 2 ? lv[s].y : lv[s].x, i % 2));
+#pragma unroll
+            for (int c = 0; c < NU; c += 2) {
+              const Unit2<E> y = lds16(Xu + (k0 + i) * XB + c * 8, E());
+#pragma unroll
+              for (int s = t; s < MR; ++s) {
+                b[s][c] = U::fma(nl[s], y.x, b[s][c]);
+                b[s][c + 1] = U::fma(nl[s], y.y, b[s][c + 1]);
+              }
+            }
+          }
+        }
+      }
+    }
+    if constexpr (NRHS > 1) {
+#pragma unroll
+      for (int s = 0; s < MR; ++s)
+#pragma unroll
+        for (int c = 0; c < NU; c += 2) {
+          const Unit2<E> y = lds16(xown[s] + c * 8, E());
+          b[s][c] = y.x;
+          b[s][c + 1] = y.y;
+        }
+      __syncwarp();
+    }
+    // backward: U x = y (LU) or L^T x = y (Cholesky)
+#pragma unroll
+    for (int t = MR - 1; t >= 0; --t) {
+      const int top = 32 * (t + 1) < NP ? 32 * (t + 1) : NP;
+#pragma unroll 1
+      for (int k0 = top - 4; k0 >= 32 * t; k0 -= 4) {
+        float uv[MR][4];
+#pragma unroll
+        for (int s = 0; s <= t; ++s) {
+          if constexpr (LU) {
+            const float4 v = *reinterpret_cast<const float4*>(M + (own[s] - Mu) + k0 * 4);
+            uv[s][0] = v.x; uv[s][1] = v.y; uv[s][2] = v.z; uv[s][3] = v.w;
+          } else {
+            const int r = lane + 32 * s < NP ? lane + 32 * s : NP - 1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) uv[s][i] = *reinterpret_cast<const float*>(M + (k0 + i) * RS + r * 4);
+          }
+        }
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {
+          const int kl = k0 + i - 32 * t;
+          if constexpr (NRHS == 1) {
+            const float x = __shfl_sync(kFull, b1[t] * dinv[t], kl);
+#pragma unroll
+            for (int s = 0; s <= t; ++s) {
+              const float v = fma_(-uv[s][i], x, b1[s]);
+              b1[s] = (s < t || lane < kl) ? v : b1[s];
+            }
+            b1[t] = lane == kl ? x : b1[t];
+          } else {
+            if (lane == kl) {
+              const E dd = U::dup(dinv[t]);
+#pragma unroll
+              for (int c = 0; c < NU; c += 2) sts16(xown[t] + c * 8, U::mul(b[t][c], dd), U::mul(b[t][c + 1], dd));
+            }
+            __syncwarp();
+            E nu[MR];
+#pragma unroll
+            for (int s = 0; s <= t; ++s) nu[s] = U::dup(-uv[s][i]);
+#pragma unroll
+            for (int c = 0; c < NU; c += 2) {
+              const Unit2<E> x = lds16(Xu + (k0 + i) * XB + c * 8, E());
+#pragma unroll
+              for (int s = 0; s <= t; ++s) {
+                b[s][c] = U::fma(nu[s], x.x, b[s][c]);
+                b[s][c + 1] = U::fma(nu[s], x.y, b[s][c + 1]);
+              }
+            }
+          }
         }
       }
     }
@@ -107,9 +413,11 @@ __global__ void __launch_bounds__(128) trs_kernel(SolveArgs<T> p, FastDiv ndiv, 
     for (int s = 0; s < MR; ++s) {
       const int r = lane + 32 * s;
       if (r >= n) continue;
+      float* row = Bm + (long long)r * p.ldb;
+      const float* x = reinterpret_cast<const float*>(M + C::OFF_X + r * XB);
 #pragma unroll
       for (int c = 0; c < NRHS; ++c)
-        if (c < p.nrhs) p.B[bbase + (long long)r * p.ldb + c] = b[s][c];
+        if (c < p.nrhs) row[c] = NRHS == 1 ? b1[s] : x[c];
     }
     __syncwarp();
   }
