@@ -6,14 +6,19 @@
 // Per panel of 8 columns (k0 = 0, 8, ...):
 //   1. pivot steps in registers (lane l holds rows l and l + 32): argmax of |a| by a
 //      warp reduction on the high word of the key (exact tie-break only when two
-//      lanes share it), the winner's remaining panel row, reciprocal and position
-//      published in a shared-memory record, multipliers through that correctly
-//      rounded reciprocal, rank-1 update of the panel;
+//      candidates share it), the winner's remaining panel row and reciprocal published
+//      in a shared-memory record, multipliers through that correctly rounded reciprocal,
+//      rank-1 update of the panel. Positions are not tracked: pivots follow from the
+//      order of the winners (position_of, rows.cuh);
 //   2. U12: the panel's pivot rows on the trailing columns, one lane per column;
-//   3. trailing update A22 -= L21 U12 on 8 x 8 tiles: tile (I, J) covers logical
-//      positions j1 + 8I .. j1 + 8I + 7 (gathered through the position -> physical
-//      row map, so exactly the rows still active) and columns 8J .. 8J + 7, one
-//      m8n8k4 MMA per 4 columns of the panel (two per tile).
+//   3. trailing update A22 -= L21 U12 on 8 x 8 tiles: tile (I, J) covers the active rows
+//      8I .. 8I + 7 in physical order (gathered through a map of the rows still active)
+//      and columns 8J .. 8J + 7, one m8n8k4 MMA per 4 columns of the panel (two per
+//      tile).
+// The back substitution runs in blocks of 8 rows on the same instruction: the block is
+// solved by shuffles, then the rows above take it by tile products whose fragments count
+// the columns downwards, so every element keeps the chain of a column-oriented back
+// substitution.
 //
 // Exactness. mma.sync.m8n8k4 with float64 operands accumulates its four products in
 // k order as fused multiply-adds, d = fma(a3, b3, fma(a2, b2, fma(a1, b1,
@@ -25,7 +30,7 @@
 // bit-identical to the CPU backends. A zero-pivot step enters as a = -0, b = +0,
 // and fma(-0, +0, c) = c for every c, which is the reference's skipped column.
 #pragma once
-#include "blk.cuh"
+#include "rows.cuh"
 
 namespace tsdx {
 namespace dev {
@@ -78,9 +83,9 @@ struct TcCfg {
   static constexpr int RS = B::RS, MAT = B::MAT, MR = B::MR, NC = B::NC, NCP = B::NCP;
   static constexpr int PB = 8;
   static constexpr int NT = NP / 8 - 1;     // most row tiles below a panel
-  // ord[NP] (physical row retired at each step), pvs[NP] (pivots), pmap[NP] (position -> row),
-  // then the mbarrier of the bulk loads
-  static constexpr int OFF_BAR = (MAT + 3 * NP * 4 + 7) / 8 * 8;
+  // ord[NP] (physical row retired at each step), pmap[NP] (the active rows; before that,
+  // the winners' records), then the mbarrier of the bulk loads
+  static constexpr int OFF_BAR = (MAT + 2 * NP * 4 + 7) / 8 * 8;
   static constexpr int WARPB = (OFF_BAR + 8 + 15) / 16 * 16;
   static_assert(NP % 8 == 0 && NP >= 32 && NP <= 64, "one warp per matrix, two row slots at most");
   static_assert(NCP % 8 == 0, "columns in tiles of 8");
@@ -200,54 +205,65 @@ __device__ __forceinline__ void tc_update(unsigned char* M, const int* ord, cons
   __syncwarp();
 }
 
-// Back substitution over physical rows: lane l solves its rows l and l + 32 (at
-// positions pos[s]) with the right-hand sides that the factorization left in the
-// augmented columns. Step k (from the last position down): the row at position k
-// computes x_k = y_k * RN(1/u_kk) and broadcasts it; rows at positions below k take
-// y <- fma(-u(row, k), x_k, y) (predicated). A row's y is final after its own step,
-// so every row forms its x = y * RN(1/u_kk) once more at the end, the same product.
-// These are the operations of a column-oriented back substitution over positions,
-// without its per-step selects.
+// Back substitution in blocks of 8 positions, from the last one down, on the right-hand
+// sides that the factorization left in the augmented columns (one tile of 8 columns,
+// zero past NRHS). Lane (fr, fq) holds columns 2 fq, 2 fq + 1 of position 8 I + fr of every
+// block I. Step k of a block: the lanes of its row form x_k = y_k * RN(1/u_kk) and
+// broadcast it, the rows above it in the block take y <- fma(-u, x_k, y); the blocks above
+// take the 8 steps as two MMAs with the columns counted downwards, the same fused
+// multiply-adds in the same order.
 template <int NP, int NRHS>
-__device__ __forceinline__ void tc_backsolve(const unsigned char* M, const int* ord, const int (&pos)[TcCfg<NP, NRHS>::MR],
-                                             const MatJob<double>& j, int lane) {
+__device__ __forceinline__ void tc_backsolve(const unsigned char* M, const int* ord, const MatJob<double>& j, int lane) {
   using C = TcCfg<NP, NRHS>;
-  constexpr int MR = C::MR, RS = C::RS;
-  double y[MR][NRHS], dv[MR];
-  const unsigned char* rowp[MR];
+  constexpr int RS = C::RS, NB = NP / 8;
+  const int fr = lane >> 2, fq = lane & 3;
+  const unsigned char* row[NB];
+  double2 y[NB];
 #pragma unroll
-  for (int s = 0; s < MR; ++s) {
-    const int r = lane + 32 * s;
-    const int rr = r < NP ? r : 0;
-    rowp[s] = M + rr * RS;
-    dv[s] = rcp_(*reinterpret_cast<const double*>(rowp[s] + (r < NP ? pos[s] : 0) * 8));
-#pragma unroll
-    for (int c = 0; c < NRHS; ++c) y[s][c] = *reinterpret_cast<const double*>(rowp[s] + (NP + c) * 8);
+  for (int I = 0; I < NB; ++I) {
+    row[I] = M + ord[8 * I + fr] * RS;
+    y[I] = *reinterpret_cast<const double2*>(row[I] + (NP + 2 * fq) * 8);
   }
-#pragma unroll 4
-  for (int k = NP - 1; k >= 0; --k) {
-    const int po = ord[k];
-    const bool mine0 = MR == 1 || pos[0] == k;
-    const double d = mine0 ? dv[0] : dv[MR - 1];
-    double x[NRHS];
 #pragma unroll
-    for (int c = 0; c < NRHS; ++c) x[c] = __shfl_sync(kFull, (mine0 ? y[0][c] : y[MR - 1][c]) * d, po & 31);
+  for (int K = NB - 1; K >= 0; --K) {
+    double u[8];
 #pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const double u = *reinterpret_cast<const double*>(rowp[s] + k * 8);
-      const bool below = pos[s] < k;
+    for (int q = 0; q < 8; q += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(row[K] + (8 * K + q) * 8);
+      u[q] = v.x;
+      u[q + 1] = v.y;
+    }
+    const double d = rcp_(*reinterpret_cast<const double*>(row[K] + (8 * K + fr) * 8));
 #pragma unroll
-      for (int c = 0; c < NRHS; ++c) fma_if(y[s][c], below, u, x[c]);
+    for (int q = 7; q >= 0; --q) {
+      y[K].x = fr == q ? y[K].x * d : y[K].x;
+      y[K].y = fr == q ? y[K].y * d : y[K].y;
+      if (q == 0) continue;
+      const double xx = __shfl_sync(kFull, y[K].x, 4 * q + fq), xy = __shfl_sync(kFull, y[K].y, 4 * q + fq);
+      y[K].x = fr < q ? fma_(-u[q], xx, y[K].x) : y[K].x;
+      y[K].y = fr < q ? fma_(-u[q], xy, y[K].y) : y[K].y;
+    }
+    if (K > 0) {
+      // B fragments: x of rows 7 - fq and 3 - fq of the block, column fr
+      const int s0 = 4 * (7 - fq) + (fr >> 1), s1 = 4 * (3 - fq) + (fr >> 1);
+      const double p0 = __shfl_sync(kFull, y[K].x, s0), q0 = __shfl_sync(kFull, y[K].y, s0);
+      const double p1 = __shfl_sync(kFull, y[K].x, s1), q1 = __shfl_sync(kFull, y[K].y, s1);
+      const double b0 = (fr & 1) ? q0 : p0, b1 = (fr & 1) ? q1 : p1;
+#pragma unroll
+      for (int I = 0; I < K; ++I) {
+        dmma_m8n8k4(y[I], -*reinterpret_cast<const double*>(row[I] + (8 * K + 7 - fq) * 8), b0);
+        dmma_m8n8k4(y[I], -*reinterpret_cast<const double*>(row[I] + (8 * K + 3 - fq) * 8), b1);
+      }
     }
   }
   if (j.live && j.B) {
 #pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      if (pos[s] >= j.n) continue;
-      double* brow = j.B + (long long)pos[s] * j.ldb + j.b0;
-#pragma unroll
-      for (int c = 0; c < NRHS; ++c)
-        if (c < j.nrhs) brow[c] = y[s][c] * dv[s];
+    for (int I = 0; I < NB; ++I) {
+      const int i = 8 * I + fr;
+      if (i >= j.n) continue;
+      double* brow = j.B + (long long)i * j.ldb + j.b0;
+      if (2 * fq < j.nrhs) brow[2 * fq] = y[I].x;
+      if (2 * fq + 1 < j.nrhs) brow[2 * fq + 1] = y[I].y;
     }
   }
 }
@@ -260,8 +276,7 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
   using T = double;
   constexpr int MR = C::MR, PB = C::PB, NC = C::NC, NCP = C::NCP, RS = C::RS, NT = C::NT;
   int* ord = reinterpret_cast<int*>(M + C::MAT);
-  int* pvs = ord + NP;
-  int* pmap = pvs + NP;
+  int* pmap = ord + NP;
   auto at = [&](int r, int c) -> T& { return *reinterpret_cast<T*>(M + r * RS + c * 8); };
   auto vat = [&](int r, int c) -> double2& { return *reinterpret_cast<double2*>(M + r * RS + c * 8); };
 
@@ -319,14 +334,10 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
     for (int c = NC; c < NCP; ++c) at(r, c) = 0.0;
   }
   __syncwarp();
-  int pos[MR];
-  bool act[MR];
+  using D = DivRange<double>;
+  unsigned act[MR];  // key mask of the lane's rows, 0 once retired
 #pragma unroll
-  for (int s = 0; s < MR; ++s) {
-    const int r = lane + 32 * s;
-    act[s] = r < NP;
-    pos[s] = r < NP ? r : 0x3fffffff;
-  }
+  for (int s = 0; s < MR; ++s) act[s] = lane + 32 * s < NP ? 0x7fffffffu : 0u;
   int info = 0;
 
   for (int k0 = 0; k0 < NP; k0 += PB) {
@@ -344,54 +355,65 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
       }
     }
     unsigned zb = 0;
+    // the winner's record (panel row, reciprocal) in the map's area, which is free until the
+    // panel's map is written
+    T* rec = reinterpret_cast<T*>(pmap);
+    static_assert(NP * 4 >= 9 * 8, "the record fits the map");
 #pragma unroll
     for (int i = 0; i < PB; ++i) {
       const int k = k0 + i;
-      unsigned long long bk = 0;
-      int bp = 0x7fffffff, bs = 0;
+      unsigned key[MR], m = 0, b[MR];
+      bool win[MR];
+      T cand = T(1);
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
-        const T v = pan[s][i];
-        const unsigned long long key = isnan(v) ? (pos[s] == k ? ~0ull : 0ull) : key_bits(v) + 1;
-        const bool better = act[s] && (key > bk || (key == bk && pos[s] < bp));
-        bk = better ? key : bk;
-        bp = better ? pos[s] : bp;
-        bs = better ? s : bs;
+        key[s] = hi_word(pan[s][i]) & act[s];
+        cand = key[s] > m ? pan[s][i] : cand;
+        m = max(m, key[s]);
       }
-      const unsigned hi = (unsigned)(bk >> 32);
-      const unsigned mhi = __reduce_max_sync(kFull, hi);
-      // while the reduction runs: the reciprocal of this lane's candidate (the winner
-      // publishes it with its row)
-      const T rcand = rcp_((MR > 1 && bs) ? pan[MR - 1][i] : pan[0][i]);
-      const unsigned bal = __ballot_sync(kFull, hi == mhi);
-      int wl;
-      bool zero;
-      if (__popc(bal) == 1) {  // one lane holds the largest high word: it wins
-        wl = __ffs(bal) - 1;
-        zero = false;
-      } else {                 // exact tie-break on the full key, then the position
-        const unsigned lo = (unsigned)bk;
-        const unsigned mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-        zero = (mhi == 0u && mlo == 1u);
-        const int bx = __reduce_min_sync(kFull, (hi == mhi && lo == mlo) ? bp : 0x7fffffff);
-        wl = __ffs(__ballot_sync(kFull, bp == bx)) - 1;
-      }
-      // the winner's record (80 bytes: panel row, reciprocal, position) in the
-      // position-map area, which is free until the panel's map is written
-      T* rec = reinterpret_cast<T*>(pmap);
-      static_assert(NP * 4 >= 10 * 8, "the record fits the position map");
-      if (lane == wl) {
+      m = __reduce_max_sync(kFull, m);
+      T rcand = rcp_in_range(cand);  // of this lane's candidate, while the reduction runs
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {  // stored from the candidate's slot: predicated stores, no selects
-          if (bs != s) continue;
+      for (int s = 0; s < MR; ++s) {
+        win[s] = key[s] == m;
+        b[s] = __ballot_sync(kFull, win[s]);
+      }
+      Seg g;
+      g.lane = lane;
+      g.segbase = 0;
+      int wr;
+      const bool one = one_row<32, MR>(b, g, wr);
+      bool zero = false;
+      // rare, by the whole warp: a tie, or a column whose largest entry is zero, tiny,
+      // huge, infinite or NaN
+      const bool odd = !one || m - D::kLo > D::kHi - D::kLo;
+      if (odd) {
+        Candidates<T, MR> c;
+#pragma unroll
+        for (int s = 0; s < MR; ++s) {
+          c.v[s] = pan[s][i];
+          c.act[s] = act[s];
+        }
+        const Choice w = exact_pivot<T, MR, 32>(c, ord, k, lane);
+#pragma unroll
+        for (int s = 0; s < MR; ++s) {
+          win[s] = w.slot == s;
+          cand = win[s] ? pan[s][i] : cand;
+        }
+        wr = w.row;
+        zero = w.zero;
+        rcand = rcp_(cand);
+      }
+#pragma unroll
+      for (int s = 0; s < MR; ++s) {
+        if (win[s]) {
 #pragma unroll
           for (int jj = i & ~1; jj < PB; jj += 2)
             *reinterpret_cast<double2*>(rec + jj) = make_double2(pan[s][jj], pan[s][jj + 1]);
+          rec[8] = rcand;
+          ord[k] = wr;
+          act[s] = 0u;
         }
-        rec[8] = rcand;
-        reinterpret_cast<int*>(rec + 9)[0] = bp;
-        ord[k] = lane + 32 * bs;
-        pvs[k] = bp;
       }
       __syncwarp();
       T uw[PB];
@@ -402,39 +424,28 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
         uw[jj + 1] = v.y;
       }
       const T ry = rec[8];
-      const int bpos = reinterpret_cast<const int*>(rec + 9)[0];
       __syncwarp();  // all reads done before the next step's record
-      // retire the winner and replay the reference's swap of positions k and bpos
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const bool win = pos[s] == bpos;  // retired rows hold positions below k <= bpos
-        pos[s] = win ? k : (pos[s] == k ? bpos : pos[s]);
-        act[s] = act[s] && !win;
-      }
-      info = (zero && info == 0) ? k + 1 : info;
       if (zero) {
+        info = info == 0 ? k + 1 : info;
         zb |= 1u << i;
       } else {
-        // l = a / pivot by the shared reciprocal with Markstein's correction (div_by),
-        // both rows at once; operands outside its range take the IEEE division on a
-        // warp-uniform rare path
+        // l = a / pivot by the shared reciprocal with Markstein's correction; operands
+        // outside its range take the IEEE division on a warp-uniform rare path
         const T vpk = uw[i];
         T l[MR];
-        bool slow = false;
+        bool slow = odd;
 #pragma unroll
         for (int s = 0; s < MR; ++s) {
           const T a = pan[s][i];
           const T q = __dmul_rn(a, ry);
-          const T aq = fabs(q), aa = fabs(a);
-          const bool ok = aq >= 0x1p-960 && aq <= 0x1p+960 && aa >= 0x1p-960 && aa <= 0x1p+960;
-          const T e = __fma_rn(-vpk, q, a);
-          l[s] = ok ? __fma_rn(e, ry, q) : q;  // a zero numerator: q is IEEE's signed zero
-          slow = slow || (act[s] && !ok && !(a == 0.0 && q == 0.0));
+          l[s] = __fma_rn(__fma_rn(-vpk, q, a), ry, q);
+          slow = slow || D::outside(a, D::kLo);
         }
         if (__any_sync(kFull, slow)) {
 #pragma unroll
-          for (int s = 0; s < MR; ++s) l[s] = act[s] ? div_by(pan[s][i], vpk, ry) : l[s];
+          for (int s = 0; s < MR; ++s) l[s] = act[s] ? div_slow(pan[s][i], vpk) : T(0);
         }
+        // a retired row keeps its U; the rows of this step's multipliers take the update
 #pragma unroll
         for (int s = 0; s < MR; ++s) {
           if (act[s]) {
@@ -445,14 +456,20 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
         }
       }
     }
-    __syncwarp();  // every lane has read the last record before the position map is written
+    // the panel back to its rows, and the map of the rows still active
+    unsigned ab[MR];
+#pragma unroll
+    for (int s = 0; s < MR; ++s) ab[s] = __ballot_sync(kFull, act[s] != 0);
+    int before = 0;
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
       const int r = lane + 32 * s;
-      if (r >= NP) continue;
+      if (r < NP) {
 #pragma unroll
-      for (int i0 = 0; i0 < PB; i0 += 2) vat(r, k0 + i0) = make_double2(pan[s][i0], pan[s][i0 + 1]);
-      if (act[s]) pmap[pos[s]] = r;
+        for (int i0 = 0; i0 < PB; i0 += 2) vat(r, k0 + i0) = make_double2(pan[s][i0], pan[s][i0 + 1]);
+        if (act[s]) pmap[k0 + PB + before + __popc(ab[s] & ((1u << lane) - 1u))] = r;
+      }
+      before += __popc(ab[s]);
     }
     __syncwarp();
     const int j1 = k0 + PB;
@@ -464,13 +481,13 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
     else tc_update<NP, NRHS, true>(M, ord, pmap, zb, k0, lane);
   }
 
-  if constexpr (NRHS > 0) tc_backsolve<NP, NRHS>(M, ord, pos, j, lane);
+  if constexpr (NRHS > 0) tc_backsolve<NP, NRHS>(M, ord, j, lane);
   if (j.live) {
     if (j.piv) {
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
         const int k = lane + 32 * s;
-        if (k < j.n) j.piv[k] = pvs[k];
+        if (k < j.n) j.piv[k] = position_of(ord, ord[k], k);
       }
     }
     if (lane == 0 && j.info) *j.info = info;
@@ -486,7 +503,7 @@ template <int NP, int NRHS, int WPC>
 __global__ void __launch_bounds__(WPC * 32, 1) tc_kernel(SolveArgs<double> p) {
   using C = TcCfg<NP, NRHS>;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   unsigned char* M = smem + warp * C::WARPB;
   const long long nn = (long long)p.n * p.n;
   const long long step = (long long)gridDim.x * WPC;
