@@ -1,6 +1,8 @@
 // C-ABI of the GPU error metrics (metrics.cuh). Device pointers, stream-ordered.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/tsdx_cuda.h"
 #include "launch.cuh"
 #include "metrics.cuh"
@@ -9,8 +11,8 @@
 
 namespace {
 using namespace tsdx;
-constexpr int kWpc = 6;
-constexpr int kFactorSmem = kWpc * (64 * dev::kMetStride * (int)sizeof(double) + 64 * (int)sizeof(int));
+// warps per CTA: one matrix each, as many as shared memory holds, at most 16
+int warps_for(int warp_bytes) { return std::max(1, std::min(16, 227 * 1024 / warp_bytes)); }
 
 int finish(const char* what) {
   const cudaError_t e = cudaGetLastError();
@@ -33,10 +35,11 @@ int factor_metric(const double* A, const double* F, const int* piv, int n, int64
   if (int rc = check(n, batch)) return rc;
   if (batch == 0) return TSDX_OK;
   if (!A || !F || !out || (!CHOL && !piv)) return TSDX_ERR_NULL;
-  auto kern = dev::factor_bwd_kernel<kWpc, CHOL>;
-  if (int rc = host::prepare(kern, kFactorSmem)) return rc;
-  const int grid = host::grid_for(kern, kFactorSmem, (batch + kWpc - 1) / kWpc, kWpc * 32);
-  kern<<<grid, kWpc * 32, kFactorSmem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
+  auto kern = dev::factor_bwd_kernel<CHOL>;
+  const int wpc = warps_for(dev::met_factor_bytes(n)), smem = wpc * dev::met_factor_bytes(n);
+  if (int rc = host::prepare(kern, smem)) return rc;
+  const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
+  kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
   return finish(CHOL ? "cholesky backward error kernel" : "lu backward error kernel");
 }
 }  // namespace
@@ -46,9 +49,11 @@ API int tsdx_cuda_solve_backward_error_f64(const double* A, const double* x, con
   if (int rc = check(n, batch)) return rc;
   if (batch == 0) return TSDX_OK;
   if (!A || !x || !b || !out) return TSDX_ERR_NULL;
-  auto kern = dev::solve_bwd_kernel<8>;
-  const int grid = host::grid_for(kern, 0, (batch + 7) / 8, 256);
-  kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);
+  auto kern = dev::solve_bwd_kernel;
+  const int wpc = warps_for(dev::met_solve_bytes(n)), smem = wpc * dev::met_solve_bytes(n);
+  if (int rc = host::prepare(kern, smem)) return rc;
+  const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
+  kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);
   return finish("solve backward error kernel");
 }
 

@@ -10,11 +10,20 @@
 // about 106 significand bits, more than the reference's x87 long double (64), so
 // the sums of products here are at least as accurate as the reference's. The
 // building blocks are the published error-free transformations: TwoSum (Knuth,
-// TAOCP vol. 2, 4.2.2), TwoProduct with a fused multiply-add, and the
-// double-double additions of Hida, Li and Bailey ("Algorithms for quad-double
-// precision floating point arithmetic", ARITH-15, 2001).
+// TAOCP vol. 2, 4.2.2), TwoProduct with a fused multiply-add, sums of products by
+// Dot2 (Ogita, Rump and Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput.
+// 26(6), 2005: as accurate as in twice the working precision, 10 operations a
+// product), and the double-double additions of Hida, Li and Bailey ("Algorithms for
+// quad-double precision floating point arithmetic", ARITH-15, 2001) across lanes.
+//
+// What bounds them: the factor metrics are FP64 arithmetic (n^3 / 3 products at 10
+// operations), the solve metric reads A once. The matrix is staged in shared memory
+// (cp.async, coalesced) in rows of an odd number of 16-byte units, so that a lane per row
+// reads two columns at a time without bank conflicts.
 #pragma once
 #include <cuda_runtime.h>
+
+#include "rows.cuh"
 
 namespace tsdx {
 namespace dev {
@@ -41,19 +50,26 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
   s.lo = __dadd_rn(s.lo, t.lo);
   return fast_two_sum(s.hi, s.lo);
 }
-// a + x*y with the product taken exactly (TwoProduct by FMA)
-__device__ __forceinline__ DD dd_fma(DD a, double x, double y) {
-  const double p = __dmul_rn(x, y);
-  const double e = __fma_rn(x, y, -p);
-  return dd_add(a, DD{p, e});
+// A sum of products: hi is the rounded running sum, lo the errors of its additions and
+// products.
+struct Dot2 {
+  double hi, lo;
+  __device__ __forceinline__ void add(double p, double e) {  // p + e, |e| an error term of p
+    const DD t = two_sum(hi, p);
+    hi = t.hi;
+    lo = __dadd_rn(lo, __dadd_rn(t.lo, e));
+  }
+  __device__ __forceinline__ void fma(double x, double y) {
+    const double p = __dmul_rn(x, y);
+    add(p, __fma_rn(x, y, -p));
+  }
+  __device__ __forceinline__ DD value() const { return two_sum(hi, lo); }
+};
+// + d^2
+__device__ __forceinline__ void add_square(Dot2& a, DD d) {
+  const double p = __dmul_rn(d.hi, d.hi);
+  a.add(p, __fma_rn(__dmul_rn(2.0, d.hi), d.lo, __fma_rn(d.hi, d.hi, -p)));
 }
-__device__ __forceinline__ DD dd_sqr(DD a) {
-  const double p = __dmul_rn(a.hi, a.hi);
-  double e = __fma_rn(a.hi, a.hi, -p);
-  e = __fma_rn(__dmul_rn(2.0, a.hi), a.lo, e);
-  return fast_two_sum(p, e);
-}
-__device__ __forceinline__ DD dd_neg(DD a) { return {-a.hi, -a.lo}; }
 __device__ __forceinline__ DD dd_warp_sum(DD v) {
   for (int o = 16; o > 0; o >>= 1) {
     DD w;
@@ -65,96 +81,158 @@ __device__ __forceinline__ DD dd_warp_sum(DD v) {
 }
 __device__ __forceinline__ double dd_sqrt(DD a) { return sqrt(__dadd_rn(a.hi, a.lo)); }
 
-constexpr int kMetStride = 65;  // doubles per staged factor row (n <= 64)
+// Shared-memory row of an order-n matrix: an odd number of 16-byte units.
+__host__ __device__ constexpr int met_row_bytes(int n) { return (((n + 1) / 2) | 1) * 16; }
+__host__ __device__ constexpr int met_factor_bytes(int n) { return n * met_row_bytes(n) + 64 * 4; }  // + pivots
+__host__ __device__ constexpr int met_solve_bytes(int n) { return n * met_row_bytes(n) + 64 * 8; }   // + x
+
+// Stages an n x n matrix; a last odd column is paired with zero.
+__device__ __forceinline__ void met_stage(unsigned char* M, const double* A, int n, int rs, int lane) {
+  const int rowb = n * 8;
+  const char* src = reinterpret_cast<const char*>(A);
+  if (vec_of<double>(A, n) == 16) walk_chunks<double, 64, 32, 16>(n, lane, [&](int r, int c) { cp_async<16>(M + r * rs + c * 16, src + r * rowb + c * 16); });
+  else walk_chunks<double, 64, 32, 8>(n, lane, [&](int r, int c) { cp_async<8>(M + r * rs + c * 8, src + r * rowb + c * 8); });
+  cp_async_commit();
+  if (n & 1)
+    for (int r = lane; r < n; r += 32) *reinterpret_cast<double*>(M + r * rs + rowb) = 0.0;
+}
 
 // ||b - A x|| / (||A||_F ||x|| + ||b||); lane i owns rows i and i + 32.
-template <int WPC>
-__global__ void __launch_bounds__(WPC * 32) solve_bwd_kernel(const double* __restrict__ A, const double* __restrict__ x,
-                                                             const double* __restrict__ b, int n, long long batch,
-                                                             double* out) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (long long m = (long long)blockIdx.x * WPC + warp; m < batch; m += (long long)gridDim.x * WPC) {
-    const double* a = A + m * n * n;
-    const double* xv = x + m * n;
-    const double* rhs = b + m * n;
-    DD num{0, 0}, fa{0, 0}, fx{0, 0}, fb{0, 0};
+__global__ void __launch_bounds__(512) solve_bwd_kernel(const double* __restrict__ A, const double* __restrict__ x,
+                                                        const double* __restrict__ b, int n, long long batch,
+                                                        double* out) {
+  extern __shared__ __align__(16) unsigned char met_smem[];
+  const int wpc = blockDim.x >> 5, warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rs = met_row_bytes(n);
+  unsigned char* M = met_smem + warp * met_solve_bytes(n);
+  double* xs = reinterpret_cast<double*>(M + n * rs);
+  const long long step = (long long)gridDim.x * wpc;
+  for (long long m = (long long)blockIdx.x * wpc + warp; m < batch; m += step) {
+    if (lane == 0 && m + step < batch) prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
+    met_stage(M, A + m * n * n, n, rs, lane);
+    Dot2 fx{0, 0}, fb{0, 0}, num{0, 0}, fa[2] = {{0, 0}, {0, 0}}, r[2] = {{0, 0}, {0, 0}};
+#pragma unroll
     for (int s = 0; s < 2; ++s) {
       const int i = lane + 32 * s;
-      if (i < n) {
-        DD r{rhs[i], 0};
-        const double* row = a + (long long)i * n;
-        for (int j = 0; j < n; ++j) {
-          const double v = row[j];
-          r = dd_fma(r, -v, xv[j]);
-          fa = dd_fma(fa, v, v);
-        }
-        num = dd_add(num, dd_sqr(r));
-        fx = dd_fma(fx, xv[i], xv[i]);
-        fb = dd_fma(fb, rhs[i], rhs[i]);
+      const double xi = i < n ? x[m * n + i] : 0.0;
+      xs[i] = xi;  // zero from n on: the partner of a last odd column
+      r[s].hi = i < n ? b[m * n + i] : 0.0;
+      fx.fma(xi, xi);
+      fb.fma(r[s].hi, r[s].hi);
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    const unsigned char* row0 = M + (lane < n ? lane : 0) * rs;
+    const unsigned char* row1 = M + (lane + 32 < n ? lane + 32 : 0) * rs;
+#pragma unroll 2
+    for (int j = 0; j < n; j += 2) {
+      const double2 a0 = *reinterpret_cast<const double2*>(row0 + j * 8);
+      const double x0 = -xs[j], x1 = -xs[j + 1];
+      r[0].fma(a0.x, x0);
+      r[0].fma(a0.y, x1);
+      fa[0].fma(a0.x, a0.x);
+      fa[0].fma(a0.y, a0.y);
+      if (n > 32) {
+        const double2 a1 = *reinterpret_cast<const double2*>(row1 + j * 8);
+        r[1].fma(a1.x, x0);
+        r[1].fma(a1.y, x1);
+        fa[1].fma(a1.x, a1.x);
+        fa[1].fma(a1.y, a1.y);
       }
     }
-    num = dd_warp_sum(num);
-    fa = dd_warp_sum(fa);
-    fx = dd_warp_sum(fx);
-    fb = dd_warp_sum(fb);
-    if (lane == 0) out[m] = dd_sqrt(num) / (dd_sqrt(fa) * dd_sqrt(fx) + dd_sqrt(fb));
+    DD f{0, 0};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      if (lane + 32 * s >= n) continue;
+      add_square(num, r[s].value());
+      f = dd_add(f, fa[s].value());
+    }
+    const DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(f), sx = dd_warp_sum(fx.value()), sb = dd_warp_sum(fb.value());
+    if (lane == 0) out[m] = dd_sqrt(sn) / (dd_sqrt(sa) * dd_sqrt(sx) + dd_sqrt(sb));
+    __syncwarp();
   }
 }
 
 // ||P A - L U||_F / ||A||_F (LU packed, unit L) or ||A - L L^T||_F / ||A||_F: the
-// factor is staged in shared memory, lane i owns rows i and i + 32 of the product.
-template <int WPC, bool CHOL>
-__global__ void __launch_bounds__(WPC * 32) factor_bwd_kernel(const double* __restrict__ A,
-                                                              const double* __restrict__ F, const int* __restrict__ piv,
-                                                              int n, long long batch, double* out) {
-  extern __shared__ __align__(16) double msm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* S = msm + warp * 64 * kMetStride;
-  int* perm = reinterpret_cast<int*>(msm + WPC * 64 * kMetStride) + warp * 64;
-  for (long long m = (long long)blockIdx.x * WPC + warp; m < batch; m += (long long)gridDim.x * WPC) {
+// factor is staged in shared memory, lane i owns rows i and i + 32 of the product, two
+// columns at a time. Products beyond min(i, j) enter with a zero multiplier.
+template <bool CHOL>
+__global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restrict__ A, const double* __restrict__ F,
+                                                         const int* __restrict__ piv, int n, long long batch,
+                                                         double* out) {
+  extern __shared__ __align__(16) unsigned char met_smem[];
+  const int wpc = blockDim.x >> 5, warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rs = met_row_bytes(n);
+  unsigned char* M = met_smem + warp * met_factor_bytes(n);
+  int* pv = reinterpret_cast<int*>(M + n * rs);
+  const long long step = (long long)gridDim.x * wpc;
+  for (long long m = (long long)blockIdx.x * wpc + warp; m < batch; m += step) {
     const double* a = A + m * n * n;
-    const double* f = F + m * n * n;
-    for (int r = 0; r < n; ++r)
-      for (int c = lane; c < n; c += 32) S[r * kMetStride + c] = f[(long long)r * n + c];
-    if (!CHOL && lane == 0) {
-      // row i of P A is row perm[i] of A (the sequential swaps of the pivots)
-      for (int i = 0; i < n; ++i) perm[i] = i;
-      const int* pv = piv + m * n;
-      for (int k = 0; k < n; ++k) {
+    if (lane == 0 && m + step < batch) {
+      prefetch_l2(F + (m + step) * n * n, (long long)n * n * 8);
+      prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
+    }
+    met_stage(M, F + m * n * n, n, rs, lane);
+    int src[2] = {lane, lane + 32};  // the row of A behind each row of P A
+    if constexpr (!CHOL) {
+      for (int k = lane; k < n; k += 32) pv[k] = piv[m * n + k];
+      __syncwarp();
+      // the sequential swaps, followed backwards for every row at once
+      for (int k = n - 1; k >= 0; --k) {
         const int p = pv[k];
-        if (p >= 0 && p < n) {
-          const int t = perm[k];
-          perm[k] = perm[p];
-          perm[p] = t;
-        }
+        if (p < 0 || p >= n) continue;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) src[s] = src[s] == k ? p : (src[s] == p ? k : src[s]);
       }
     }
+    cp_async_wait<0>();
     __syncwarp();
-    DD num{0, 0}, fa{0, 0};
+    Dot2 num{0, 0}, fa{0, 0};
+#pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const int i = lane + 32 * s;
-      if (i >= n) continue;
-      const double* arow = a + (long long)(CHOL ? i : perm[i]) * n;
-      for (int j = 0; j < n; ++j) {
-        DD acc{0, 0};
-        const int kmax = i < j ? i : j;
-        for (int k = 0; k <= kmax; ++k) {
-          if (CHOL) {
-            acc = dd_fma(acc, S[i * kMetStride + k], S[j * kMetStride + k]);
+      if (32 * s >= n) break;
+      const int i = lane + 32 * s, last = min(n - 1, 32 * s + 31);  // the slot's last row
+      const bool live = i < n;
+      const unsigned char* row = M + (live ? i : 0) * rs;
+      const double* arow = a + (long long)(live ? src[s] : 0) * n;
+      for (int j = 0; j < n; j += 2) {
+        const bool two = j + 1 < n;
+        const double a0 = arow[j], a1 = two ? arow[j + 1] : 0.0;
+        Dot2 d0{a0, 0}, d1{a1, 0};
+        const int kend = min(last, j + 1);
+#pragma unroll 2
+        for (int k = 0; k <= kend; k += 2) {
+          // -L(i, k), -L(i, k + 1): zero past the diagonal, one on it (LU)
+          const double2 l = *reinterpret_cast<const double2*>(row + k * 8);
+          const double l0 = k > i ? 0.0 : (!CHOL && k == i ? -1.0 : -l.x);
+          const double l1 = k + 1 > i ? 0.0 : (!CHOL && k + 1 == i ? -1.0 : -l.y);
+          double2 u0, u1;  // U(k, j..j+1), U(k + 1, j..j+1), zero below the diagonal
+          if constexpr (CHOL) {
+            const double2 lj = *reinterpret_cast<const double2*>(M + j * rs + k * 8);
+            const double2 lj1 = *reinterpret_cast<const double2*>(M + (two ? j + 1 : j) * rs + k * 8);
+            u0 = make_double2(lj.x, lj1.x);
+            u1 = make_double2(lj.y, lj1.y);
           } else {
-            const double lik = (k == i) ? 1.0 : S[i * kMetStride + k];
-            acc = dd_fma(acc, lik, S[k * kMetStride + j]);
+            u0 = *reinterpret_cast<const double2*>(M + k * rs + j * 8);
+            u1 = *reinterpret_cast<const double2*>(M + (k + 1 < n ? k + 1 : k) * rs + j * 8);
+          }
+          d0.fma(l0, u0.x);               // k <= j: k is even, j is even and k <= j + 1
+          d1.fma(l0, u0.y);
+          d0.fma(l1, k + 1 > j ? 0.0 : u1.x);
+          d1.fma(l1, u1.y);
+        }
+        if (live) {
+          add_square(num, d0.value());
+          fa.fma(a0, a0);
+          if (two) {
+            add_square(num, d1.value());
+            fa.fma(a1, a1);
           }
         }
-        const double av = arow[j];
-        const DD d = dd_add(DD{av, 0}, dd_neg(acc));
-        num = dd_add(num, dd_sqr(d));
-        fa = dd_fma(fa, av, av);
       }
     }
-    num = dd_warp_sum(num);
-    fa = dd_warp_sum(fa);
-    if (lane == 0) out[m] = dd_sqrt(num) / dd_sqrt(fa);
+    const DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(fa.value());
+    if (lane == 0) out[m] = dd_sqrt(sn) / dd_sqrt(sa);
     __syncwarp();
   }
 }
