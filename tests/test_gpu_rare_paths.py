@@ -82,3 +82,19 @@ def test_solves_from_factor(oracle, n, nrhs, dtype):
         num = np.linalg.norm(B64 - M64 @ X, axis=1)
         den = np.linalg.norm(M64, axis=(1, 2))[:, None] * np.linalg.norm(X, axis=1) + np.linalg.norm(B64, axis=1)
         assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
+
+
+@pytest.mark.parametrize("batch", [1, 63, 64, 65, 600])
+def test_training_gradient_of_partial_blocks(batch):
+    """Against float64: float32 sums of at most 600 samples over 64 units carry a few
+    hundred roundings of 2^-24 of the largest term; 2e-5 of the largest entry bounds them."""
+    from oracle import selector_ref as R
+    sel = load_pkg("selector")
+    r = np.random.default_rng(batch)
+    X = (r.standard_normal((batch, 24)) * 2 + 1).astype(np.float32)
+    y = r.integers(0, 4, batch).astype(np.int8)
+    s = sel.Selector(seed=3)
+    grad, loss = s.loss_grad(dev(X), dev(y), torch.tensor([1.0, 2.0, 0.5, 0.7]))
+    lo, g = R.loss_and_grad(s.params.cpu().numpy(), s.norm.cpu().numpy(), X, y, np.array([1.0, 2.0, 0.5, 0.7]))
+    assert np.abs(grad.cpu().numpy() - g).max() <= 2e-5 * np.abs(g).max()
+    assert abs(float(loss) - float(lo)) <= 2e-5 * abs(float(lo))

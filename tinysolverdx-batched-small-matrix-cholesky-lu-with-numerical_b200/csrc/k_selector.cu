@@ -35,7 +35,7 @@ API int tsdx_cuda_selector_features_f64(const double* A, int n, int64_t batch, c
   if (batch < 0) return TSDX_ERR_BATCH;
   if (batch == 0) return TSDX_OK;
   if (!A || !features) return TSDX_ERR_NULL;
-  auto kern = dev::features_kernel<kFeatWpc>;
+  auto kern = n <= 32 ? dev::features_kernel<kFeatWpc, 1> : dev::features_kernel<kFeatWpc, 2>;
   const int grid = host::grid_for(kern, kFeatSmem, (batch + kFeatWpc - 1) / kFeatWpc, kFeatWpc * 32);
   kern<<<grid, kFeatWpc * 32, kFeatSmem, static_cast<cudaStream_t>(stream)>>>(A, n, batch, kind, kind_all, features);
   return finish("features kernel");
@@ -70,7 +70,7 @@ API int tsdx_cuda_mlp_grad(const float* params, const float* norm, const float* 
   dev::mlp_train_kernel<<<(unsigned)blocks, dev::kTrainThreads, kTrainSmem, st>>>(params, norm, features, label,
                                                                                 class_weight, batch, part);
   if (int rc = finish("mlp train kernel")) return rc;
-  dev::grad_reduce_kernel<<<(dev::kParams + 1 + 255) / 256, 256, 0, st>>>(part, (int)blocks, grad, loss);
+  dev::grad_reduce_kernel<<<(dev::kParams + 1 + 31) / 32, 256, 0, st>>>(part, (int)blocks, grad, loss);
   return finish("gradient reduce kernel");
 }
 
