@@ -127,12 +127,19 @@ int tsdx_cuda_posv_ir_f64(const double* A, int n, int64_t batch, double* B, cons
 /* ---- emulated fp16 / bf16 on the GPU (host pointers, synchronous) -----------------
  * The reference's per-operation-rounding formats (precision.hpp:41-97), which it runs
  * only on the CPU (batched.hpp:130-132), bit-identical to its CPU results. Storage is
- * float64 as in the runtime API (runtime.cpp:95-141); fmt 0 = fp16, 1 = bf16.
+ * float64 as in the runtime API (runtime.cpp:95-141); _f32: float32, _f16: binary16 bits
+ * (values are rounded into the format on entry); fmt 0 = fp16, 1 = bf16.
  *   factor: lu = 0 Cholesky (A <- L, info), lu = 1 LU (A <- L\U, piv, info)
  *   solve:  lu = 0 B <- (L L^T)^{-1} B, lu = 1 B <- (P L U)^{-1} B */
 int tsdx_cuda_emu_factor_host(int fmt, int lu, double* A, int n, int64_t batch, int* piv, int* info);
 int tsdx_cuda_emu_solve_host(int fmt, int lu, const double* F, const int* piv, int n, int64_t batch, double* B,
                              int nrhs);
+int tsdx_cuda_emu_factor_host_f32(int fmt, int lu, float* A, int n, int64_t batch, int* piv, int* info);
+int tsdx_cuda_emu_solve_host_f32(int fmt, int lu, const float* F, const int* piv, int n, int64_t batch, float* B,
+                                 int nrhs);
+int tsdx_cuda_emu_factor_host_f16(int fmt, int lu, uint16_t* A, int n, int64_t batch, int* piv, int* info);
+int tsdx_cuda_emu_solve_host_f16(int fmt, int lu, const uint16_t* F, const int* piv, int n, int64_t batch, uint16_t* B,
+                                 int nrhs);
 
 /* ---- error metrics on the GPU ------------------------------------------------------
  * The reference's ground-truth metrics (src/runtime.cpp:194-242, long double on the

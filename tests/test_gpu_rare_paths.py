@@ -84,6 +84,26 @@ def test_solves_from_factor(oracle, n, nrhs, dtype):
         assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
+def test_binary16_storage_equals_cpu(n):
+    r = np.random.default_rng(n)
+    S = M.spd(r, 5, n, 10.0).astype(np.float16)
+    G = r.standard_normal((5, n, n)).astype(np.float16)
+    B = r.standard_normal((5, n, 3)).astype(np.float16)
+    if n > 2:
+        S[1, 1, 1] = -1.0
+        G[1, :, 1] = 0.0
+        G[2] = r.integers(-1, 2, (n, n))
+    for f, X in ((tsdx.cholesky, S), (tsdx.lu, G)):
+        got, want = f(X, backend="cuda"), f(X, backend="scalar")
+        assert got[0].dtype == np.float16 and same(got[0], want[0])
+        assert all(np.array_equal(a, b) for a, b in zip(got[1:], want[1:]))
+    L, _ = tsdx.cholesky(S[2:], backend="scalar")
+    assert same(tsdx.cholesky_solve(L, B[2:], backend="cuda"), tsdx.cholesky_solve(L, B[2:], backend="scalar"))
+    LU, piv, _ = tsdx.lu(G[3:], backend="scalar")
+    assert same(tsdx.lu_solve(LU, piv, B[3:], backend="cuda"), tsdx.lu_solve(LU, piv, B[3:], backend="scalar"))
+
+
 @pytest.mark.parametrize("batch", [1, 63, 64, 65, 600])
 def test_training_gradient_of_partial_blocks(batch):
     """Against float64: float32 sums of at most 600 samples over 64 units carry a few

@@ -41,11 +41,12 @@ _NATIVE = {np.dtype(np.float32): "fp32", np.dtype(np.float64): "fp64"}
 
 
 class _Operand:
-    """A matrix argument normalised by the rules above."""
+    """A matrix argument normalised by the rules above. On backend "cuda", float16 storage
+    at precision fp16 goes through as it is (its bits; no conversion on the host)."""
 
-    __slots__ = ("work", "precision", "single", "storage")
+    __slots__ = ("work", "precision", "single", "storage", "half")
 
-    def __init__(self, a, precision):
+    def __init__(self, a, precision, backend=None):
         a = np.asarray(a)
         if precision is None:
             precision = _IMPLIED_PRECISION.get(a.dtype)
@@ -56,18 +57,26 @@ class _Operand:
         self.precision = precision
         self.storage = a.dtype
         self.single = a.ndim == 2
-        wide = a.dtype == np.float64
-        self.work = np.ascontiguousarray(a[None] if self.single else a, dtype=np.float64 if wide else np.float32)
+        self.half = backend == "cuda" and precision == "fp16" and a.dtype == np.float16
+        dt = a.dtype if self.half or a.dtype == np.float64 else np.float32
+        self.work = np.ascontiguousarray(a[None] if self.single else a, dtype=dt)
+        if self.half:
+            self.work = self.work.view(np.uint16)
 
-    def entry(self, op):
-        """The core entry point of ``op`` for the working dtype."""
-        return getattr(_core, op + ("_f64" if self.work.dtype == np.float64 else "_f32"))
+    def call(self, op, *args, backend):
+        """The core entry point of ``op`` for the working dtype on the working array and args."""
+        if self.half:
+            return getattr(_core, op + "_f16")(self.work, *args)
+        sfx = "_f64" if self.work.dtype == np.float64 else "_f32"
+        return getattr(_core, op + sfx)(self.work, *args, self.precision, backend)
 
     def native(self):
         """True when the precision is the working dtype's own (no emulation)."""
         return _NATIVE.get(self.work.dtype) == self.precision
 
     def cast(self, x):
+        if self.half:
+            return x.view(np.float16)
         return x.astype(np.float16) if (self.precision == "fp16" and self.storage == np.float16) else x
 
     def unbatch(self, *results):
@@ -82,6 +91,8 @@ class _Operand:
             B = B[..., None]
         if self.single:
             B = B[None]
+        if self.half:
+            return np.ascontiguousarray(B).view(np.uint16), vector
         return np.ascontiguousarray(B, dtype=self.work.dtype), vector
 
     def solution(self, X, vector):
@@ -91,33 +102,35 @@ class _Operand:
 
 def cholesky(A, precision=None, backend="auto"):
     """Lower Cholesky factors and LAPACK-style info (0 = ok, k>0: pivot k not positive)."""
-    op = _Operand(A, precision)
-    L, info = op.entry("cholesky")(op.work, op.precision, backend)
+    op = _Operand(A, precision, backend)
+    L, info = op.call("cholesky", backend=backend)
     return op.unbatch(op.cast(L), info)
 
 
 def lu(A, precision=None, backend="auto"):
     """Packed LU with partial pivoting: (LU, piv, info). piv is scipy/LAPACK style (0-based)."""
-    op = _Operand(A, precision)
-    LU, piv, info = op.entry("lu")(op.work, op.precision, backend)
+    op = _Operand(A, precision, backend)
+    LU, piv, info = op.call("lu", backend=backend)
     return op.unbatch(op.cast(LU), piv, info)
 
 
 def cholesky_solve(L, B, precision=None, backend="auto"):
     """Solve L L^T x = B given factors from :func:`cholesky`."""
-    op = _Operand(L, precision)
+    B = np.asarray(B)
+    op = _Operand(L, precision, backend if B.dtype == np.float16 else None)
     rhs, vector = op.rhs(B)
-    X = op.entry("cholesky_solve")(op.work, rhs, op.precision, backend)
+    X = op.call("cholesky_solve", rhs, backend=backend)
     return op.solution(op.cast(X), vector)
 
 
 def lu_solve(LU, piv, B, precision=None, backend="auto"):
     """Solve A x = B given (LU, piv) from :func:`lu`."""
-    op = _Operand(LU, precision)
+    B = np.asarray(B)
+    op = _Operand(LU, precision, backend if B.dtype == np.float16 else None)
     p = np.asarray(piv)
     p = np.ascontiguousarray(p[None] if op.single else p, dtype=np.int32)
     rhs, vector = op.rhs(B)
-    X = op.entry("lu_solve")(op.work, p, rhs, op.precision, backend)
+    X = op.call("lu_solve", p, rhs, backend=backend)
     return op.solution(op.cast(X), vector)
 
 
@@ -127,7 +140,8 @@ def _fused(kind, A, B, precision):
     if not op.native():
         return None
     rhs, vector = op.rhs(B)
-    X, info = op.entry(kind + "_cuda")(op.work, rhs)
+    sfx = "_f64" if op.work.dtype == np.float64 else "_f32"
+    X, info = getattr(_core, kind + "_cuda" + sfx)(op.work, rhs)
     return op.solution(X, vector), (info[0] if op.single else info)
 
 

@@ -210,6 +210,40 @@ void bind_solvers(py::module_& m, const std::string& sfx) {
   }
 }
 
+// ------------------------------------------- fp16 on the GPU, binary16 storage
+// Arrays of binary16 bits (uint16), the values the emulated format computes with: no
+// conversion on the host.
+void bind_half(py::module_& m) {
+  using S = std::uint16_t;
+  m.def("cholesky_f16", [](const Arr<S>& A) {
+    return solver_entry<S, Writes::Stack, false, true>(A, nullptr, nullptr, [&](const Stack& s, S* a, int*, int* info) {
+      tsdx::detail::check_dims(s.n, s.batch);
+      tsdx::detail::check_cuda(tsdx_cuda_emu_factor_host_f16(0, 0, a, s.n, s.batch, nullptr, info));
+    });
+  });
+  m.def("lu_f16", [](const Arr<S>& A) {
+    return solver_entry<S, Writes::Stack, true, true>(A, nullptr, nullptr, [&](const Stack& s, S* a, int* piv, int* info) {
+      tsdx::detail::check_dims(s.n, s.batch);
+      tsdx::detail::check_cuda(tsdx_cuda_emu_factor_host_f16(0, 1, a, s.n, s.batch, piv, info));
+    });
+  });
+  m.def("cholesky_solve_f16", [](const Arr<S>& L, const Arr<S>& B) {
+    const S* l = L.data();
+    return solver_entry<S, Writes::Rhs, false, false>(L, &B, nullptr, [&](const Stack& s, S* x, int*, int*) {
+      tsdx::detail::check_dims(s.n, s.batch);
+      tsdx::detail::check_cuda(tsdx_cuda_emu_solve_host_f16(0, 0, l, nullptr, s.n, s.batch, x, s.nrhs));
+    });
+  });
+  m.def("lu_solve_f16", [](const Arr<S>& LU, const IntArr& piv, const Arr<S>& B) {
+    const S* l = LU.data();
+    const int* pv = piv.data();
+    return solver_entry<S, Writes::Rhs, false, false>(LU, &B, &piv, [&](const Stack& s, S* x, int*, int*) {
+      tsdx::detail::check_dims(s.n, s.batch);
+      tsdx::detail::check_cuda(tsdx_cuda_emu_solve_host_f16(0, 1, l, pv, s.n, s.batch, x, s.nrhs));
+    });
+  });
+}
+
 // ------------------------------------------------------------ metrics (float64)
 using F64 = Arr<double>;
 
@@ -262,6 +296,7 @@ PYBIND11_MODULE(_core, m) {
   m.doc() = "B200-native batched small-matrix Cholesky/LU (drop-in for TinySolverDx _core)";
   bind_solvers<float>(m, "f32");
   bind_solvers<double>(m, "f64");
+  bind_half(m);
   m.def("has_cuda", &tsdx::has_cuda);
   m.def("has_openmp", &tsdx::has_openmp);
   m.def("num_threads", &tsdx::num_threads);

@@ -29,6 +29,10 @@ int run_ir(bool spd, const double* A, int n, long long batch, double* B, const s
            int itmax, double tol, int* info, int* status, double* bwd, cudaStream_t st);
 long long stream_scratch_bytes(long long count);
 template <class T> int run_stream(dev::StreamArgs<T> a, void* scratch, long long scratch_bytes, cudaStream_t st);
+template <class S>
+int run_emu_factor(int fmt, bool lu, S* A, int n, long long batch, int* piv, int* info, cudaStream_t st);
+template <class S>
+int run_emu_solve(int fmt, bool lu, const S* F, const int* piv, int n, long long batch, S* B, int nrhs, cudaStream_t st);
 
 namespace {
 thread_local std::string g_err;
@@ -160,9 +164,10 @@ int grow(void** p, size_t* cap, size_t need) {
 
 // keep_a: the one-shot solve leaves the caller's A untouched and returns no pivots
 // (the reference's Python-level gesv/posv return only (x, info), __init__.py:102-111).
-template <class T>
-int run_host(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int nrhs, int* piv, int* info,
-             bool keep_a = false) {
+// launch(A, piv, batch, B, info, stream) runs one chunk on device pointers.
+template <class T, class Launch>
+int run_host_with(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int nrhs, int* piv, int* info,
+                  bool keep_a, Launch&& launch) {
   if (int rc = check_common(n, batch, nrhs)) return rc;
   const bool has_b = (kind == POTRS || kind == GETRS || kind == POSV || kind == GESV);
   if (!has_b) nrhs = 0;
@@ -209,7 +214,7 @@ int run_host(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int
       if (kind == GETRS)
         TSDX_CK(cudaMemcpyAsync(s.piv, piv_in + m * n, size_t(n) * cnt * sizeof(int), cudaMemcpyHostToDevice, s.st), "H2D piv");
       // the device workspace copy of A may take the factor even when the caller's A is kept
-      const int rc = run_device<T>(kind, dA, s.piv, n, cnt, dB, nrhs, s.piv, writes_info ? s.info : nullptr, s.st);
+      const int rc = launch(dA, s.piv, cnt, dB, writes_info ? s.info : nullptr, s.st);
       if (rc) return rc;
       if (writes_a)
         TSDX_CK(cudaMemcpyAsync(reinterpret_cast<char*>(A) + m * mat, dA, mat * cnt, cudaMemcpyDeviceToHost, s.st), "D2H A");
@@ -232,6 +237,45 @@ int run_host(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int
     }
   }
   return rc;
+}
+
+template <class T>
+int run_host(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int nrhs, int* piv, int* info,
+             bool keep_a = false) {
+  return run_host_with<T>(kind, A, piv_in, n, batch, B, nrhs, piv, info, keep_a,
+                          [&](T* dA, int* dpiv, int64_t cnt, T* dB, int* dinfo, cudaStream_t st) {
+                            return run_device<T>(kind, dA, dpiv, n, cnt, dB, nrhs, dpiv, dinfo, st);
+                          });
+}
+
+// ---- emulated formats (S: the storage type), through the same pipeline
+int emu_check(int fmt, int n, int64_t batch) {
+  if (fmt != 0 && fmt != 1) return TSDX_ERR_NULL;
+  if (n < 1 || n > 64) return TSDX_ERR_N;
+  if (batch < 0) return TSDX_ERR_BATCH;
+  int count = 0;
+  if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) {
+    cudaGetLastError();
+    return TSDX_ERR_NODEV;
+  }
+  return TSDX_OK;
+}
+template <class S> int emu_factor_host(int fmt, int lu, S* A, int n, int64_t batch, int* piv, int* info) {
+  if (int rc = emu_check(fmt, n, batch)) return rc;
+  return run_host_with<S>(lu ? GETRF : POTRF, A, nullptr, n, batch, nullptr, 0, piv, info, false,
+                          [&](S* dA, int* dpiv, int64_t cnt, S*, int* dinfo, cudaStream_t st) {
+                            return run_emu_factor<S>(fmt, lu != 0, dA, n, cnt, dpiv, dinfo, st);
+                          });
+}
+template <class S>
+int emu_solve_host(int fmt, int lu, const S* F, const int* piv, int n, int64_t batch, S* B, int nrhs) {
+  if (int rc = emu_check(fmt, n, batch)) return rc;
+  if (nrhs < 0) return TSDX_ERR_NRHS;
+  if (batch == 0 || nrhs == 0) return TSDX_OK;
+  return run_host_with<S>(lu ? GETRS : POTRS, const_cast<S*>(F), piv, n, batch, B, nrhs, nullptr, nullptr, false,
+                          [&](S* dF, int* dpiv, int64_t cnt, S* dB, int*, cudaStream_t st) {
+                            return run_emu_solve<S>(fmt, lu != 0, dF, dpiv, n, cnt, dB, nrhs, st);
+                          });
 }
 
 }  // namespace
@@ -286,6 +330,19 @@ API int tsdx_internal_div_check_f32(const float* a, const float* b, float* fast,
                                      void* st) {
   return div_check<float>(a, b, fast, ieee, count, st);
 }
+
+// ---- emulated fp16 / bf16 ---------------------------------------------------------
+#define TSDX_EMU_API(SFX, S)                                                                                        \
+  API int tsdx_cuda_emu_factor_host##SFX(int fmt, int lu, S* A, int n, int64_t batch, int* piv, int* info) {        \
+    return tsdx::host::emu_factor_host<S>(fmt, lu, A, n, batch, piv, info);                                         \
+  }                                                                                                                 \
+  API int tsdx_cuda_emu_solve_host##SFX(int fmt, int lu, const S* F, const int* piv, int n, int64_t batch, S* B,    \
+                                        int nrhs) {                                                                 \
+    return tsdx::host::emu_solve_host<S>(fmt, lu, F, piv, n, batch, B, nrhs);                                       \
+  }
+TSDX_EMU_API(, double)
+TSDX_EMU_API(_f32, float)
+TSDX_EMU_API(_f16, uint16_t)
 
 // ---- mixed precision + iterative refinement ------------------------------------
 namespace {

@@ -388,11 +388,17 @@ namespace detail {
 // Emulated formats on the GPU (tsdx_cuda_emu_*_host, bit-identical to the CPU path):
 // the reference throws here (batched.hpp:130-132); this build runs them instead.
 template <class T> constexpr int emu_fmt() { return std::is_same<T, Half>::value ? 0 : 1; }
-template <class S> std::vector<double> f64_copy(const S* x, std::int64_t count) {
-  return std::vector<double>(x, x + count);
+inline int emu_factor(int fmt, int lu, double* A, int n, std::int64_t batch, int* piv, int* info) {
+  return tsdx_cuda_emu_factor_host(fmt, lu, A, n, batch, piv, info);
 }
-template <class S> void f64_back(const std::vector<double>& v, S* x) {
-  for (std::size_t i = 0; i < v.size(); ++i) x[i] = static_cast<S>(v[i]);
+inline int emu_factor(int fmt, int lu, float* A, int n, std::int64_t batch, int* piv, int* info) {
+  return tsdx_cuda_emu_factor_host_f32(fmt, lu, A, n, batch, piv, info);
+}
+inline int emu_solve(int fmt, int lu, const double* F, const int* piv, int n, std::int64_t batch, double* B, int nrhs) {
+  return tsdx_cuda_emu_solve_host(fmt, lu, F, piv, n, batch, B, nrhs);
+}
+inline int emu_solve(int fmt, int lu, const float* F, const int* piv, int n, std::int64_t batch, float* B, int nrhs) {
+  return tsdx_cuda_emu_solve_host_f32(fmt, lu, F, piv, n, batch, B, nrhs);
 }
 }  // namespace detail
 
@@ -405,10 +411,7 @@ void cholesky(Precision p, S* A, int n, std::int64_t batch, int* info, Backend b
       if constexpr (!is_native<T>::value) {
         if (be == Backend::Cuda) {
           detail::check_dims(n, batch);
-          auto w = detail::f64_copy(A, batch * n * n);
-          detail::check_cuda(tsdx_cuda_emu_factor_host(detail::emu_fmt<T>(), 0, w.data(), n, batch, nullptr, info));
-          detail::f64_back(w, A);
-          return;
+          return detail::check_cuda(detail::emu_factor(detail::emu_fmt<T>(), 0, A, n, batch, nullptr, info));
         }
       }
       auto v = detail::to_t<T>(A, batch * n * n);
@@ -427,10 +430,7 @@ void lu(Precision p, S* A, int n, std::int64_t batch, int* piv, int* info, Backe
         if (be == Backend::Cuda) {
           detail::check_dims(n, batch);
           if (!piv) throw std::invalid_argument("piv must not be null");
-          auto w = detail::f64_copy(A, batch * n * n);
-          detail::check_cuda(tsdx_cuda_emu_factor_host(detail::emu_fmt<T>(), 1, w.data(), n, batch, piv, info));
-          detail::f64_back(w, A);
-          return;
+          return detail::check_cuda(detail::emu_factor(detail::emu_fmt<T>(), 1, A, n, batch, piv, info));
         }
       }
       auto v = detail::to_t<T>(A, batch * n * n);
@@ -446,11 +446,7 @@ void cholesky_solve(Precision p, const S* L, int n, std::int64_t batch, S* B, in
     if constexpr (!is_native<T>::value) {
       if (be == Backend::Cuda) {
         detail::check_dims(n, batch);
-        auto l = detail::f64_copy(L, batch * n * n);
-        auto b = detail::f64_copy(B, batch * n * nrhs);
-        detail::check_cuda(tsdx_cuda_emu_solve_host(detail::emu_fmt<T>(), 0, l.data(), nullptr, n, batch, b.data(), nrhs));
-        detail::f64_back(b, B);
-        return;
+        return detail::check_cuda(detail::emu_solve(detail::emu_fmt<T>(), 0, L, nullptr, n, batch, B, nrhs));
       }
     }
     auto l = detail::to_t<T>(L, batch * n * n);
@@ -466,11 +462,7 @@ void lu_solve(Precision p, const S* LU, const int* piv, int n, std::int64_t batc
     if constexpr (!is_native<T>::value) {
       if (be == Backend::Cuda) {
         detail::check_dims(n, batch);
-        auto l = detail::f64_copy(LU, batch * n * n);
-        auto b = detail::f64_copy(B, batch * n * nrhs);
-        detail::check_cuda(tsdx_cuda_emu_solve_host(detail::emu_fmt<T>(), 1, l.data(), piv, n, batch, b.data(), nrhs));
-        detail::f64_back(b, B);
-        return;
+        return detail::check_cuda(detail::emu_solve(detail::emu_fmt<T>(), 1, LU, piv, n, batch, B, nrhs));
       }
     }
     auto l = detail::to_t<T>(LU, batch * n * n);
