@@ -1,26 +1,11 @@
-// Shared pieces of the kernels that keep a matrix in shared memory (layout, staging,
-// copies), and the general LU body: one G-lane segment per matrix, the matrix plus its
-// right-hand sides (appended as columns) in shared memory, factored in panels of PB
-// columns:
-//   1. panel factorization in registers (lane l owns rows l + G*s): pivot search by
-//      segment reduction with implicit row swaps, multipliers, rank-1 update of the
-//      panel only;
-//   2. U12, the panel's pivot rows brought up to date on the trailing columns by a
-//      unit-lower triangular solve (one lane per column);
-//   3. trailing update A22 -= L21 U12 for the rows still active, column chunk by column
-//      chunk, from shared memory with the panel multipliers kept in registers.
-// Every element receives exactly the reference's chain of operations, so factors,
-// pivots and info are bit-identical to TinySolverDx's CPU backends (kernels.hpp:91-119):
-//   a_ij <- fma(-l_ik, u_kj, a_ij) in increasing k, l_ik = a_ik / u_kk correctly rounded,
-//   a zero pivot skips the column; ties go to the first maximum and NaN never wins unless
-//   on the diagonal position.
-// Rows never move: ord[k] records the physical row retired at step k and the factor is
-// written in that order, which is where the reference's full-row swaps leave each row.
-// The forward substitution rides along as extra columns (the reference's chain,
-// kernels.hpp:184-193 / 214-218); the backward substitution is column-oriented with
-// reciprocal diagonals, so X agrees to rounding.
-//
-// This body covers every input; rows.cuh holds the faster ones and falls back on it.
+// Shared pieces of the kernels that keep a matrix in shared memory: layout, copies, and
+// the back substitution of the two-warp LU kernels (blk2.cuh, blk3.cuh). The matrix and
+// its right-hand sides (appended as columns) stand in padded rows. Rows never move in an
+// LU: ord[k] records the physical row retired at step k and the factor is written in that
+// order, which is where the reference's full-row swaps leave each row
+// (TinySolverDx kernels.hpp:91-119). The forward substitution rides along as extra columns
+// (the reference's chain, kernels.hpp:184-193 / 214-218); the backward substitution is
+// column-oriented with reciprocal diagonals, so X agrees to rounding.
 #pragma once
 #include "common.cuh"
 
@@ -70,7 +55,6 @@ struct MatJob {
 
 struct Seg {
   int lane, lsl, segbase;
-  unsigned segmask;
   unsigned zrow;  // shared address of a row of zeros (rows.cuh)
 };
 
@@ -141,31 +125,6 @@ __device__ __forceinline__ void fma_if(float& y, bool p, float u, float x) {
       : "r"((int)p), "f"(-u), "f"(x));
 }
 
-// Stage the job's matrix (identity-padded to NP) and right-hand sides.
-template <class T, int NP, int NRHS, int GO>
-__device__ __forceinline__ void seg_load(unsigned char* M, const MatJob<T>& j, const Seg& g) {
-  using C = BlkCfg<T, NP, NRHS, GO>;
-  constexpr int G = C::G, MR = C::MR, RS = C::RS;
-  auto at = [&](int r, int c) -> T& { return *reinterpret_cast<T*>(M + r * RS + c * int(sizeof(T))); };
-  if (j.live) seg_copy_in<T, G, RS>(M, j.A, j.n, g.lsl);
-  cp_async_wait<0>();
-  __syncwarp();
-#pragma unroll
-  for (int s = 0; s < MR; ++s) {
-    const int r = g.lsl + G * s;
-    if (r >= NP) continue;
-    const bool full = !j.live || r >= j.n;
-    for (int c = full ? 0 : j.n; c < NP; ++c) at(r, c) = (r == c) ? T(1) : T(0);
-    if constexpr (NRHS > 0) {
-      const bool rowok = j.live && j.B && r < j.n;
-      const T* brow = rowok ? j.B + (long long)r * j.ldb + j.b0 : nullptr;
-#pragma unroll
-      for (int c = 0; c < NRHS; ++c) at(r, NP + c) = (rowok && c < j.nrhs) ? brow[c] : T(0);
-    }
-  }
-  __syncwarp();
-}
-
 // Column-oriented back substitution with reciprocal diagonals; U(i,k) sits in shared row
 // ord[i].
 template <class T, int NP, int NRHS, int GO>
@@ -224,197 +183,6 @@ __device__ __forceinline__ void seg_backsolve(unsigned char* M, const int* ord, 
         if (c < j.nrhs) brow[c] = yv[t][c] * dv[t];
     }
   }
-}
-
-// ------------------------------------------------------------------------- LU
-template <class T, int NP, int NRHS, int GO>
-__device__ __forceinline__ void lu_matrix(unsigned char* M, const MatJob<T>& j, const Seg& g) {
-  using C = BlkCfg<T, NP, NRHS, GO>;
-  using K = typename KeyT<T>::U;
-  using V = Vec16<T>;
-  using VT = typename V::type;
-  constexpr int G = C::G, MR = C::MR, PB = C::PB, NC = C::NC, CH = C::CH, RS = C::RS;
-  constexpr int VN = V::n, TS = int(sizeof(T));
-  const int lane = g.lane, lsl = g.lsl, segbase = g.segbase;
-  const unsigned segmask = g.segmask;
-  int* ord = reinterpret_cast<int*>(M + C::MAT);
-  int* pvs = ord + NP;
-  auto at = [&](int r, int c) -> T& { return *reinterpret_cast<T*>(M + r * RS + c * TS); };
-  auto vat = [&](int r, int c) -> VT& { return *reinterpret_cast<VT*>(M + r * RS + c * TS); };
-
-  seg_load<T, NP, NRHS, GO>(M, j, g);
-  int pos[MR];
-  bool act[MR];
-#pragma unroll
-  for (int s = 0; s < MR; ++s) {
-    const int r = lsl + G * s;
-    act[s] = r < NP;
-    pos[s] = r < NP ? r : 0x3fffffff;
-  }
-  int info = 0;
-
-  for (int k0 = 0; k0 < NP; k0 += PB) {
-    // ------------------------------------------------ 1. panel in registers
-    T pan[MR][PB];
-#pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lsl + G * s;
-      const int rr = r < NP ? r : 0;
-#pragma unroll
-      for (int i0 = 0; i0 < PB; i0 += VN) {
-        const VT v = vat(rr, k0 + i0);
-#pragma unroll
-        for (int q = 0; q < VN; ++q) pan[s][i0 + q] = V::get(v, q);
-      }
-    }
-    unsigned zbits = 0;
-#pragma unroll
-    for (int i = 0; i < PB; ++i) {
-      const int k = k0 + i;
-      K bk = 0;
-      int bp = 0x7fffffff;
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const T v = pan[s][i];
-        const K key = isnan(v) ? (pos[s] == k ? ~K(0) : K(0)) : key_bits(v) + 1;
-        const bool better = act[s] && (key > bk || (key == bk && pos[s] < bp));
-        bk = better ? key : bk;
-        bp = better ? pos[s] : bp;
-      }
-      K best;
-      const int bpos = seg_argmax(segmask, bk, bp, &best);
-      const bool zero = (best == K(1));
-      int myslot = -1;
-#pragma unroll
-      for (int s = 0; s < MR; ++s) myslot = (act[s] && pos[s] == bpos) ? s : myslot;
-      const unsigned bal = __ballot_sync(kFull, myslot >= 0);
-      const int wl = segbase + __ffs((bal & segmask) >> segbase) - 1;
-      int wslot = 0;
-      if (MR > 1) wslot = __shfl_sync(kFull, myslot, wl);
-      T uw[PB];  // the winner's panel row, columns i..PB-1
-#pragma unroll
-      for (int jj = i; jj < PB; ++jj) {
-        T v = pan[0][jj];
-#pragma unroll
-        for (int t = 1; t < MR; ++t) v = (wslot == t) ? pan[t][jj] : v;
-        uw[jj] = __shfl_sync(kFull, v, wl);
-      }
-      if (lane == wl) {
-        ord[k] = lsl + G * wslot;
-        pvs[k] = bpos;
-      }
-      // retire the winner and replay the reference's swap of positions k and bpos
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const bool win = act[s] && pos[s] == bpos;
-        const bool atk = act[s] && !win && pos[s] == k;
-        pos[s] = win ? k : (atk ? bpos : pos[s]);
-        act[s] = act[s] && !win;
-      }
-      info = (zero && info == 0) ? k + 1 : info;
-      if (zero) {
-        zbits |= 1u << i;
-      } else {
-        const T vpk = uw[i];
-        const T ry = rcp_(vpk);
-#pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          if (!act[s]) continue;
-          const T l = div_by(pan[s][i], vpk, ry);
-          pan[s][i] = l;
-#pragma unroll
-          for (int jj = i + 1; jj < PB; ++jj) pan[s][jj] = fma_(-l, uw[jj], pan[s][jj]);
-        }
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lsl + G * s;
-      if (r >= NP) continue;
-#pragma unroll
-      for (int i0 = 0; i0 < PB; i0 += VN) {
-        VT v;
-#pragma unroll
-        for (int q = 0; q < VN; ++q) V::set(v, q, pan[s][i0 + q]);
-        vat(r, k0 + i0) = v;
-      }
-    }
-    __syncwarp();
-    const int j1 = k0 + PB;
-    if (j1 >= NC) continue;
-    // ------------------------------- 2. U12: pivot rows on the trailing columns
-    for (int jc = j1 + lsl; jc < NC; jc += G) {
-      T u[PB];
-#pragma unroll
-      for (int i = 0; i < PB; ++i) {
-        const int pr = ord[k0 + i];
-        T acc = at(pr, jc);
-#pragma unroll
-        for (int i2 = 0; i2 < i; ++i2)
-          if (!((zbits >> i2) & 1u)) acc = fma_(-at(pr, k0 + i2), u[i2], acc);
-        u[i] = acc;
-        if (i > 0) at(pr, jc) = acc;
-      }
-    }
-    __syncwarp();
-    // --------------------------------- 3. trailing update of the active rows
-    for (int jc = j1; jc < NC; jc += CH) {
-      T acc[MR][CH];
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        const int r = act[s] ? lsl + G * s : 0;
-#pragma unroll
-        for (int c0 = 0; c0 < CH; c0 += VN) {
-          const VT v = vat(r, jc + c0);
-#pragma unroll
-          for (int q = 0; q < VN; ++q) acc[s][c0 + q] = V::get(v, q);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < PB; ++i) {
-        if ((zbits >> i) & 1u) continue;
-        const int pr = ord[k0 + i];
-#pragma unroll
-        for (int c0 = 0; c0 < CH; c0 += VN) {
-          const VT v = vat(pr, jc + c0);
-#pragma unroll
-          for (int q = 0; q < VN; ++q) {
-            const T u = V::get(v, q);
-#pragma unroll
-            for (int s = 0; s < MR; ++s) acc[s][c0 + q] = fma_(-pan[s][i], u, acc[s][c0 + q]);
-          }
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < MR; ++s) {
-        if (!act[s]) continue;
-        const int r = lsl + G * s;
-#pragma unroll
-        for (int c0 = 0; c0 < CH; c0 += VN) {
-          VT v;
-#pragma unroll
-          for (int q = 0; q < VN; ++q) V::set(v, q, acc[s][c0 + q]);
-          vat(r, jc + c0) = v;
-        }
-      }
-    }
-    __syncwarp();
-  }
-
-  if constexpr (NRHS > 0) seg_backsolve<T, NP, NRHS, GO>(M, ord, j, g);
-  if (j.live) {
-    if (j.piv) {
-#pragma unroll
-      for (int t = 0; t < MR; ++t) {
-        const int k = lsl + G * t;
-        if (k < j.n) j.piv[k] = pvs[k];
-      }
-    }
-    if (lsl == 0 && j.info) *j.info = info;
-  }
-  __syncwarp();
-  if (j.live && j.Aout) seg_copy_out<T, G, RS>(M, j.Aout, j.n, lsl, ord);
-  __syncwarp();
 }
 
 }  // namespace dev

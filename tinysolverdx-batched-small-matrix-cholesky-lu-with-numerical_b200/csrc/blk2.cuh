@@ -216,7 +216,6 @@ __device__ __forceinline__ void lu2_matrix(unsigned char* M, const MatJob<T>& j,
       g0.lane = lane;
       g0.lsl = lane;
       g0.segbase = 0;
-      g0.segmask = kFull;
       seg_backsolve<T, NP, NRHS, 32>(M, ord, j, g0);
     }
   } else if (j.live) {

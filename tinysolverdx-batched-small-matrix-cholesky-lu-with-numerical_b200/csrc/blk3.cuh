@@ -345,7 +345,6 @@ __device__ __forceinline__ void lu3_matrix(unsigned char* M, const MatJob<T>& j,
       g0.lane = lane;
       g0.lsl = lane;
       g0.segbase = 0;
-      g0.segmask = kFull;
       seg_backsolve<T, NP, NRHS, 32>(M, ord, j, g0);
     }
     if (j.live && lane == 0 && j.info) *j.info = info;

@@ -498,19 +498,19 @@ __device__ __forceinline__ bool lu_tc_matrix(unsigned char* M, const MatJob<doub
   return true;
 }
 
-// Dense batch: a persistent CTA of WPC warps, one matrix per warp per round.
+// Dense batch: a persistent CTA of at most WPC warps, one matrix per warp per round.
 template <int NP, int NRHS, int WPC>
 __global__ void __launch_bounds__(WPC * 32, 1) tc_kernel(SolveArgs<double> p) {
   using C = TcCfg<NP, NRHS>;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   unsigned char* M = smem + warp * C::WARPB;
   const long long nn = (long long)p.n * p.n;
-  const long long step = (long long)gridDim.x * WPC;
+  const long long step = (long long)gridDim.x * wpc;
   if (lane == 0) mbar_init(reinterpret_cast<unsigned long long*>(M + C::OFF_BAR));
   __syncwarp();
   unsigned par = 0;  // parity of the mbarrier phase the next bulk load completes
-  for (long long m = (long long)blockIdx.x * WPC + warp; m < p.batch; m += step) {
+  for (long long m = (long long)blockIdx.x * wpc + warp; m < p.batch; m += step) {
     if (p.status && p.status[m] >= 0) continue;  // already solved: nothing to read or write
     // this warp's next matrix heads for L2 while this one is factored
     if (lane == 0 && m + step < p.batch) {

@@ -91,48 +91,6 @@ __device__ __forceinline__ int seg_argmax(unsigned mask, unsigned key, int pos, 
   return __reduce_min_sync(mask, key == mk ? pos : 0x7fffffff);
 }
 
-// Exact warp argmax: the largest key wins, ties go to the smallest position. The
-// first reduction runs on the key's high word; when one lane alone holds that
-// word, it is the winner and no further reduction is needed. *zero: the winning
-// key is 1 (|a| = 0).
-__device__ __forceinline__ int warp_argmax(unsigned long long key, int pos, bool* zero) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(kFull, hi);
-  const unsigned bal = __ballot_sync(kFull, hi == mhi);
-  if (__popc(bal) == 1) {  // then mhi > 0, so the key is not 1
-    *zero = false;
-    return __shfl_sync(kFull, pos, __ffs(bal) - 1);
-  }
-  const unsigned mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-  *zero = (mhi == 0u && mlo == 1u);
-  return __reduce_min_sync(kFull, (hi == mhi && lo == mlo) ? pos : 0x7fffffff);
-}
-__device__ __forceinline__ int warp_argmax(unsigned key, int pos, bool* zero) {
-  const unsigned mk = __reduce_max_sync(kFull, key);
-  *zero = (mk == 1u);
-  const unsigned bal = __ballot_sync(kFull, key == mk);
-  if (__popc(bal) == 1) return __shfl_sync(kFull, pos, __ffs(bal) - 1);
-  return __reduce_min_sync(kFull, key == mk ? pos : 0x7fffffff);
-}
-
-// The same, also returning the winner's lane: the lane whose best candidate is the
-// winning (key, position).
-__device__ __forceinline__ int warp_argmax_lane(unsigned long long key, int pos, bool* zero, int* wl) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(kFull, hi);
-  const unsigned bal = __ballot_sync(kFull, hi == mhi);
-  if (__popc(bal) == 1) {
-    *zero = false;
-    *wl = __ffs(bal) - 1;
-    return __shfl_sync(kFull, pos, *wl);
-  }
-  const unsigned mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-  *zero = (mhi == 0u && mlo == 1u);
-  const int bpos = __reduce_min_sync(kFull, (hi == mhi && lo == mlo) ? pos : 0x7fffffff);
-  *wl = __ffs(__ballot_sync(kFull, pos == bpos)) - 1;
-  return bpos;
-}
-
 // ---- cp.async (LDGSTS) staging of a global byte range into padded rows --------
 template <int VEC>
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
@@ -144,15 +102,6 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Fast division of small non-negative ints by a runtime divisor d (d <= 4096,
-// x < 2^19): q = umulhi(x, ceil(2^32/d)) is exact in that range.
-struct FastDiv {
-  unsigned d, m;
-  __host__ __device__ FastDiv() : d(1), m(0) {}
-  __host__ __device__ explicit FastDiv(unsigned dd) : d(dd), m((unsigned)((0x100000000ull + dd - 1) / dd)) {}
-  __device__ __forceinline__ unsigned div(unsigned x) const { return d == 1 ? x : __umulhi(x, m); }
-};
-
 template <class T>
 struct SolveArgs {
   T* A;            // (batch, n, n) row-major; overwritten by the factor
@@ -161,7 +110,6 @@ struct SolveArgs {
   int* info;       // (batch) or nullptr
   long long batch;
   int n, ldb, b0, nrhs;
-  FastDiv rowdiv;      // divides by the number of copy chunks per row
   const int* status;   // optional: matrices with status[m] >= 0 are skipped (no reads, no writes)
   int wf;              // 1: A <- factor and piv written (reference semantics); 0: A left untouched
 };
@@ -188,34 +136,6 @@ template <> struct Vec16<float> {
     if (i == 0) v.x = x; else if (i == 1) v.y = x; else if (i == 2) v.z = x; else v.w = x;
   }
 };
-
-// Copies rows [0, rows) of a dense (rows x n) stack at g into padded staging rows
-// (row stride RS bytes) with VEC-byte cp.async chunks; rc = n*sizeof(T)/VEC.
-template <class T, int VEC, int RS, int BUF>
-__device__ __forceinline__ void stage_in(unsigned char* stage, const char* g, int rows, int n, int rc,
-                                         const FastDiv& rowdiv, const FastDiv& ndiv, int tt, int TT) {
-  const int chunks = rows * rc;
-  for (int e = tt; e < chunks; e += TT) {
-    const int row = (int)rowdiv.div(e), ch = e - row * rc;
-    const int mm = (int)ndiv.div(row), r = row - mm * n;
-    cp_async<VEC>(stage + mm * BUF + r * RS + ch * VEC, g + (long long)row * n * int(sizeof(T)) + ch * VEC);
-  }
-  cp_async_commit();
-}
-template <class T, int VEC, int RS, int BUF>
-__device__ __forceinline__ void stage_out(const unsigned char* stage, char* g, int rows, int n, int rc,
-                                          const FastDiv& rowdiv, const FastDiv& ndiv, int tt, int TT) {
-  const int chunks = rows * rc;
-  for (int e = tt; e < chunks; e += TT) {
-    const int row = (int)rowdiv.div(e), ch = e - row * rc;
-    const int mm = (int)ndiv.div(row), r = row - mm * n;
-    const unsigned char* src = stage + mm * BUF + r * RS + ch * VEC;
-    char* dst = g + (long long)row * n * int(sizeof(T)) + ch * VEC;
-    if constexpr (VEC == 16) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-    else if constexpr (VEC == 8) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
-    else *reinterpret_cast<unsigned*>(dst) = *reinterpret_cast<const unsigned*>(src);
-  }
-}
 
 }  // namespace dev
 }  // namespace tsdx

@@ -8,11 +8,13 @@
 //   2. The scaled matrix is factored in fp32 with partial pivoting (LU) or, for
 //      symmetric positive definite input, without pivoting (A = L U with U = D L^T,
 //      the Cholesky factor up to a diagonal: SPD matrices need no pivoting, and the
-//      shared code keeps one fast path): 16-column panels in registers, the trailing update
-//      A22 -= L21 U12 either on the tensor cores (mma.sync m16n8k16, fp16 or bf16
-//      operands, fp32 accumulation) or on the fp32 CUDA cores, by tier.
-//   3. x0 = A^{-1} b with the low-precision factors (fp32 triangular solves,
-//      reciprocal pivots computed once after the factorization).
+//      shared code keeps one fast path): 16-column panels in registers, a step's pivot
+//      row published by the store that also writes it to the factor (as in rows.cuh), the
+//      trailing update A22 -= L21 U12 either on the tensor cores (mma.sync m16n8k16,
+//      fp16 or bf16 operands, fp32 accumulation) or on the fp32 CUDA cores, two columns
+//      to an instruction, by tier.
+//   3. x0 = A^{-1} b with the low-precision factors (fp32 triangular solves, a lane per
+//      position, reciprocal pivots computed once after the factorization).
 //   4. Refinement: r = b - A x in fp64 straight from A in global memory (rows
 //      read coalesced, 32 row sums per lane folded by a transposing butterfly),
 //      normwise backward error ||r|| / (||A||_F ||x|| + ||b||)
@@ -25,7 +27,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "common.cuh"
+#include "rows.cuh"
 
 namespace tsdx {
 namespace dev {
@@ -72,8 +74,9 @@ struct IrCfg {
   static constexpr int PB = 16;
   static constexpr int RSF = NP * 4 + 16;  // fp32 row: an odd number of 16-byte units
   static constexpr int F = NP * RSF;
-  // ord (int), x (double), column scales, row scales, reciprocal pivots (float)
-  static constexpr int AUX = NP * 4 + NP * 8 + NP * 4 * 3 + 32;
+  // ord (int), x (double), column scales, row scales (float; after the scaling, the
+  // right-hand side on its way to the pivots' order)
+  static constexpr int AUX = NP * 4 + NP * 8 + NP * 4 * 2 + 32;
   static constexpr int WARPB = (F + AUX + 127) / 128 * 128;
   // cooperative float4 passes: CG groups of 4 columns, RPI rows per pass
   static constexpr int CG = NP / 4;
@@ -87,23 +90,21 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
   using C = IrCfg<NP>;
   constexpr int MR = C::MR, PB = C::PB, RSF = C::RSF, CG = C::CG, CGP = C::CGP, RPI = C::RPI;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   unsigned char* Fb = smem + warp * C::WARPB;
   int* ord = reinterpret_cast<int*>(Fb + C::F);
   double* xs = reinterpret_cast<double*>(Fb + C::F + NP * 4);
   float* csc = reinterpret_cast<float*>(Fb + C::F + NP * 12);
   float* rsd = csc + NP;
-  float* rinv = rsd + NP;
+  const unsigned Fu = (unsigned)__cvta_generic_to_shared(Fb);
+  using U2 = Unit<float>;
   auto F = [&](int r, int c) -> float& { return *reinterpret_cast<float*>(Fb + r * RSF + c * 4); };
   auto F4 = [&](int r, int c) -> float4& { return *reinterpret_cast<float4*>(Fb + r * RSF + c * 4); };
   const int n = p.n;
-  const long long per_round = (long long)gridDim.x * WPC;
+  const long long per_round = (long long)gridDim.x * wpc;
   const int q4 = lane % CGP, rho = lane / CGP;  // cooperative pass coordinates
 
-  for (long long base = (long long)blockIdx.x * WPC; base < p.batch; base += per_round) {
-    __syncthreads();
-    const long long t = base + warp;
-    if (t >= p.batch) continue;
+  for (long long t = (long long)blockIdx.x * wpc + warp; t < p.batch; t += per_round) {
     const long long m = p.idx ? (long long)p.idx[t] : t;
     const int tier = p.tier ? (int)p.tier[m] : p.default_tier;
     if (tier >= kTierF64) {  // solved directly by the fp64 pass
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
     float rsc[MR];
     {
       // coalesced row reads (lane c holds columns c, c + 32), unscaled fp32 copy
-#pragma unroll 4
+#pragma unroll 8
       for (int r = 0; r < n; ++r) {
         const double* row = Ag + (long long)r * n;
 #pragma unroll
@@ -214,85 +215,109 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
     bnrm = sqrt(bnrm);
 
     // ------------------------------------------------ 2. low-precision factor
-    int pos[MR];
-    bool act[MR];
+    unsigned act[MR];  // key mask of the lane's rows, 0 once retired
 #pragma unroll
-    for (int s = 0; s < MR; ++s) {
-      const int r = lane + 32 * s;
-      act[s] = r < NP;
-      pos[s] = r < NP ? r : 0x3fffffff;
-    }
+    for (int s = 0; s < MR; ++s) act[s] = lane + 32 * s < NP ? 0x7fffffffu : 0u;
     int info = 0;
     for (int k0 = 0; k0 < NP; k0 += PB) {
-      float pan[MR][PB];
+      // a row's panel columns, two to a register pair
+      U2::E pan[MR][PB / 2];
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
         const int rr = (lane + 32 * s < NP) ? lane + 32 * s : 0;
 #pragma unroll
         for (int i0 = 0; i0 < PB; i0 += 4) {
-          const float4 v = F4(rr, k0 + i0);
-          pan[s][i0] = v.x; pan[s][i0 + 1] = v.y; pan[s][i0 + 2] = v.z; pan[s][i0 + 3] = v.w;
+          const Unit2<U2::E> v = lds16(Fu + rr * RSF + (k0 + i0) * 4, U2::E());
+          pan[s][i0 / 2] = v.x;
+          pan[s][i0 / 2 + 1] = v.y;
         }
       }
 #pragma unroll
       for (int i = 0; i < PB; ++i) {
         const int k = k0 + i;
-        {
-          int bpos = k;  // SPD: no pivoting (A = L U with U = D L^T)
-          if (!SPD) {
-          unsigned bk = 0;
-          int bp = 0x7fffffff;
+        int wr = k;  // SPD: no pivoting (A = L U with U = D L^T)
+        float x[MR];
+        bool win[MR];
+#pragma unroll
+        for (int s = 0; s < MR; ++s) x[s] = U2::get(pan[s][i / 2], i % 2);
+        if (!SPD) {
+          // the largest |a_ik| by its bits (a NaN is larger than all), ties by position
+          unsigned key[MR], m = 0, b[MR];
 #pragma unroll
           for (int s = 0; s < MR; ++s) {
-            const unsigned key = act[s] ? __float_as_uint(fabsf(pan[s][i])) + 1u : 0u;
-            const bool better = key > bk || (key == bk && pos[s] < bp);
-            bk = (act[s] && better) ? key : bk;
-            bp = (act[s] && better) ? pos[s] : bp;
+            key[s] = __float_as_uint(x[s]) & act[s];
+            m = max(m, key[s]);
           }
-          const unsigned mk = __reduce_max_sync(kFull, bk);
-          bpos = __reduce_min_sync(kFull, bk == mk ? bp : 0x7fffffff);
-          }
-          int myslot = -1;
-#pragma unroll
-          for (int s = 0; s < MR; ++s) myslot = (act[s] && pos[s] == bpos) ? s : myslot;
-          const int wl = __ffs(__ballot_sync(kFull, myslot >= 0)) - 1;
-          const int wslot = MR > 1 ? __shfl_sync(kFull, myslot, wl) : 0;
-          float uw[PB];
-#pragma unroll
-          for (int j = i; j < PB; ++j) {
-            float v = pan[0][j];
-#pragma unroll
-            for (int t2 = 1; t2 < MR; ++t2) v = (wslot == t2) ? pan[t2][j] : v;
-            uw[j] = __shfl_sync(kFull, v, wl);
-          }
-          if (lane == wl) ord[k] = lane + 32 * wslot;
+          m = __reduce_max_sync(kFull, m);
 #pragma unroll
           for (int s = 0; s < MR; ++s) {
-            const bool win = act[s] && pos[s] == bpos;
-            const bool atk = act[s] && !win && pos[s] == k;
-            pos[s] = win ? k : (atk ? bpos : pos[s]);
-            act[s] = act[s] && !win;
+            win[s] = key[s] == m;
+            b[s] = __ballot_sync(kFull, win[s]);
           }
-          const bool zero = SPD ? (!(uw[i] > 0.f) || !isfinite(uw[i])) : (!(uw[i] != 0.f) || !isfinite(uw[i]));
-          if (zero && info == 0) info = k + 1;
-          const float ry = zero ? 0.f : 1.f / uw[i];
+          Seg g;
+          g.lane = lane;
+          g.segbase = 0;
+          if (!one_row<32, MR>(b, g, wr)) {
+            int bp = 0x7fffffff;
+            int q[MR];
 #pragma unroll
-          for (int s = 0; s < MR; ++s) {
-            if (!act[s]) continue;
-            const float l = pan[s][i] * ry;
-            pan[s][i] = l;
+            for (int s = 0; s < MR; ++s) {
+              q[s] = (act[s] && key[s] == m) ? position_of(ord, lane + 32 * s, k) : 0x7fffffff;
+              bp = min(bp, q[s]);
+            }
+            __syncwarp();
+            bp = __reduce_min_sync(kFull, bp);
 #pragma unroll
-            for (int j = i + 1; j < PB; ++j) pan[s][j] = fmaf(-l, uw[j], pan[s][j]);
+            for (int s = 0; s < MR; ++s) {
+              win[s] = q[s] == bp;
+              b[s] = __ballot_sync(kFull, win[s]);
+            }
+            one_row<32, MR>(b, g, wr);
           }
+        } else {
+#pragma unroll
+          for (int s = 0; s < MR; ++s) win[s] = lane + 32 * s == k;
+        }
+#pragma unroll
+        for (int s = 0; s < MR; ++s) {
+          if (win[s]) {
+#pragma unroll
+            for (int j = 0; j < PB; j += 4) sts16(Fu + (lane + 32 * s) * RSF + (k0 + j) * 4, pan[s][j / 2], pan[s][j / 2 + 1]);
+            act[s] = 0u;
+            ord[k] = lane + 32 * s;
+          }
+        }
+        __syncwarp();
+        U2::E u[PB / 2];
+#pragma unroll
+        for (int j = i & ~3; j < PB; j += 4) {
+          const Unit2<U2::E> v = lds16(Fu + wr * RSF + (k0 + j) * 4, U2::E());
+          u[j / 2] = v.x;
+          u[j / 2 + 1] = v.y;
+        }
+        const float piv = U2::get(u[i / 2], i % 2);
+        const bool zero = SPD ? (!(piv > 0.f) || !isfinite(piv)) : (!(piv != 0.f) || !isfinite(piv));
+        if (zero && info == 0) info = k + 1;
+        float ry = rcp_in_range(piv);
+        const unsigned pb = abs_hi(piv);
+        if (pb - DivRange<float>::kLo > DivRange<float>::kHi - DivRange<float>::kLo) ry = 1.f / piv;
+        if (zero) ry = 0.f;
+        // retired rows are in shared memory: what their registers hold is not used again
+#pragma unroll
+        for (int s = 0; s < MR; ++s) {
+          const float l = x[s] * ry;
+          U2::set(pan[s][i / 2], i % 2, l);
+          if (i % 2 == 0) U2::set(pan[s][i / 2], 1, fmaf(-l, U2::get(u[i / 2], 1), U2::get(pan[s][i / 2], 1)));
+          const U2::E nl = U2::dup(-l);
+#pragma unroll
+          for (int j = i / 2 + 1; j < PB / 2; ++j) pan[s][j] = U2::fma(nl, u[j], pan[s][j]);
         }
       }
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
-        const int r = lane + 32 * s;
-        if (r >= NP) continue;
+        if (!act[s]) continue;
 #pragma unroll
-        for (int i0 = 0; i0 < PB; i0 += 4)
-          F4(r, k0 + i0) = make_float4(pan[s][i0], pan[s][i0 + 1], pan[s][i0 + 2], pan[s][i0 + 3]);
+        for (int i0 = 0; i0 < PB; i0 += 4) sts16(Fu + (lane + 32 * s) * RSF + (k0 + i0) * 4, pan[s][i0 / 2], pan[s][i0 / 2 + 1]);
       }
       __syncwarp();
       const int j1 = k0 + PB;
@@ -308,7 +333,13 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
           for (int i = 0; i < PB; ++i) {
             float acc = F(ordp[i], j);
 #pragma unroll
-            for (int i2 = 0; i2 < i; ++i2) acc = fmaf(-F(ordp[i], k0 + i2), u[i2], acc);
+            for (int i0 = 0; i0 < i; i0 += 4) {
+              const float4 l = F4(ordp[i], k0 + i0);
+              const float ll[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (i0 + e < i) acc = fmaf(-ll[e], u[i0 + e], acc);
+            }
             u[i] = acc;
             if (i > 0) F(ordp[i], j) = acc;
           }
@@ -318,21 +349,14 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
       // trailing update of the rows still active
       if (tc) {
         const int g = lane >> 2, tq = lane & 3;
+        unsigned ab[MR];
+#pragma unroll
+        for (int s = 0; s < MR; ++s) ab[s] = __ballot_sync(kFull, act[s] != 0);
 #pragma unroll
         for (int rt = 0; rt < NP / 16; ++rt) {
           const int ra = rt * 16 + g, rb = ra + 8;
           // rows still being updated: those not yet retired
-          bool sa, sb;
-          {
-            int va = act[0], vb = act[0];
-#pragma unroll
-            for (int t2 = 1; t2 < MR; ++t2) {
-              va = ((ra >> 5) == t2) ? (int)act[t2] : va;
-              vb = ((rb >> 5) == t2) ? (int)act[t2] : vb;
-            }
-            sa = __shfl_sync(kFull, va, ra & 31) != 0;
-            sb = __shfl_sync(kFull, vb, rb & 31) != 0;
-          }
+          const bool sa = (ab[ra >> 5] >> (ra & 31)) & 1u, sb = (ab[rb >> 5] >> (rb & 31)) & 1u;
           // L21 fragment (negated): rows ra/rb, panel columns k0 + [2tq, 2tq+1, 2tq+8, 2tq+9]
           unsigned af[4];
           af[0] = pack2(-F(ra, k0 + 2 * tq), -F(ra, k0 + 2 * tq + 1), f16);
@@ -356,87 +380,116 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
         // fp32 CUDA-core update, 8 columns at a time; each pivot-row segment is read
         // once for all of a lane's rows
         for (int jc = j1; jc < NP; jc += 8) {
-          float acc[MR][8];
+          U2::E acc[MR][4];
 #pragma unroll
           for (int s = 0; s < MR; ++s) {
             const int r = (lane + 32 * s < NP) ? lane + 32 * s : 0;
-            const float4 a0 = F4(r, jc), a1 = F4(r, jc + 4);
-            acc[s][0] = a0.x; acc[s][1] = a0.y; acc[s][2] = a0.z; acc[s][3] = a0.w;
-            acc[s][4] = a1.x; acc[s][5] = a1.y; acc[s][6] = a1.z; acc[s][7] = a1.w;
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+              const Unit2<U2::E> v = lds16(Fu + r * RSF + (jc + 2 * h) * 4, U2::E());
+              acc[s][h] = v.x;
+              acc[s][h + 1] = v.y;
+            }
           }
 #pragma unroll
           for (int i = 0; i < PB; ++i) {
-            float u[8];
-            const float4 v0 = F4(ordp[i], jc), v1 = F4(ordp[i], jc + 4);
-            u[0] = v0.x; u[1] = v0.y; u[2] = v0.z; u[3] = v0.w;
-            u[4] = v1.x; u[5] = v1.y; u[6] = v1.z; u[7] = v1.w;
+            const Unit2<U2::E> v0 = lds16(Fu + ordp[i] * RSF + jc * 4, U2::E());
+            const Unit2<U2::E> v1 = lds16(Fu + ordp[i] * RSF + (jc + 4) * 4, U2::E());
 #pragma unroll
-            for (int s = 0; s < MR; ++s)
-#pragma unroll
-              for (int q = 0; q < 8; ++q) acc[s][q] = fmaf(-pan[s][i], u[q], acc[s][q]);
+            for (int s = 0; s < MR; ++s) {
+              const U2::E nl = U2::dup(-U2::get(pan[s][i / 2], i % 2));
+              acc[s][0] = U2::fma(nl, v0.x, acc[s][0]);
+              acc[s][1] = U2::fma(nl, v0.y, acc[s][1]);
+              acc[s][2] = U2::fma(nl, v1.x, acc[s][2]);
+              acc[s][3] = U2::fma(nl, v1.y, acc[s][3]);
+            }
           }
 #pragma unroll
           for (int s = 0; s < MR; ++s) {
-            const int r = lane + 32 * s;
-            const bool on = act[s] && r < NP;
-            if (!on) continue;
-            F4(r, jc) = make_float4(acc[s][0], acc[s][1], acc[s][2], acc[s][3]);
-            F4(r, jc + 4) = make_float4(acc[s][4], acc[s][5], acc[s][6], acc[s][7]);
+            if (!act[s]) continue;
+            sts16(Fu + (lane + 32 * s) * RSF + jc * 4, acc[s][0], acc[s][1]);
+            sts16(Fu + (lane + 32 * s) * RSF + (jc + 4) * 4, acc[s][2], acc[s][3]);
           }
         }
       }
       __syncwarp();
     }
     if (p.info && lane == 0) p.info[m] = info;
-    // reciprocal pivots U(ord[k], k)
+    // from here on lane l owns positions l and l + 32: their rows of the factor and
+    // reciprocal pivots
+    __syncwarp();
+    unsigned rowp[MR];
+    float rinv[MR];
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
-      const int k = lane + 32 * s;
-      if (k < NP) rinv[k] = 1.f / F(ord[k], k);
+      const int k = lane + 32 * s < NP ? lane + 32 * s : NP - 1;
+      rowp[s] = Fu + ord[k] * RSF;
+      rinv[s] = 1.f / F(ord[k], k);
     }
-    __syncwarp();
 
     // ---------------------------------------- 3./4. solve and refine in fp64
-    // lowsolve(v): v = D_r * rhs by physical row in; the scaled solution by physical row out
+    // lowsolve(v): v = D_r * rhs by physical row in; the scaled solution by position out
     auto lowsolve = [&](float* v) {
-      // forward: y_k at physical row ord[k]; rows retired after k take -L(row,k) y_k
-      for (int k = 0; k < NP; ++k) {
-        const int pk = ord[k];
-        float vk = v[0];
 #pragma unroll
-        for (int t2 = 1; t2 < MR; ++t2) vk = ((pk >> 5) == t2) ? v[t2] : vk;
-        const float y = __shfl_sync(kFull, vk, pk & 31);
+      for (int s = 0; s < MR; ++s)
+        if (lane + 32 * s < NP) rsd[lane + 32 * s] = v[s];
+      __syncwarp();
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = lane + 32 * s;
-          if (pos[s] > k && r < NP) v[s] = fmaf(-F(r, k), y, v[s]);
+      for (int s = 0; s < MR; ++s) v[s] = lane + 32 * s < NP ? rsd[ord[lane + 32 * s]] : 0.f;
+      // forward: y_k, then positions after k take -L(k', k) y_k
+#pragma unroll
+      for (int t2 = 0; t2 < MR; ++t2) {
+        const int top = 32 * (t2 + 1) < NP ? 32 * (t2 + 1) : NP;
+#pragma unroll 2
+        for (int kb = 32 * t2; kb < top; kb += 4) {
+          Unit2<U2::E> lv[MR];
+#pragma unroll
+          for (int s = t2; s < MR; ++s) lv[s] = lds16(rowp[s] + kb * 4, U2::E());
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int kl = kb + q - 32 * t2;
+            const float y = __shfl_sync(kFull, v[t2], kl);
+#pragma unroll
+            for (int s = t2; s < MR; ++s) {
+              const float w = fmaf(-U2::get(q / 2 ? lv[s].y : lv[s].x, q % 2), y, v[s]);
+              v[s] = (s > t2 || lane > kl) ? w : v[s];
+            }
+          }
         }
       }
-      // backward: x_k = y_k / U(ord[k],k); rows retired before k take -U(row,k) x_k
-      for (int k = NP - 1; k >= 0; --k) {
-        const int pk = ord[k];
-        float vk = v[0];
+      // backward: x_k = y_k / U(k, k), then positions before k take -U(k', k) x_k
 #pragma unroll
-        for (int t2 = 1; t2 < MR; ++t2) vk = ((pk >> 5) == t2) ? v[t2] : vk;
-        const float x = __shfl_sync(kFull, vk, pk & 31) * rinv[k];
+      for (int t2 = MR - 1; t2 >= 0; --t2) {
+        const int top = 32 * (t2 + 1) < NP ? 32 * (t2 + 1) : NP;
+#pragma unroll 2
+        for (int kb = top - 4; kb >= 32 * t2; kb -= 4) {
+          Unit2<U2::E> uv[MR];
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = lane + 32 * s;
-          if (r == pk) v[s] = x;
-          else if (pos[s] < k && r < NP) v[s] = fmaf(-F(r, k), x, v[s]);
+          for (int s = 0; s <= t2; ++s) uv[s] = lds16(rowp[s] + kb * 4, U2::E());
+#pragma unroll
+          for (int q = 3; q >= 0; --q) {
+            const int kl = kb + q - 32 * t2;
+            const float x = __shfl_sync(kFull, v[t2] * rinv[t2], kl);
+#pragma unroll
+            for (int s = 0; s <= t2; ++s) {
+              const float w = fmaf(-U2::get(q / 2 ? uv[s].y : uv[s].x, q % 2), x, v[s]);
+              v[s] = (s < t2 || lane < kl) ? w : v[s];
+            }
+          }
         }
       }
+#pragma unroll
+      for (int s = 0; s < MR; ++s) v[s] = v[s] * rinv[s];
       __syncwarp();
     };
-    // the solution component of unknown pos[s] sits at physical row r; unscale into xs
+    // unscale the solution into xs
     auto gather = [&](const float* v, bool add) {
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
-        const int r = lane + 32 * s;
-        if (r >= NP) continue;
-        const int kk = pos[s];
+        const int kk = lane + 32 * s;
+        if (kk >= n) continue;
         const double xk = (double)v[s] * (double)csc[kk];
-        if (kk < n) xs[kk] = add ? xs[kk] + xk : xk;
+        xs[kk] = add ? xs[kk] + xk : xk;
       }
       __syncwarp();
     };

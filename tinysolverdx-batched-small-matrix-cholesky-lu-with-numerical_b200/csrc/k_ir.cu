@@ -20,9 +20,9 @@ int launch_ir(const dev::IrArgs& a, cudaStream_t st) {
   constexpr int SMEM = WPC * C::WARPB;
   auto kern = dev::ir_kernel<NP, SPD, WPC>;
   if (int rc = prepare(kern, SMEM)) return rc;
-  const long long ctas = (a.batch + WPC - 1) / WPC;
-  const int grid = grid_for(kern, SMEM, ctas, WPC * 32);
-  kern<<<grid, WPC * 32, SMEM, st>>>(a);
+  const int wpc = warps_for(a.batch, WPC), smem = wpc * C::WARPB;
+  const int grid = grid_for(kern, smem, (a.batch + wpc - 1) / wpc, wpc * 32);
+  kern<<<grid, wpc * 32, smem, st>>>(a);
   launch_counter().fetch_add(1);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_cuda_error(e, "kernel launch"); return -5; }

@@ -36,7 +36,7 @@ int factor_metric(const double* A, const double* F, const int* piv, int n, int64
   if (batch == 0) return TSDX_OK;
   if (!A || !F || !out || (!CHOL && !piv)) return TSDX_ERR_NULL;
   auto kern = dev::factor_bwd_kernel<CHOL>;
-  const int wpc = warps_for(dev::met_factor_bytes(n)), smem = wpc * dev::met_factor_bytes(n);
+  const int wpc = host::warps_for(batch, warps_for(dev::met_factor_bytes(n))), smem = wpc * dev::met_factor_bytes(n);
   if (int rc = host::prepare(kern, smem)) return rc;
   const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
@@ -50,7 +50,7 @@ API int tsdx_cuda_solve_backward_error_f64(const double* A, const double* x, con
   if (batch == 0) return TSDX_OK;
   if (!A || !x || !b || !out) return TSDX_ERR_NULL;
   auto kern = dev::solve_bwd_kernel;
-  const int wpc = warps_for(dev::met_solve_bytes(n)), smem = wpc * dev::met_solve_bytes(n);
+  const int wpc = host::warps_for(batch, warps_for(dev::met_solve_bytes(n))), smem = wpc * dev::met_solve_bytes(n);
   if (int rc = host::prepare(kern, smem)) return rc;
   const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);

@@ -879,10 +879,59 @@ __device__ __forceinline__ void rows_load(unsigned char* M, const MatJob<T>& j, 
   __syncwarp();
 }
 
-// The general body (blk.cuh), kept out of line: few matrices need it.
-template <class T, int NP, int NRHS, int GO>
-__device__ __noinline__ void lu_general(unsigned Mu, MatJob<T> j, Seg g) {
-  lu_matrix<T, NP, NRHS, GO>(static_cast<unsigned char*>(__cvta_shared_to_generic(Mu)), j, g);
+// The LU of one matrix staged at shared address Mu (NP rows of RS bytes, NC columns, the
+// right-hand sides included) for every input, one step at a time in shared memory: what
+// lu_rows leaves to it is a zero pivot over a column that holds -0 or NaN. The reference's
+// loop (kernels.hpp:91-119) with the rows behind a map; ord[k] <- the row at position k.
+// Returns info. Out of line and sized at run time: few matrices need it.
+template <class T>
+__device__ __noinline__ int lu_plain(unsigned Mu, int RS, int NP, int NC, unsigned ordu, int lsl, int G) {
+  using K = typename KeyT<T>::U;
+  unsigned char* M = static_cast<unsigned char*>(__cvta_shared_to_generic(Mu));
+  int* ord = static_cast<int*>(__cvta_shared_to_generic(ordu));
+  auto row = [&](int p) { return reinterpret_cast<T*>(M + ord[p] * RS); };
+  for (int p = lsl; p < NP; p += G) ord[p] = p;
+  __syncwarp();
+  int info = 0;
+  for (int k = 0; k < NP; ++k) {
+    K bk = 0;
+    int bp = 0x7fffffff;
+    for (int p = k + lsl; p < NP; p += G) {
+      const T v = row(p)[k];
+      const K key = isnan(v) ? (p == k ? ~K(0) : K(0)) : key_bits(v) + 1;
+      if (key > bk || (key == bk && p < bp)) {
+        bk = key;
+        bp = p;
+      }
+    }
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const K ok = __shfl_xor_sync(kFull, bk, o);
+      const int op = __shfl_xor_sync(kFull, bp, o);
+      if (ok > bk || (ok == bk && op < bp)) {
+        bk = ok;
+        bp = op;
+      }
+    }
+    if (lsl == 0) {
+      const int t = ord[k];
+      ord[k] = ord[bp];
+      ord[bp] = t;
+    }
+    __syncwarp();
+    if (bk == K(1)) {
+      info = info == 0 ? k + 1 : info;
+    } else {
+      const T* u = row(k);
+      for (int p = k + 1 + lsl; p < NP; p += G) {
+        T* x = row(p);
+        const T l = div_(x[k], u[k]);
+        x[k] = l;
+        for (int c = k + 1; c < NC; ++c) x[c] = fma_(-l, u[c], x[c]);
+      }
+    }
+    __syncwarp();
+  }
+  return info;
 }
 
 template <class T, int NP, int NRHS, int GO>
@@ -918,8 +967,15 @@ __device__ __forceinline__ void lu_rows(unsigned char* M, const MatJob<T>& j, co
     __syncwarp();
   }
   if (__any_sync(kFull, st.bad)) {  // nothing has left shared memory yet: start over
-    lu_general<T, NP, NRHS, GO>(Mu, j, g);
-    return;
+    T rhs[MR][NRHS > 0 ? NRHS : 1];
+    rows_load<T, NP, NRHS, GO>(M, j, g, rhs);
+#pragma unroll
+    for (int s = 0; s < MR; ++s)
+#pragma unroll
+      for (int c = 0; c < NRHS; ++c)
+        if (g.lsl + G * s < NP) sts(Mu + (g.lsl + G * s) * RS + (NP + c) * int(sizeof(T)), rhs[s][c]);
+    __syncwarp();
+    st.info = lu_plain<T>(Mu, RS, NP, C::NC, Mu + C::MAT, g.lsl, G);
   }
   if constexpr (NRHS > 0) rows_backsolve<T, NP, NRHS, false, GO>(M, ord, j, g);
   if (j.live) {
@@ -1003,7 +1059,7 @@ __device__ __forceinline__ unsigned rows_constants(unsigned char* at) {
   return (unsigned)__cvta_generic_to_shared(at);
 }
 
-// Dense batch: one persistent CTA of WPC warps per SM slot; every round each segment
+// Dense batch: one persistent CTA of at most WPC warps per SM; every round each segment
 // takes the next matrix.
 template <class T, int NP, int NRHS, int WPC, bool CHOL, int GO = 0>
 __global__ void __launch_bounds__(WPC * 32, 1) blk_kernel(SolveArgs<T> p) {
@@ -1013,18 +1069,17 @@ __global__ void __launch_bounds__(WPC * 32, 1) blk_kernel(SolveArgs<T> p) {
   __shared__ __align__(16) unsigned char consts[kRowConst];
   // the warp index through a shuffle, so that the compiler knows it to be uniform: the
   // warp-wide operations below then need no divergence checks
-  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   Seg g;
   g.lane = lane;
   g.lsl = lane & (G - 1);
   g.segbase = (lane / G) * G;
-  g.segmask = (G == 32) ? kFull : (((1u << (G & 31)) - 1u) << g.segbase);
   g.zrow = rows_constants(consts);
   unsigned char* M = smem + warp * C::WARPB + (lane / G) * C::SEGB;
   const long long nn = (long long)p.n * p.n;
-  const long long per_round = (long long)gridDim.x * WPC * S;
+  const long long per_round = (long long)gridDim.x * wpc * S;
   // warps own disjoint shared memory, so they run their rounds without a block barrier
-  for (long long base = (long long)blockIdx.x * WPC * S; base < p.batch; base += per_round) {
+  for (long long base = (long long)blockIdx.x * wpc * S; base < p.batch; base += per_round) {
     const long long m = base + (long long)warp * S + lane / G;
     {
       // this warp's next unit heads for L2 while this one is solved

@@ -101,15 +101,15 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> 
   using C = TrsCfg<double, NP>;
   constexpr int RS = C::RS, NB = NP / 8;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   const int fr = lane >> 2, fq = lane & 3;
   unsigned char* M = smem + warp * C::WARPB;
   const int* perm = reinterpret_cast<const int*>(M + C::OFF_PERM) + NP;
   auto at = [&](int r, int c) -> double { return *reinterpret_cast<const double*>(M + r * RS + c * 8); };
   const int n = p.n;
-  const long long nn = (long long)n * n, step = (long long)gridDim.x * WPC;
+  const long long nn = (long long)n * n, step = (long long)gridDim.x * wpc;
 
-  for (long long m = (long long)blockIdx.x * WPC + warp; m < p.batch; m += step) {
+  for (long long m = (long long)blockIdx.x * wpc + warp; m < p.batch; m += step) {
     if (lane == 0 && m + step < p.batch) {
       prefetch_l2(p.A + (m + step) * nn, nn * 8);
       prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 8);
@@ -255,14 +255,14 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
   constexpr int RS = C::RS, XB = C::XB, MR = (NP + 31) / 32, NU = NRHS > 1 ? NRHS / 2 : 1;
   static_assert(NRHS == 1 || NRHS % 4 == 0, "whole 16-byte vectors");
   extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   unsigned char* M = smem + warp * C::WARPB;
   const unsigned Mu = (unsigned)__cvta_generic_to_shared(M), Xu = Mu + C::OFF_X;
   const int* perm = reinterpret_cast<const int*>(M + C::OFF_PERM) + NP;
   const int n = p.n;
-  const long long nn = (long long)n * n, step = (long long)gridDim.x * WPC;
+  const long long nn = (long long)n * n, step = (long long)gridDim.x * wpc;
 
-  for (long long m = (long long)blockIdx.x * WPC + warp; m < p.batch; m += step) {
+  for (long long m = (long long)blockIdx.x * wpc + warp; m < p.batch; m += step) {
     if (lane == 0 && m + step < p.batch) {
       prefetch_l2(p.A + (m + step) * nn, nn * 4);
       prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 4);

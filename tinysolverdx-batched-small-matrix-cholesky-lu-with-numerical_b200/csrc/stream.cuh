@@ -137,7 +137,6 @@ __device__ __forceinline__ void stream_unit(unsigned char* M, const StreamArgs<T
   g.lane = lane;
   g.lsl = lane & (G - 1);
   g.segbase = (lane / G) * G;
-  g.segmask = (G == 32) ? kFull : (((1u << (G & 31)) - 1u) << g.segbase);
   g.zrow = zrow;
   const int idx = first + lane / G;
   MatJob<T> j;

@@ -1,6 +1,6 @@
 // Host side of the uneven stream (stream.cuh): counting sort into buckets + persistent
-// drains (one per order class above order 16, one for n <= 16), instantiated per element type in k_stream_f32.cu /
-// k_stream_f64.cu.
+// drains (one per order class above order 16, one for n <= 16), instantiated per element
+// type in k_stream_*.cu.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -51,6 +51,25 @@ int launch_drain(const dev::StreamArgs<T>& a, cudaStream_t st) {
 }
 }  // namespace
 
+// The drains of the larger orders (above 40) and of the others, largest first; instantiated
+// in translation units of their own (k_stream_*_hi.cu, k_stream_*_lo.cu), which compile
+// side by side.
+template <class T> int launch_drains_hi(const dev::StreamArgs<T>& a, cudaStream_t st);
+template <class T> int launch_drains_lo(const dev::StreamArgs<T>& a, cudaStream_t st);
+#define TSDX_STREAM_HI(T)                                                               \
+  template <> int launch_drains_hi<T>(const dev::StreamArgs<T>& a, cudaStream_t st) {   \
+    int rc = launch_drain<T, 7, 7>(a, st);                                              \
+    if (!rc) rc = launch_drain<T, 6, 6>(a, st);                                         \
+    return rc ? rc : launch_drain<T, 5, 5>(a, st);                                      \
+  }
+#define TSDX_STREAM_LO(T)                                                               \
+  template <> int launch_drains_lo<T>(const dev::StreamArgs<T>& a, cudaStream_t st) {   \
+    int rc = launch_drain<T, 4, 4>(a, st);                                              \
+    if (!rc) rc = launch_drain<T, 3, 3>(a, st);                                         \
+    if (!rc) rc = launch_drain<T, 2, 2>(a, st);                                         \
+    return rc ? rc : launch_drain<T, 0, 1>(a, st);                                      \
+  }
+
 constexpr long long stream_scratch_bytes_of(long long count) { return (4LL * dev::kStreamBuckets + 2 + count) * 4; }
 
 template <class T>
@@ -80,13 +99,8 @@ int run_stream(dev::StreamArgs<T> a, void* scratch, long long scratch_bytes, cud
   // n <= 16. Shared memory per warp is sized for each class, so the smaller orders keep
   // more warps per SM, and each drain carries only its class's code variants (one
   // drain over n <= 48 carried about 40 and stalled on instruction fetch).
-  if (e == cudaSuccess) rc = launch_drain<T, 7, 7>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 6, 6>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 5, 5>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 4, 4>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 3, 3>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 2, 2>(a, st);
-  if (e == cudaSuccess && !rc) rc = launch_drain<T, 0, 1>(a, st);
+  if (e == cudaSuccess) rc = launch_drains_hi<T>(a, st);
+  if (e == cudaSuccess && !rc) rc = launch_drains_lo<T>(a, st);
   if (e == cudaSuccess && !rc) {
     launch_counter().fetch_add(10);
     e = cudaGetLastError();
