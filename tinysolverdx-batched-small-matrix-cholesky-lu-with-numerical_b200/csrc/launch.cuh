@@ -46,8 +46,8 @@ int grid_for(Kern kern, int smem, long long ctas_needed, int threads = 128) {
 }
 
 // Warps per CTA for this many work units of one warp each: the kernel's WPC, fewer when
-// they would leave SMs without a CTA (posv float64 order 7, 5,959 matrices on 47 of 148
-// SMs: PLACEHOLDER).
+// they would leave SMs without a CTA (float64 Cholesky of order 7, 5,959 matrices: 47 of
+// 148 SMs with full CTAs).
 inline int warps_for(long long units, int wpc) {
   int devi = 0;
   cudaGetDevice(&devi);

@@ -201,9 +201,7 @@ struct RowCfg {
   static constexpr int PW = NP <= 16 ? NP : 8;
   static constexpr int LASTW = NCV - (NP - 1) / PW * PW;       // the last panel holds the right-hand sides
   static constexpr int RW = LASTW > PW ? LASTW : PW;
-  // steps per phase: a phase updates a fixed width, in a rolled loop of VN steps
-  static constexpr int PH = NP <= 16 ? VN : 8;
-  static_assert(NP % VN == 0 && PW % VN == 0, "whole vectors of matrix columns");
+  static_assert(NP % VN == 0 && NP % PW == 0 && PW % VN == 0, "whole vectors of matrix columns, whole panels");
 };
 
 // The position, before step k, of a row still active: its own index, unless an earlier
@@ -373,7 +371,7 @@ __device__ __forceinline__ void lu_rows_group(unsigned Mu, RowRegs<T, NP, NRHS, 
       if (win[s]) {
         unrolled<0, W, VN>([&](auto qc) {
           constexpr int q = decltype(qc)::value;
-          if (!ROLLED || q < W - R::PH + VN || k0 + q < cend) sts16<q * TS>(own + G * RS * s, a[s][q / UN], a[s][q / UN + 1]);
+          if (!ROLLED || q < W - R::PW + VN || k0 + q < cend) sts16<q * TS>(own + G * RS * s, a[s][q / UN], a[s][q / UN + 1]);
         });
         st.act[s] = 0u;
       }
@@ -594,14 +592,14 @@ __device__ __forceinline__ void chol_rows_group(unsigned Mu, RowRegs<T, NP, 0, G
   }
 }
 
-// W staged columns from C0 on into registers.
-template <class T, int G, int MR, int RS, int NP, int C0, int W, int NU>
-__device__ __forceinline__ void rows_fetch(unsigned Mu, typename Unit<T>::E (&a)[MR][NU], const Seg& g) {
+// W staged columns from c0 on into registers.
+template <class T, int G, int MR, int RS, int NP, int W, int NU>
+__device__ __forceinline__ void rows_fetch(unsigned Mu, typename Unit<T>::E (&a)[MR][NU], int c0, const Seg& g) {
   using E = typename Unit<T>::E;
 #pragma unroll
   for (int s = 0; s < MR; ++s) {
     const int r = g.lsl + G * s;
-    const unsigned row = Mu + (r < NP ? r : NP - 1) * RS + C0 * int(sizeof(T));
+    const unsigned row = Mu + (r < NP ? r : NP - 1) * RS + c0 * int(sizeof(T));
 #pragma unroll
     for (int q = 0; q < W / Unit<T>::n; q += 2) {
       const Unit2<E> v = lds16(row + q * 8, E());
@@ -611,56 +609,60 @@ __device__ __forceinline__ void rows_fetch(unsigned Mu, typename Unit<T>::E (&a)
   }
 }
 
-// All panels from column C0 on, and within a panel all phases from column K0 on.
-template <class T, int NP, int NRHS, int GO, int K0, int CEND, int KEND>
+// All phases of an order whose whole rows are in registers, from column K0 on.
+template <class T, int NP, int NRHS, int GO, int K0>
 __device__ __forceinline__ void lu_rows_phases(unsigned Mu, RowRegs<T, NP, NRHS, GO>& a,
                                                RowState<BlkCfg<T, NP, NRHS, GO>::MR>& st, int* ord, const Seg& g) {
   using R = RowCfg<T, NP, NRHS, GO>;
-  if constexpr (K0 < KEND) {
-    constexpr int W = CEND - K0, END = K0 + R::PH < KEND ? K0 + R::PH : KEND;
-    if constexpr (R::PH == R::VN) {
-      lu_rows_group<T, NP, NRHS, GO, W, false>(Mu, a, st, K0, CEND, ord, g);
-    } else {
-#pragma unroll 1
-      for (int k0 = K0; k0 < END; k0 += R::VN) lu_rows_group<T, NP, NRHS, GO, W, true>(Mu, a, st, k0, CEND, ord, g);
-    }
-    lu_rows_phases<T, NP, NRHS, GO, END, CEND, KEND>(Mu, a, st, ord, g);
+  if constexpr (K0 < NP) {
+    lu_rows_group<T, NP, NRHS, GO, R::NCV - K0, false>(Mu, a, st, K0, R::NCV, ord, g);
+    lu_rows_phases<T, NP, NRHS, GO, K0 + R::VN>(Mu, a, st, ord, g);
   }
 }
-template <class T, int NP, int NRHS, int GO, int C0>
-__device__ __forceinline__ void lu_rows_panels(unsigned Mu, RowRegs<T, NP, NRHS, GO>& a,
-                                               RowState<BlkCfg<T, NP, NRHS, GO>::MR>& st, int* ord, const Seg& g) {
+// The panel at c0, W columns of it (the last one's with the right-hand sides).
+template <class T, int NP, int NRHS, int GO, int W>
+__device__ __forceinline__ void lu_rows_panel(unsigned Mu, RowRegs<T, NP, NRHS, GO>& a,
+                                              RowState<BlkCfg<T, NP, NRHS, GO>::MR>& st, int c0, int* ord, const Seg& g) {
   using C = BlkCfg<T, NP, NRHS, GO>;
   using R = RowCfg<T, NP, NRHS, GO>;
-  if constexpr (C0 < NP) {
-    constexpr int KEND = C0 + R::PW < NP ? C0 + R::PW : NP, CEND = KEND < NP ? KEND : R::NCV;
-    if constexpr (C0 > 0) {
-      __syncwarp();
-      rows_fetch<T, C::G, C::MR, C::RS, NP, C0, CEND - C0>(Mu, a, g);
-      if (__any_sync(kFull, st.zmask != 0)) lu_rows_catch_up<T, NP, NRHS, GO, CEND - C0, true>(Mu, a, st.zmask, C0, ord, g);
-      else lu_rows_catch_up<T, NP, NRHS, GO, CEND - C0, false>(Mu, a, 0, C0, ord, g);
-    }
-    lu_rows_phases<T, NP, NRHS, GO, C0, CEND, KEND>(Mu, a, st, ord, g);
-    lu_rows_panels<T, NP, NRHS, GO, KEND>(Mu, a, st, ord, g);
+  if (c0 > 0) {
+    __syncwarp();
+    rows_fetch<T, C::G, C::MR, C::RS, NP, W>(Mu, a, c0, g);
+    if (__any_sync(kFull, st.zmask != 0)) lu_rows_catch_up<T, NP, NRHS, GO, W, true>(Mu, a, st.zmask, c0, ord, g);
+    else lu_rows_catch_up<T, NP, NRHS, GO, W, false>(Mu, a, 0, c0, ord, g);
+  }
+#pragma unroll 1
+  for (int k0 = c0; k0 < c0 + R::PW; k0 += R::VN) lu_rows_group<T, NP, NRHS, GO, W, true>(Mu, a, st, k0, c0 + W, ord, g);
+}
+// Panels in a rolled loop: a copy of the code per panel, with its column a constant, does
+// not fit the instruction cache (order 64, 8 right-hand sides: Cholesky 13,900 instructions
+// instead of 3,300, LU 10,700 instead of 5,600). float32 posv n = 45, 50,000 matrices, 3
+// right-hand sides 1253 -> 1056 us, gesv n = 32, 262,144 1691 -> 1621, a mixed stream of
+// 262,144 matrices 4946 -> 4323 (passes with their input copies).
+template <class T, int NP, int NRHS, int GO>
+__device__ __forceinline__ void lu_rows_panels(unsigned Mu, RowRegs<T, NP, NRHS, GO>& a,
+                                               RowState<BlkCfg<T, NP, NRHS, GO>::MR>& st, int* ord, const Seg& g) {
+  using R = RowCfg<T, NP, NRHS, GO>;
+  if constexpr (R::PW == NP) {
+    lu_rows_phases<T, NP, NRHS, GO, 0>(Mu, a, st, ord, g);
+  } else {
+    constexpr int LAST = R::LASTW == R::PW ? NP : NP - R::PW;  // from there on with right-hand sides
+#pragma unroll 1
+    for (int c0 = 0; c0 < LAST; c0 += R::PW) lu_rows_panel<T, NP, NRHS, GO, R::PW>(Mu, a, st, c0, ord, g);
+    if constexpr (LAST < NP) lu_rows_panel<T, NP, NRHS, GO, R::LASTW>(Mu, a, st, LAST, ord, g);
   }
 }
-template <class T, int NP, int NRHS, int GO, int K0, int KEND>
+template <class T, int NP, int NRHS, int GO, int K0>
 __device__ __forceinline__ void chol_rows_phases(unsigned Mu, RowRegs<T, NP, 0, GO>& a,
                                                  T (&b)[BlkCfg<T, NP, NRHS, GO>::MR][NRHS > 0 ? NRHS : 1], int& info,
                                                  typename Unit<T>::E nz, const Seg& g) {
   using R = RowCfg<T, NP, NRHS, GO>;
-  if constexpr (K0 < KEND) {
-    constexpr int W = KEND - K0, END = K0 + R::PH < KEND ? K0 + R::PH : KEND;
-    if constexpr (R::PH == R::VN) {
-      chol_rows_group<T, NP, NRHS, GO, W>(Mu, a, b, K0, info, nz, g);
-    } else {
-#pragma unroll 1
-      for (int k0 = K0; k0 < END; k0 += R::VN) chol_rows_group<T, NP, NRHS, GO, W>(Mu, a, b, k0, info, nz, g);
-    }
-    chol_rows_phases<T, NP, NRHS, GO, END, KEND>(Mu, a, b, info, nz, g);
+  if constexpr (K0 < NP) {
+    chol_rows_group<T, NP, NRHS, GO, NP - K0>(Mu, a, b, K0, info, nz, g);
+    chol_rows_phases<T, NP, NRHS, GO, K0 + R::VN>(Mu, a, b, info, nz, g);
   }
 }
-template <class T, int NP, int NRHS, int GO, int C0>
+template <class T, int NP, int NRHS, int GO>
 __device__ __forceinline__ void chol_rows_panels(unsigned Mu, RowRegs<T, NP, 0, GO>& a,
                                                  T (&b)[BlkCfg<T, NP, NRHS, GO>::MR][NRHS > 0 ? NRHS : 1], int& info,
                                                  typename Unit<T>::E nz, const Seg& g) {
@@ -668,41 +670,45 @@ __device__ __forceinline__ void chol_rows_panels(unsigned Mu, RowRegs<T, NP, 0, 
   using R = RowCfg<T, NP, NRHS, GO>;
   using U = Unit<T>;
   using E = typename U::E;
-  constexpr int G = C::G, MR = C::MR, RS = C::RS, VN = R::VN, UN = U::n, TS = int(sizeof(T));
-  if constexpr (C0 < NP) {
-    constexpr int KEND = C0 + R::PW < NP ? C0 + R::PW : NP, W = KEND - C0;
-    if constexpr (C0 > 0) {
-      __syncwarp();
-      // rows above the panel take their place in shared memory only: what their
-      // registers hold is never used
-      rows_fetch<T, G, MR, RS, NP, C0, W>(Mu, a, g);
+  constexpr int G = C::G, MR = C::MR, RS = C::RS, VN = R::VN, UN = U::n, TS = int(sizeof(T)), W = R::PW;
+  if constexpr (W == NP) {
+    chol_rows_phases<T, NP, NRHS, GO, 0>(Mu, a, b, info, nz, g);
+  } else {
 #pragma unroll 1
-      for (int k0 = 0; k0 < C0; k0 += VN) {
-        Unit2<E> lv[MR];
+    for (int c0 = 0; c0 < NP; c0 += W) {
+      if (c0 > 0) {
+        __syncwarp();
+        // rows above the panel take their place in shared memory only: what their
+        // registers hold is never used
+        rows_fetch<T, G, MR, RS, NP, W>(Mu, a, c0, g);
+#pragma unroll 1
+        for (int k0 = 0; k0 < c0; k0 += VN) {
+          Unit2<E> lv[MR];
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int r = g.lsl + G * s;
-          lv[s] = lds16(Mu + (r < NP ? r : NP - 1) * RS + k0 * TS, E());
-        }
+          for (int s = 0; s < MR; ++s) {
+            const int r = g.lsl + G * s;
+            lv[s] = lds16(Mu + (r < NP ? r : NP - 1) * RS + k0 * TS, E());
+          }
 #pragma unroll
-        for (int i = 0; i < VN; ++i) {
-          E nl[MR];
+          for (int i = 0; i < VN; ++i) {
+            E nl[MR];
 #pragma unroll
-          for (int s = 0; s < MR; ++s) nl[s] = U::dup(-U::get(i / UN == 0 ? lv[s].x : lv[s].y, i % UN));
+            for (int s = 0; s < MR; ++s) nl[s] = U::dup(-U::get(i / UN == 0 ? lv[s].x : lv[s].y, i % UN));
 #pragma unroll
-          for (int q = 0; q < W; q += VN) {
-            const Unit2<E> u = lds16(Mu + (k0 + i) * RS + (C0 + q) * TS, E());
+            for (int q = 0; q < W; q += VN) {
+              const Unit2<E> u = lds16(Mu + (k0 + i) * RS + (c0 + q) * TS, E());
 #pragma unroll
-            for (int s = 0; s < MR; ++s) {
-              a[s][q / UN] = NP <= 16 ? U::fma(nl[s], u.x, a[s][q / UN]) : U::muladd(nl[s], u.x, a[s][q / UN], nz);
-              a[s][q / UN + 1] = NP <= 16 ? U::fma(nl[s], u.y, a[s][q / UN + 1]) : U::muladd(nl[s], u.y, a[s][q / UN + 1], nz);
+              for (int s = 0; s < MR; ++s) {
+                a[s][q / UN] = U::muladd(nl[s], u.x, a[s][q / UN], nz);
+                a[s][q / UN + 1] = U::muladd(nl[s], u.y, a[s][q / UN + 1], nz);
+              }
             }
           }
         }
       }
+#pragma unroll 1
+      for (int k0 = c0; k0 < c0 + W; k0 += VN) chol_rows_group<T, NP, NRHS, GO, W>(Mu, a, b, k0, info, nz, g);
     }
-    chol_rows_phases<T, NP, NRHS, GO, C0, KEND>(Mu, a, b, info, nz, g);
-    chol_rows_panels<T, NP, NRHS, GO, KEND>(Mu, a, b, info, nz, g);
   }
 }
 
@@ -947,7 +953,7 @@ __device__ __forceinline__ void lu_rows(unsigned char* M, const MatJob<T>& j, co
     RowRegs<T, NP, NRHS, GO> a;
     T rhs[MR][NRHS > 0 ? NRHS : 1];
     rows_load<T, NP, NRHS, GO>(M, j, g, rhs);
-    rows_fetch<T, G, MR, RS, NP, 0, R::PW>(Mu, a, g);
+    rows_fetch<T, G, MR, RS, NP, R::PW>(Mu, a, 0, g);
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
       const int r = g.lsl + G * s;
@@ -963,7 +969,7 @@ __device__ __forceinline__ void lu_rows(unsigned char* M, const MatJob<T>& j, co
     st.zmask = 0;
 #pragma unroll
     for (int s = 0; s < MR; ++s) st.act[s] = g.lsl + G * s < NP ? 0x7fffffffu : 0u;
-    lu_rows_panels<T, NP, NRHS, GO, 0>(Mu, a, st, ord, g);
+    lu_rows_panels<T, NP, NRHS, GO>(Mu, a, st, ord, g);
     __syncwarp();
   }
   if (__any_sync(kFull, st.bad)) {  // nothing has left shared memory yet: start over
@@ -1010,10 +1016,10 @@ __device__ __forceinline__ void chol_rows(unsigned char* M, const MatJob<T>& j, 
   RowRegs<T, NP, 0, GO> a;
   T b[MR][NRHS > 0 ? NRHS : 1];
   rows_load<T, NP, NRHS, GO>(M, j, g, b);
-  rows_fetch<T, G, MR, RS, NP, 0, RowCfg<T, NP, NRHS, GO>::PW>(Mu, a, g);
+  rows_fetch<T, G, MR, RS, NP, RowCfg<T, NP, NRHS, GO>::PW>(Mu, a, 0, g);
   int info = 0;
   __syncwarp();  // every row is in registers before the first column overwrites its row
-  chol_rows_panels<T, NP, NRHS, GO, 0>(Mu, a, b, info, lds16(g.zrow + kZeroRow, typename U::E()).x, g);
+  chol_rows_panels<T, NP, NRHS, GO>(Mu, a, b, info, lds16(g.zrow + kZeroRow, typename U::E()).x, g);
   __syncwarp();
   if constexpr (NRHS > 0) rows_backsolve<T, NP, NRHS, true, GO>(M, nullptr, j, g);
   if (j.live) {
