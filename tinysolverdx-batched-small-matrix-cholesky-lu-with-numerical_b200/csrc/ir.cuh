@@ -121,18 +121,18 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
     float rsc[MR];
     {
       // coalesced row reads (lane c holds columns c, c + 32), unscaled fp32 copy
-#pragma unroll 8
-      for (int r = 0; r < n; ++r) {
-        const double* row = Ag + (long long)r * n;
+#pragma unroll 1
+      for (int r0 = 0; r0 < n; r0 += 8) {
+        double v[8][MR];
+        load_rows<8, MR>(Ag, n, r0, lane, v);
 #pragma unroll
-        for (int s = 0; s < MR; ++s) {
-          const int c = lane + 32 * s;
-          if (c < n) {
-            const double v = __ldg(row + c);
-            afro = fma(v, v, afro);
-            F(r, c) = (float)v;
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int s = 0; s < MR; ++s) {
+            const int r = r0 + j, c = lane + 32 * s;
+            afro = fma(v[j][s], v[j][s], afro);
+            if (r < n && c < n) F(r, c) = (float)v[j][s];
           }
-        }
       }
       if (n < NP) {  // identity padding
         for (int r = 0; r < NP; ++r)
@@ -510,18 +510,16 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
       for (int ch = 0; ch < NCH; ++ch) {
         double pp[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int r = 16 * ch + j;
-          double acc = 0.0;
-          if (r < n) {
-            const double* row = Ag + (long long)r * n;
+        for (int h = 0; h < 16; h += 8) {
+          double v[8][MR];
+          load_rows<8, MR>(Ag, n, 16 * ch + h, lane, v);
 #pragma unroll
-            for (int s = 0; s < MR; ++s) {
-              const int c = lane + 32 * s;
-              if (c < n) acc = fma(__ldg(row + c), xl[s], acc);
-            }
+          for (int j = 0; j < 8; ++j) {
+            double acc = 0.0;
+#pragma unroll
+            for (int s = 0; s < MR; ++s) acc = fma(v[j][s], xl[s], acc);
+            pp[h + j] = acc;
           }
-          pp[j] = acc;
         }
 #pragma unroll
         for (int o = 16, w = 8; w >= 1; o >>= 1, w >>= 1) {

@@ -110,26 +110,22 @@ __global__ void __launch_bounds__(WPC * 32, 2) features_kernel(const double* __r
 #pragma unroll
     for (int ch = 0; ch < 2 * SL; ++ch) {
       if (16 * ch < n) {
-        double pp[16];
+        double pp[16], v[16][SL];
+        load_rows<16, SL>(Ag, n, 16 * ch, lane, v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int r = 16 * ch + j;
           double acc = 0;
-          if (r < n) {
-            const double* row = Ag + (long long)r * n;
 #pragma unroll
-            for (int s = 0; s < SL; ++s) {
-              const int c = lane + 32 * s;
-              if (c < n) {
-                const double v = __ldg(row + c), av = fabs(v), v2 = v * v;
-                acc += av;
-                csum[s] += av;
-                amax = fmax(amax, av);
-                if (c < r) lo += v2;
-                else if (c > r) up += v2;
-                else cdg[s] = av;
-              }
-            }
+          for (int s = 0; s < SL; ++s) {
+            const int c = lane + 32 * s;
+            const double av = fabs(v[j][s]), v2 = v[j][s] * v[j][s];
+            acc += av;
+            csum[s] += av;
+            amax = fmax(amax, av);
+            if (c < r) lo += v2;
+            else if (c > r) up += v2;
+            else cdg[s] = av;
           }
           pp[j] = acc;
         }
