@@ -35,11 +35,12 @@ int factor_metric(const double* A, const double* F, const int* piv, int n, int64
   if (int rc = check(n, batch)) return rc;
   if (batch == 0) return TSDX_OK;
   if (!A || !F || !out || (!CHOL && !piv)) return TSDX_ERR_NULL;
-  auto kern = dev::factor_bwd_kernel<CHOL>;
-  const int wpc = host::warps_for(batch, warps_for(dev::met_factor_bytes(n))), smem = wpc * dev::met_factor_bytes(n);
+  const int tw = n > 32 ? 2 : 1, bytes = dev::met_factor_bytes(n);
+  auto kern = tw == 2 ? dev::factor_bwd_kernel<CHOL, 2> : dev::factor_bwd_kernel<CHOL, 1>;
+  const int upc = host::warps_for(batch, std::min(16 / tw, warps_for(bytes))), smem = upc * bytes, threads = upc * tw * 32;
   if (int rc = host::prepare(kern, smem)) return rc;
-  const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
-  kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
+  const int grid = host::grid_for(kern, smem, (batch + upc - 1) / upc, threads);
+  kern<<<grid, threads, smem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
   return finish(CHOL ? "cholesky backward error kernel" : "lu backward error kernel");
 }
 }  // namespace

@@ -83,18 +83,33 @@ __device__ __forceinline__ double dd_sqrt(DD a) { return sqrt(__dadd_rn(a.hi, a.
 
 // Shared-memory row of an order-n matrix: an odd number of 16-byte units.
 __host__ __device__ constexpr int met_row_bytes(int n) { return (((n + 1) / 2) | 1) * 16; }
-__host__ __device__ constexpr int met_factor_bytes(int n) { return n * met_row_bytes(n) + 64 * 4; }  // + pivots
+__host__ __device__ constexpr int met_factor_bytes(int n) { return n * met_row_bytes(n) + 64 * 4 + 32; }  // + pivots, partial sums
 __host__ __device__ constexpr int met_solve_bytes(int n) { return n * met_row_bytes(n) + 64 * 8; }   // + x
 
-// Stages an n x n matrix; a last odd column is paired with zero.
-__device__ __forceinline__ void met_stage(unsigned char* M, const double* A, int n, int rs, int lane) {
+// Stages an n x n matrix; a last odd column is paired with zero. Two warps take every
+// other row.
+template <int TW>
+__device__ __forceinline__ void met_stage(unsigned char* M, const double* A, int n, int rs, int lane, int w) {
   const int rowb = n * 8;
   const char* src = reinterpret_cast<const char*>(A);
-  if (vec_of<double>(A, n) == 16) walk_chunks<double, 64, 32, 16>(n, lane, [&](int r, int c) { cp_async<16>(M + r * rs + c * 16, src + r * rowb + c * 16); });
-  else walk_chunks<double, 64, 32, 8>(n, lane, [&](int r, int c) { cp_async<8>(M + r * rs + c * 8, src + r * rowb + c * 8); });
+  auto rows = [&](auto vec) {
+    constexpr int V = decltype(vec)::value;
+    if constexpr (TW == 1) {
+      walk_chunks<double, 64, 32, V>(n, lane, [&](int r, int c) { cp_async<V>(M + r * rs + c * V, src + r * rowb + c * V); });
+    } else {
+      const bool first = lane * V < rowb, second = V == 8 && (lane + 32) * V < rowb;
+#pragma unroll 4
+      for (int r = w; r < n; r += TW) {
+        if (first) cp_async<V>(M + r * rs + lane * V, src + r * rowb + lane * V);
+        if (second) cp_async<V>(M + r * rs + (lane + 32) * V, src + r * rowb + (lane + 32) * V);
+      }
+    }
+  };
+  if (vec_of<double>(A, n) == 16) rows(std::integral_constant<int, 16>());
+  else rows(std::integral_constant<int, 8>());
   cp_async_commit();
   if (n & 1)
-    for (int r = lane; r < n; r += 32) *reinterpret_cast<double*>(M + r * rs + rowb) = 0.0;
+    for (int r = lane + 32 * w; r < n; r += 32 * TW) *reinterpret_cast<double*>(M + r * rs + rowb) = 0.0;
 }
 
 // ||b - A x|| / (||A||_F ||x|| + ||b||); lane i owns rows i and i + 32.
@@ -109,7 +124,7 @@ __global__ void __launch_bounds__(512) solve_bwd_kernel(const double* __restrict
   const long long step = (long long)gridDim.x * wpc;
   for (long long m = (long long)blockIdx.x * wpc + warp; m < batch; m += step) {
     if (lane == 0 && m + step < batch) prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
-    met_stage(M, A + m * n * n, n, rs, lane);
+    met_stage<1>(M, A + m * n * n, n, rs, lane, 0);
     Dot2 fx{0, 0}, fb{0, 0}, num{0, 0}, fa[2] = {{0, 0}, {0, 0}}, r[2] = {{0, 0}, {0, 0}};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -155,28 +170,39 @@ __global__ void __launch_bounds__(512) solve_bwd_kernel(const double* __restrict
 
 // ||P A - L U||_F / ||A||_F (LU packed, unit L) or ||A - L L^T||_F / ||A||_F: the
 // factor is staged in shared memory, lane i owns rows i and i + 32 of the product, two
-// columns at a time. Products beyond min(i, j) enter with a zero multiplier.
-template <bool CHOL>
+// columns at a time. Products beyond min(i, j) enter with a zero multiplier; both rows
+// share a loop over the first 32 columns of the factor, where only the first needs it.
+// Orders above 32 take two warps (TW), every other pair of columns each: shared memory
+// holds six matrices of order 64, and six warps leave the FP64 pipe half idle (LU of order
+// 64, 16,384 matrices, with the solve metric: one warp and row at a time 2855 us, rows
+// sharing a loop 2627, two warps 1877).
+template <bool CHOL, int TW>
 __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restrict__ A, const double* __restrict__ F,
                                                          const int* __restrict__ piv, int n, long long batch,
                                                          double* out) {
   extern __shared__ __align__(16) unsigned char met_smem[];
-  const int wpc = blockDim.x >> 5, warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int unit = warp / TW, w = warp % TW, units = (blockDim.x >> 5) / TW, tid = lane + 32 * w;
   const int rs = met_row_bytes(n);
-  unsigned char* M = met_smem + warp * met_factor_bytes(n);
+  unsigned char* M = met_smem + unit * met_factor_bytes(n);
   int* pv = reinterpret_cast<int*>(M + n * rs);
-  const long long step = (long long)gridDim.x * wpc;
-  for (long long m = (long long)blockIdx.x * wpc + warp; m < batch; m += step) {
+  double* part = reinterpret_cast<double*>(pv + 64);
+  auto barrier = [&]() {
+    if constexpr (TW == 1) __syncwarp();
+    else named_barrier(1 + unit, 32 * TW);
+  };
+  const long long step = (long long)gridDim.x * units;
+  for (long long m = (long long)blockIdx.x * units + unit; m < batch; m += step) {
     const double* a = A + m * n * n;
-    if (lane == 0 && m + step < batch) {
+    if (tid == 0 && m + step < batch) {
       prefetch_l2(F + (m + step) * n * n, (long long)n * n * 8);
       prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
     }
-    met_stage(M, F + m * n * n, n, rs, lane);
+    met_stage<TW>(M, F + m * n * n, n, rs, lane, w);
     int src[2] = {lane, lane + 32};  // the row of A behind each row of P A
     if constexpr (!CHOL) {
-      for (int k = lane; k < n; k += 32) pv[k] = piv[m * n + k];
-      __syncwarp();
+      for (int k = tid; k < n; k += 32 * TW) pv[k] = piv[m * n + k];
+      barrier();
       // the sequential swaps, followed backwards for every row at once
       for (int k = n - 1; k >= 0; --k) {
         const int p = pv[k];
@@ -186,54 +212,120 @@ __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restric
       }
     }
     cp_async_wait<0>();
-    __syncwarp();
+    barrier();
     Dot2 num{0, 0}, fa{0, 0};
+    const bool v16 = vec_of<double>(A, n) == 16, both = TW == 2;
+    const unsigned char* row[2];
+    const double* arow[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      if (32 * s >= n) break;
-      const int i = lane + 32 * s, last = min(n - 1, 32 * s + 31);  // the slot's last row
-      const bool live = i < n;
-      const unsigned char* row = M + (live ? i : 0) * rs;
-      const double* arow = a + (long long)(live ? src[s] : 0) * n;
-      for (int j = 0; j < n; j += 2) {
-        const bool two = j + 1 < n;
-        const double a0 = arow[j], a1 = two ? arow[j + 1] : 0.0;
-        Dot2 d0{a0, 0}, d1{a1, 0};
-        const int kend = min(last, j + 1);
-#pragma unroll 2
-        for (int k = 0; k <= kend; k += 2) {
-          // -L(i, k), -L(i, k + 1): zero past the diagonal, one on it (LU)
-          const double2 l = *reinterpret_cast<const double2*>(row + k * 8);
-          const double l0 = k > i ? 0.0 : (!CHOL && k == i ? -1.0 : -l.x);
-          const double l1 = k + 1 > i ? 0.0 : (!CHOL && k + 1 == i ? -1.0 : -l.y);
-          double2 u0, u1;  // U(k, j..j+1), U(k + 1, j..j+1), zero below the diagonal
-          if constexpr (CHOL) {
-            const double2 lj = *reinterpret_cast<const double2*>(M + j * rs + k * 8);
-            const double2 lj1 = *reinterpret_cast<const double2*>(M + (two ? j + 1 : j) * rs + k * 8);
-            u0 = make_double2(lj.x, lj1.x);
-            u1 = make_double2(lj.y, lj1.y);
-          } else {
-            u0 = *reinterpret_cast<const double2*>(M + k * rs + j * 8);
-            u1 = *reinterpret_cast<const double2*>(M + (k + 1 < n ? k + 1 : k) * rs + j * 8);
-          }
-          d0.fma(l0, u0.x);               // k <= j: k is even, j is even and k <= j + 1
-          d1.fma(l0, u0.y);
-          d0.fma(l1, k + 1 > j ? 0.0 : u1.x);
-          d1.fma(l1, u1.y);
+      const int i = lane + 32 * s;
+      row[s] = M + (i < n ? i : 0) * rs;
+      arow[s] = a + (i < n ? src[s] : 0) * n;
+    }
+    double2 an[2];  // the next two columns of A
+    auto fetch = [&](int j) {
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (s == 1 && !both) break;
+        if (v16) an[s] = __ldg(reinterpret_cast<const double2*>(arow[s] + j));
+        else an[s] = make_double2(__ldg(arow[s] + j), j + 1 < n ? __ldg(arow[s] + j + 1) : 0.0);
+      }
+    };
+    fetch(2 * w);
+#pragma unroll 1
+    for (int j = 2 * w; j < n; j += 2 * TW) {
+      const bool two = j + 1 < n;
+      Dot2 d[2][2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int i = lane + 32 * s;
+        if (s == 1 && !both) break;
+        const double x = an[s].x, y = an[s].y;
+        d[s][0] = {x, 0};
+        d[s][1] = {y, 0};
+        if (i < n) {
+          fa.fma(x, x);
+          if (two) fa.fma(y, y);
         }
-        if (live) {
-          add_square(num, d0.value());
-          fa.fma(a0, a0);
-          if (two) {
-            add_square(num, d1.value());
-            fa.fma(a1, a1);
-          }
+        if constexpr (!CHOL) {  // the unit diagonal of L: - U(i, j), - U(i, j + 1)
+          const double2 u = *reinterpret_cast<const double2*>(row[s] + j * 8);
+          const DD t0 = two_sum(x, i <= j ? -u.x : -0.0), t1 = two_sum(y, i <= j + 1 ? -u.y : -0.0);
+          d[s][0] = {t0.hi, t0.lo};
+          d[s][1] = {t1.hi, t1.lo};
         }
       }
+      if (j + 2 * TW < n) fetch(j + 2 * TW);
+      // columns k, k + 1 of L against U(k, j ..) and U(k + 1, j ..): rows FROM .. of the two
+      // slots, the first of them masked to k < i (k <= i for CHOL); LAST: k = j, where
+      // U(j + 1, j) does not exist
+      auto pair = [&](int k, auto from, auto to, auto last) {
+        constexpr int FROM = decltype(from)::value, TO = decltype(to)::value;
+        constexpr bool LAST = decltype(last)::value;
+        double2 u0, u1;
+        if constexpr (CHOL) {
+          const double2 lj = *reinterpret_cast<const double2*>(M + j * rs + k * 8);
+          const double2 lj1 = *reinterpret_cast<const double2*>(M + (two ? j + 1 : j) * rs + k * 8);
+          u0 = make_double2(lj.x, lj1.x);
+          u1 = make_double2(lj.y, lj1.y);
+        } else {
+          u0 = *reinterpret_cast<const double2*>(M + k * rs + j * 8);
+          u1 = *reinterpret_cast<const double2*>(M + (LAST && !two ? k : k + 1) * rs + j * 8);
+        }
+#pragma unroll
+        for (int s = FROM; s < TO; ++s) {
+          const int i = lane + 32 * s;
+          double2 l = *reinterpret_cast<const double2*>(row[s] + k * 8);
+          if (s == FROM) {
+            l.x = (CHOL ? k <= i : k < i) ? l.x : 0.0;
+            l.y = (CHOL ? k < i : k + 1 < i) ? l.y : 0.0;
+          }
+          d[s][0].fma(-l.x, u0.x);
+          d[s][1].fma(-l.x, u0.y);
+          if constexpr (!LAST) d[s][0].fma(-l.y, u1.x);
+          d[s][1].fma(-l.y, u1.y);
+        }
+      };
+      using Z = std::integral_constant<int, 0>;
+      using O = std::integral_constant<int, 1>;
+      using T = std::integral_constant<int, 2>;
+      const int low = min(j, 32);
+      if (both) {
+#pragma unroll 1
+        for (int k = 0; k < low; k += 2) pair(k, Z(), T(), std::false_type());
+#pragma unroll 2
+        for (int k = 32; k < j; k += 2) pair(k, O(), T(), std::false_type());
+        if (j < 32) pair(j, Z(), T(), std::true_type());
+        else pair(j, O(), T(), std::true_type());
+      } else {
+#pragma unroll 2
+        for (int k = 0; k < low; k += 2) pair(k, Z(), O(), std::false_type());
+        pair(j, Z(), O(), std::true_type());
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (lane + 32 * s >= n) continue;
+        add_square(num, d[s][0].value());
+        if (two) add_square(num, d[s][1].value());
+      }
     }
-    const DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(fa.value());
-    if (lane == 0) out[m] = dd_sqrt(sn) / dd_sqrt(sa);
-    __syncwarp();
+    DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(fa.value());
+    if constexpr (TW == 2) {
+      if (tid == 32) {
+        part[0] = sn.hi;
+        part[1] = sn.lo;
+        part[2] = sa.hi;
+        part[3] = sa.lo;
+      }
+    }
+    barrier();  // the factor's last reads are done as well
+    if (tid == 0) {
+      if constexpr (TW == 2) {
+        sn = dd_add(sn, {part[0], part[1]});
+        sa = dd_add(sa, {part[2], part[3]});
+      }
+      out[m] = dd_sqrt(sn) / dd_sqrt(sa);
+    }
   }
 }
 
