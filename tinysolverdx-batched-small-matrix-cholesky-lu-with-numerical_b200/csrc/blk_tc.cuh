@@ -278,10 +278,10 @@ __device__ __forceinline__ void tc_copy_out(const unsigned char* M, double* A, i
 // holds the largest key publishes {panel row, reciprocal, row} in one of two alternating
 // records, and after the barrier every lane reads it. Latency bounds it, with the
 // shared-memory pipe at 60% for 6 matrices of order 64 on an SM (order 64, 4 right-hand
-// sides, 65,536 matrices 4137 -> 4100 us with its input copies, the solve and U12 of a
-// matrix alone 21,000 -> 9,800 cycles). Two warps per matrix, a row per
-// thread: a matrix alone 25 instead of 33 us, six 45 instead of 44 (the same order; 36
-// instead of 32 for eight of order 48), so one.
+// sides, 65,536 matrices 4137 -> 3928 us with its input copies; of a matrix alone, the
+// solve and U12 21,000 -> 9,800 cycles, the pivot steps 30,000 -> 24,000). Two warps per
+// matrix, a row per thread: a matrix alone 25 instead of 33 us, six 45 instead of 44 (the
+// same order; 36 instead of 32 for eight of order 48), so one.
 template <int NP, int NRHS>
 __device__ __forceinline__ void lu_tc_matrix(unsigned char* M, const MatJob<double>& j, int lane) {
   using C = TcCfg<NP, NRHS>;
@@ -378,21 +378,22 @@ __device__ __forceinline__ void lu_tc_matrix(unsigned char* M, const MatJob<doub
             make_uint4((unsigned)__double2loint(rcp), (unsigned)__double2hiint(rcp), (unsigned)row[s], 0u);
         *reinterpret_cast<T*>(M + row[s] * RS + C::OFF_RCP) = rcp;  // the last one stands: the step that retires the row
       };
-      bool far = false, tie = false;
+      bool far = false;
+      unsigned tie = 0;
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
         if (key[s] == m && act[s]) publish(rec, s, rcand);  // several on a tie: it is looked at again
         const unsigned x = __ballot_sync(kFull, key[s] == m);
-        tie = tie || (x & (x - 1)) || (b && x);
+        tie |= (x & (x - 1)) | (b ? x : 0u);
         b |= x;
-        far = far || D::outside(pan[s][i], D::kLo);
+        far |= D::outside(pan[s][i], D::kLo);
       }
       far = __any_sync(kFull, far);
       __syncwarp();
       bool zero = false;
       // rare, by the whole warp: a tie, or a column whose largest entry is zero, tiny,
       // huge, infinite or NaN
-      const bool odd = tie || m - D::kLo > D::kHi - D::kLo;
+      const bool odd = (tie != 0) | (m - D::kLo > D::kHi - D::kLo);
       if (odd) {
         Candidates<T, MR> c;
 #pragma unroll
