@@ -10,7 +10,7 @@
 // reference to rounding.
 //
 //   float64: the right-hand sides are 8 x 8 accumulator tiles of the FP64 tensor cores.
-//     Blocks of 8 rows are solved by shuffles among the 8 lanes of a column pair; the
+//     Blocks of 8 rows are solved in registers by every lane of a right-hand side; the
 //     rows below (above) take the block by one tile product per 8 rows, which
 //     accumulates its four products in fragment order as fused multiply-adds (see
 //     blk_tc.cuh); the backward pass numbers the fragments downwards. So every element
@@ -94,8 +94,11 @@ __device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const in
 }
 
 // ---------------------------------------------------------------- float64
-// NT tiles of 8 right-hand sides. Accumulator fragment: lane (fr, fq) holds columns 2 fq
-// and 2 fq + 1 of row fr of each tile.
+// NT tiles of 8 right-hand sides, transposed: lane (fr, fq) holds right-hand side fr of a
+// tile at positions 8 I + 2 fq and 8 I + 2 fq + 1 of every block I. The four lanes of a
+// right-hand side gather its 8 values of a block and each solves it in registers: one
+// exchange per block, where the right-hand sides along the lanes took one per position
+// (getrs n = 48, 12 right-hand sides, 32,768 matrices 387 -> 372 us). The reciprocals of the diagonal stand in the rows' padding.
 template <int NP, int NT, bool LU, int WPC>
 __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> p) {
   using C = TrsCfg<double, NP>;
@@ -120,125 +123,119 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> 
     double2 c[NB][NT];
 #pragma unroll
     for (int I = 0; I < NB; ++I) {
-      const int r = 8 * I + fr;
-      const double* row = Bm + (long long)(LU ? perm[r] : r) * p.ldb;
+      const int r = 8 * I + 2 * fq;
+      const int2 o = LU ? *reinterpret_cast<const int2*>(perm + r) : make_int2(r, r + 1);
+      const double* row0 = Bm + (long long)o.x * p.ldb + fr;
+      const double* row1 = Bm + (long long)o.y * p.ldb + fr;
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const int col = 8 * t + 2 * fq;
-        c[I][t].x = (r < n && col < p.nrhs) ? row[col] : 0.0;
-        c[I][t].y = (r < n && col + 1 < p.nrhs) ? row[col + 1] : 0.0;
+        c[I][t].x = (r < n && 8 * t + fr < p.nrhs) ? row0[8 * t] : 0.0;
+        c[I][t].y = (r + 1 < n && 8 * t + fr < p.nrhs) ? row1[8 * t] : 0.0;
       }
     }
     cp_async_wait<0>();
     __syncwarp();
+#pragma unroll
+    for (int s = 0; s < (NP + 31) / 32; ++s) {
+      const int r = lane + 32 * s;
+      if (r < NP) *reinterpret_cast<double*>(M + r * RS + NP * 8) = rcp_(at(r, r));
+    }
+    __syncwarp();
 
-    // B fragment (k = 4 h + fq, or counted down from 7 with DOWN; column fr) of the solved
-    // block: its value stands on lane 4 k + fr / 2
-    auto bfrag = [&](const double2& v, int k) -> double {
-      const int src = 4 * k + (fr >> 1);
-      const double x = __shfl_sync(kFull, v.x, src), y = __shfl_sync(kFull, v.y, src);
-      return (fr & 1) ? y : x;
+    auto rcpd = [&](int r) { return at(r, NP); };
+    auto gather = [&](const double2& v, double (&x)[8]) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        x[2 * q] = __shfl_sync(kFull, v.x, (lane & ~3) | q);
+        x[2 * q + 1] = __shfl_sync(kFull, v.y, (lane & ~3) | q);
+      }
+    };
+    auto of4 = [&](double a, double b, double e, double f) { return (fq & 2) ? ((fq & 1) ? f : e) : ((fq & 1) ? b : a); };
+    // the block's strict lower (upper) triangle, row by row
+    auto lower = [&](int K, double (&l)[8][8]) {
+#pragma unroll
+      for (int i = 1; i < 8; ++i)
+#pragma unroll
+        for (int q = 0; q < i; q += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(M + (8 * K + i) * RS + (8 * K + q) * 8);
+          l[i][q] = v.x;
+          l[i][q + 1] = v.y;
+        }
     };
     // forward: L y = P b
 #pragma unroll
     for (int K = 0; K < NB; ++K) {
-      double l[8];
-      {
-        const double2* lr = reinterpret_cast<const double2*>(M + (8 * K + fr) * RS + 64 * K);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          l[2 * j] = lr[j].x;
-          l[2 * j + 1] = lr[j].y;
-        }
-      }
-      const double dkk = LU ? 1.0 : at(8 * K + fr, 8 * K + fr);
-      const double dinv = LU ? 1.0 : rcp_(dkk);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (!LU && fr == j) {
-#pragma unroll
-          for (int t = 0; t < NT; ++t) c[K][t] = make_double2(div_by(c[K][t].x, dkk, dinv), div_by(c[K][t].y, dkk, dinv));
-        }
-        if (!LU) __syncwarp();
-        if (j == 7) break;
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const double yx = __shfl_sync(kFull, c[K][t].x, 4 * j + fq), yy = __shfl_sync(kFull, c[K][t].y, 4 * j + fq);
-          c[K][t].x = fr > j ? fma_(-l[j], yx, c[K][t].x) : c[K][t].x;
-          c[K][t].y = fr > j ? fma_(-l[j], yy, c[K][t].y) : c[K][t].y;
-        }
-      }
-      double b0[NT], b1[NT];
+      double l[8][8], a0[NT], a1[NT];
+      lower(K, l);
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        b0[t] = bfrag(c[K][t], fq);
-        b1[t] = bfrag(c[K][t], 4 + fq);
+        double x[8];
+        gather(c[K][t], x);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if constexpr (!LU) x[q] = div_by(x[q], at(8 * K + q, 8 * K + q), rcpd(8 * K + q));
+#pragma unroll
+          for (int i = q + 1; i < 8; ++i) x[i] = fma_(-l[i][q], x[q], x[i]);
+        }
+        a0[t] = of4(x[0], x[1], x[2], x[3]);
+        a1[t] = of4(x[4], x[5], x[6], x[7]);
+        c[K][t] = make_double2(of4(x[0], x[2], x[4], x[6]), of4(x[1], x[3], x[5], x[7]));
       }
 #pragma unroll
       for (int I = K + 1; I < NB; ++I) {
-        const double a0 = -at(8 * I + fr, 8 * K + fq), a1 = -at(8 * I + fr, 8 * K + 4 + fq);
+        const double b0 = -at(8 * I + fr, 8 * K + fq), b1 = -at(8 * I + fr, 8 * K + 4 + fq);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          dmma_m8n8k4(c[I][t], a0, b0[t]);
-          dmma_m8n8k4(c[I][t], a1, b1[t]);
+          dmma_m8n8k4(c[I][t], a0[t], b0);
+          dmma_m8n8k4(c[I][t], a1[t], b1);
         }
       }
     }
     // backward: U x = y (LU) or L^T x = y (Cholesky), columns in decreasing order
 #pragma unroll
     for (int K = NB - 1; K >= 0; --K) {
-      double u[8];
+      double u[8][8], d[8], a0[NT], a1[NT];
       if constexpr (LU) {
-        const double2* ur = reinterpret_cast<const double2*>(M + (8 * K + fr) * RS + 64 * K);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          u[2 * j] = ur[j].x;
-          u[2 * j + 1] = ur[j].y;
-        }
+        for (int i = 0; i < 7; ++i)
+#pragma unroll
+          for (int q = (i + 1) & ~1; q < 8; q += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(M + (8 * K + i) * RS + (8 * K + q) * 8);
+            u[i][q] = v.x;
+            u[i][q + 1] = v.y;
+          }
       } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = at(8 * K + j, 8 * K + fr);
+        lower(K, u);
       }
-      const double dinv = rcp_(at(8 * K + fr, 8 * K + fr));
 #pragma unroll
-      for (int j = 7; j >= 0; --j) {
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          c[K][t].x = fr == j ? c[K][t].x * dinv : c[K][t].x;
-          c[K][t].y = fr == j ? c[K][t].y * dinv : c[K][t].y;
-          if (j == 0) continue;
-          const double xx = __shfl_sync(kFull, c[K][t].x, 4 * j + fq), xy = __shfl_sync(kFull, c[K][t].y, 4 * j + fq);
-          c[K][t].x = fr < j ? fma_(-u[j], xx, c[K][t].x) : c[K][t].x;
-          c[K][t].y = fr < j ? fma_(-u[j], xy, c[K][t].y) : c[K][t].y;
-        }
-      }
-      double b0[NT], b1[NT];
+      for (int q = 0; q < 8; ++q) d[q] = rcpd(8 * K + q);
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        b0[t] = bfrag(c[K][t], 7 - fq);
-        b1[t] = bfrag(c[K][t], 3 - fq);
-      }
+        double x[8];
+        gather(c[K][t], x);
 #pragma unroll
-      for (int I = 0; I < K; ++I) {
-        const double a0 = LU ? -at(8 * I + fr, 8 * K + 7 - fq) : -at(8 * K + 7 - fq, 8 * I + fr);
-        const double a1 = LU ? -at(8 * I + fr, 8 * K + 3 - fq) : -at(8 * K + 3 - fq, 8 * I + fr);
+        for (int q = 7; q >= 0; --q) {
+          x[q] = x[q] * d[q];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          dmma_m8n8k4(c[I][t], a0, b0[t]);
-          dmma_m8n8k4(c[I][t], a1, b1[t]);
+          for (int i = q - 1; i >= 0; --i) x[i] = fma_(-(LU ? u[i][q] : u[q][i]), x[q], x[i]);
+        }
+        a0[t] = of4(x[7], x[6], x[5], x[4]);
+        a1[t] = of4(x[3], x[2], x[1], x[0]);
+        if (8 * t + fr < p.nrhs) {
+          double* out = Bm + (long long)(8 * K + 7 - fq) * p.ldb + 8 * t + fr;
+          if (8 * K + 7 - fq < n) out[0] = a0[t];
+          if (8 * K + 3 - fq < n) out[-4ll * p.ldb] = a1[t];
         }
       }
-    }
 #pragma unroll
-    for (int I = 0; I < NB; ++I) {
-      const int r = 8 * I + fr;
-      if (r >= n) continue;
-      double* row = Bm + (long long)r * p.ldb;
+      for (int I = K - 1; I >= 0; --I) {
+        const double b0 = LU ? -at(8 * I + fr, 8 * K + 7 - fq) : -at(8 * K + 7 - fq, 8 * I + fr);
+        const double b1 = LU ? -at(8 * I + fr, 8 * K + 3 - fq) : -at(8 * K + 3 - fq, 8 * I + fr);
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int col = 8 * t + 2 * fq;
-        if (col < p.nrhs) row[col] = c[I][t].x;
-        if (col + 1 < p.nrhs) row[col + 1] = c[I][t].y;
+        for (int t = 0; t < NT; ++t) {
+          dmma_m8n8k4(c[I][t], a0[t], b0);
+          dmma_m8n8k4(c[I][t], a1[t], b1);
+        }
       }
     }
     __syncwarp();
