@@ -79,9 +79,9 @@ template <> struct Unit<float> {
     return d;
   }
 };
-// Shared constants of a rows kernel, at Seg::zrow: a row of zeros, then 16 bytes of
-// float32 -0.
-constexpr int kZeroRow = 576, kRowConst = kZeroRow + 16;
+// Shared constants of a rows kernel, at Seg::zrow: a row of zeros as long as the longest
+// shared row (float64, order 64, 8 right-hand sides), then 16 bytes of float32 -0.
+constexpr int kZeroRow = 592, kRowConst = kZeroRow + 16;
 template <class E> struct __align__(16) Unit2 {
   E x, y;
 };
@@ -205,6 +205,12 @@ struct RowCfg {
   static constexpr int LASTW = NCV - (NP - 1) / PW * PW;       // the last panel holds the right-hand sides
   static constexpr int RW = LASTW > PW ? LASTW : PW;
   static_assert(NP % VN == 0 && NP % PW == 0 && PW % VN == 0, "whole vectors of matrix columns, whole panels");
+  static_assert(NCV * int(sizeof(T)) <= C::RS && C::RS <= kZeroRow, "the row of zeros stands in for any row");
+  // A rolled loop over a panel's groups reads the vector at column k0 + Q in each of them,
+  // past the panel's end in the later ones (values that are not used). in_row: for every
+  // group, k0 = NP - VN included, that vector still lies in its row and its padding; else
+  // the read has to be left out where it passes the panel's end.
+  __host__ __device__ static constexpr bool in_row(int q) { return (NP + q) * int(sizeof(T)) <= C::RS; }
 };
 
 // The position, before step k, of a row still active: its own index, unless an earlier
@@ -412,6 +418,7 @@ __device__ __forceinline__ void lu_rows_group(unsigned Mu, RowRegs<T, NP, NRHS, 
     }
     unrolled<VN, W, VN>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
+      if (ROLLED && !R::in_row(q) && k0 + q >= cend) return;
       const Unit2<E> u = lds16<q * TS>(urow, E());
       const int d = (i + 1 < VN ? q : q - VN) / UN;
 #pragma unroll
@@ -574,6 +581,7 @@ __device__ __forceinline__ void chol_rows_group(unsigned Mu, RowRegs<T, NP, 0, G
     }
 #pragma unroll
     for (int q = VN; q < W; q += VN) {
+      if (R::PW < NP && !R::in_row(q) && k0 % R::PW + q >= R::PW) continue;
       const Unit2<E> u = lds16(krow + (k0 + q) * TS, E());
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
