@@ -84,6 +84,37 @@ def test_solves_from_factor(oracle, n, nrhs, dtype):
         assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1, 2, 8, 15, 16, 17, 24, 31, 47, 63, 64])
+@pytest.mark.parametrize("nrhs", [1, 3, 8, 11, 17])
+def test_solves_with_non_finite_right_hand_sides(oracle, n, nrhs, dtype):
+    """Infinities, NaN and (potrs) a zero on the diagonal of L leave the same pattern of
+    finite, infinite and NaN entries as the oracle's solve, whose terms are the same; the
+    other columns keep the bits that they have without them."""
+    r = np.random.default_rng(n * 37 + nrhs)
+    A = M.general(r, 8, n, 1e2).astype(dtype)
+    LU, piv, _ = oracle.lu(A, "scalar")
+    L, _ = oracle.cholesky(M.spd(r, 8, n, 1e2).astype(dtype), "simd")
+    B = r.standard_normal((8, n, nrhs)).astype(dtype)
+    bad = B.copy()
+    for i in range(8):
+        bad[i, r.integers(n), i % nrhs] = (np.inf, -np.inf, np.nan)[i % 3]
+    zero = L.copy()
+    zero[3:, n // 2, n // 2] = 0.0
+    for F, G, solve in ((LU, LU, lambda f, b: device.getrs(dev(f), dev(piv), b)), (L, zero, lambda f, b: device.potrs(dev(f), b))):
+        good, x = dev(B), dev(bad)
+        solve(F, good)
+        solve(G, x)
+        X, clean = x.cpu().numpy(), good.cpu().numpy()
+        with np.errstate(all="ignore"):
+            want = oracle.lu_solve(LU, piv, bad) if F is LU else oracle.cholesky_solve(zero, bad)
+        assert np.array_equal(np.isnan(X), np.isnan(want))
+        assert np.array_equal(X[np.isinf(X)], want[np.isinf(want)])
+        for i in range(3 if F is L else 8):
+            keep = [c for c in range(nrhs) if c != i % nrhs]
+            assert same(X[i][:, keep], clean[i][:, keep])
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
 def test_binary16_storage_equals_cpu(n):
     r = np.random.default_rng(n)

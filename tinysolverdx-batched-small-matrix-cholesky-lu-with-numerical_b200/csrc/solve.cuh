@@ -191,6 +191,17 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> 
         }
       }
     }
+    // the padded positions have taken 0 * y, NaN where y is not finite: zero again, or the
+    // backward pass, which starts with them, would carry it into every position
+#pragma unroll
+    for (int I = 0; I < NB; ++I) {
+      const int r = 8 * I + 2 * fq;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        c[I][t].x = r < n ? c[I][t].x : 0.0;
+        c[I][t].y = r + 1 < n ? c[I][t].y : 0.0;
+      }
+    }
     // backward: U x = y (LU) or L^T x = y (Cholesky), columns in decreasing order
 #pragma unroll
     for (int K = NB - 1; K >= 0; --K) {
@@ -343,16 +354,20 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
         }
       }
     }
+    // (positions past n: zero, as in the float64 kernel)
     if constexpr (NRHS > 1) {
 #pragma unroll
       for (int s = 0; s < MR; ++s)
 #pragma unroll
         for (int c = 0; c < NU; c += 2) {
           const Unit2<E> y = lds16(xown[s] + c * 8, E());
-          b[s][c] = y.x;
-          b[s][c + 1] = y.y;
+          b[s][c] = lane + 32 * s < n ? y.x : E(0);
+          b[s][c + 1] = lane + 32 * s < n ? y.y : E(0);
         }
       __syncwarp();
+    } else {
+#pragma unroll
+      for (int s = 0; s < MR; ++s) b1[s] = lane + 32 * s < n ? b1[s] : 0.f;
     }
     // backward: U x = y (LU) or L^T x = y (Cholesky)
 #pragma unroll
