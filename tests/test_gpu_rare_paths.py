@@ -115,6 +115,32 @@ def test_solves_with_non_finite_right_hand_sides(oracle, n, nrhs, dtype):
             assert same(X[i][:, keep], clean[i][:, keep])
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,batch", [(1, 120_001), (2, 120_001), (3, 120_001), (4, 120_001), (5, 60_001), (7, 60_001), (8, 60_001),
+                                     (9, 30_001), (11, 30_001), (12, 30_001), (13, 6_001), (16, 6_001), (17, 6_001), (24, 6_001), (33, 6_001), (40, 6_001),
+                                     (56, 6_001), (63, 6_001)])
+@pytest.mark.parametrize("nrhs", [1, 2, 5, 9])
+def test_solves_of_large_batches(oracle, n, batch, nrhs, dtype):
+    """More matrices than the resident warps hold, every warp of a block and every matrix of
+    a warp: seven systems repeated over the batch, each copy with the bits of the first,
+    and the first ones within the bound of test_solves_from_factor."""
+    r = np.random.default_rng(n * 41 + nrhs)
+    A, S = M.general(r, 7, n, 1e2).astype(dtype), M.spd(r, 7, n, 1e2).astype(dtype)
+    B = r.standard_normal((7, n, nrhs)).astype(dtype)
+    LU, piv, _ = oracle.lu(A, "scalar")
+    L, _ = oracle.cholesky(S, "simd")
+    at = torch.arange(batch, device="cuda") % 7
+    for mats, run in ((A, lambda i, b: device.getrs(dev(LU)[i], dev(piv)[i], b)), (S, lambda i, b: device.potrs(dev(L)[i], b))):
+        b = dev(B)[at]
+        run(at, b)
+        bits = b.view(torch.int32 if dtype == np.float32 else torch.int64)
+        assert torch.equal(bits, bits[:7][at])
+        X, M64, B64 = b[:7].cpu().numpy().astype(np.float64), mats.astype(np.float64), B.astype(np.float64)
+        num = np.linalg.norm(B64 - M64 @ X, axis=1)
+        den = np.linalg.norm(M64, axis=(1, 2))[:, None] * np.linalg.norm(X, axis=1) + np.linalg.norm(B64, axis=1)
+        assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
 def test_binary16_storage_equals_cpu(n):
     r = np.random.default_rng(n)

@@ -248,10 +248,42 @@ int run_blk(const SolveArgs<T>& a, cudaStream_t st) {
   return 0;
 }
 
-// One solve pass from a factor (nrhs <= kTrsRhs). Orders run in the next multiple of 16.
+template <class T, int NP, bool LU>
+int launch_trs_small(const SolveArgs<T>& a, cudaStream_t st) {
+  auto kern = dev::trs_small_kernel<T, NP, LU>;
+  constexpr int MOST = dev::kSmallWpc * dev::trs_small_elems(NP, 0) * int(sizeof(T));
+  if (int rc = prepare(kern, MOST)) return rc;
+  int lg = 0;
+  while ((1 << lg) < a.nrhs) ++lg;
+  const long long units = (a.batch + (32 >> lg) - 1) / (32 >> lg);
+  const int wpc = warps_for(units, dev::kSmallWpc), smem = wpc * dev::trs_small_elems(a.n, lg) * int(sizeof(T));
+  const int grid = grid_for(kern, smem, (units + wpc - 1) / wpc, wpc * 32);
+  kern<<<grid, wpc * 32, smem, st>>>(a, lg);
+  launch_counter().fetch_add(1);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_cuda_error(e, "kernel launch"); return -5; }
+  return 0;
+}
+
+// One solve pass from a factor (nrhs <= kTrsRhs). Orders up to 12 take the kernel with a
+// lane per right-hand side (measured up to there, beside it in solve.cuh: faster than the
+// warp per matrix at every width). Above, orders run in the next multiple of 8 in float64
+// (one block of the kernel; order 17, one right-hand side, 64,878 matrices getrs 184 us in
+// 32, 135 in 24), of 16 in float32 (whose steps stop at the order anyway; the multiple
+// only sets the shared memory).
 constexpr int kTrsRhs = 16;
 template <class T, bool LU, int W>
 int run_trs_np(const SolveArgs<T>& a, cudaStream_t st) {
+  if (a.n <= 4) return launch_trs_small<T, 4, LU>(a, st);
+  if (a.n <= 8) return launch_trs_small<T, 8, LU>(a, st);
+  if (a.n <= 12) return launch_trs_small<T, 12, LU>(a, st);
+  if constexpr (sizeof(T) == 8) {
+    switch ((a.n + 7) / 8) {
+      case 3: return launch_trs<T, 24, W, LU>(a, st);
+      case 5: return launch_trs<T, 40, W, LU>(a, st);
+      case 7: return launch_trs<T, 56, W, LU>(a, st);
+    }
+  }
   switch ((a.n + 15) / 16) {
     case 1: return launch_trs<T, 16, W, LU>(a, st);
     case 2: return launch_trs<T, 32, W, LU>(a, st);

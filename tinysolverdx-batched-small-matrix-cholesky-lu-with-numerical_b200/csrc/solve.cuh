@@ -2,8 +2,8 @@
 // (P L U x = b) — TinySolverDx kernels.hpp:184-227 driven by batched.hpp:248-268
 // (which the reference always runs on the CPU; here they run on the GPU).
 //
-// One warp per matrix, up to 16 right-hand sides at a time: the factor is staged to
-// shared memory with cp.async, the right-hand sides live in registers. The forward
+// Up to 16 right-hand sides at a time, one warp per matrix above order 12: the factor is
+// staged to shared memory with cp.async, the right-hand sides live in registers. The forward
 // substitution keeps the reference's chain (increasing k, fused multiply-add, and for
 // Cholesky the division by l_ii); the backward substitution is column-oriented
 // (decreasing k) and multiplies by the reciprocal of the diagonal, so X agrees with the
@@ -18,6 +18,8 @@
 //   float32: lane l owns rows l and l + 32; the solved row goes through shared memory
 //     (which keeps it as the result) and every lane updates its rows, two columns to an
 //     instruction.
+//   Orders up to 12, both types: a lane per right-hand side, as many matrices in a warp as
+//     that leaves room for.
 #pragma once
 #include "blk_tc.cuh"
 #include "rows.cuh"
@@ -32,15 +34,15 @@ struct TrsCfg {
   static constexpr int XB = 16 * int(sizeof(T));       // one solved row (float32)
   static constexpr int OFF_X = MAT, OFF_PERM = MAT + (sizeof(T) == 4 ? NP * XB : 0);
   static constexpr int WARPB = (OFF_PERM + 2 * NP * 4 + 127) / 128 * 128;
-  static_assert(NP % 16 == 0, "row stride in an odd number of 16-byte units");
+  static_assert(NP % 8 == 0, "row stride in an odd number of 16-byte units");
 };
 
-// Stages the factor, identity-padded to NP, and for LU the row that the pivots bring to
+// Stages the factor, identity-padded to order np <= NP (a multiple of 4), and for LU the row that the pivots bring to
 // each position: kernels.hpp:207-213 swaps rows j and piv[j] in increasing j, so a
 // position's origin is found by following it backwards through the swaps. All positions
 // are traced at once, one swap at a time; a pivot outside [0, n) is ignored.
 template <class T, int NP, bool LU>
-__device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const int* piv, int n, int lane) {
+__device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const int* piv, int n, int np, int lane) {
   using C = TrsCfg<T, NP>;
   constexpr int RS = C::RS, TS = int(sizeof(T)), MR = (NP + 31) / 32;
   const int vec = vec_of<T>(A, n), rowb = n * TS;
@@ -49,15 +51,15 @@ __device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const in
   else if (vec == 8) walk_chunks<T, NP, 32, 8>(n, lane, [&](int r, int c) { cp_async<8>(M + r * RS + c * 8, src + r * rowb + c * 8); });
   else if constexpr (sizeof(T) == 4) walk_chunks<T, NP, 32, 4>(n, lane, [&](int r, int c) { cp_async<4>(M + r * RS + c * 4, src + r * rowb + c * 4); });
   cp_async_commit();
-  if (n < NP) {
+  if (n < np) {
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
       const int r = lane + 32 * s;
       T* row = reinterpret_cast<T*>(M + r * RS);
       if (r < n) {
-        for (int c = n; c < NP; ++c) row[c] = T(0);
-      } else if (r < NP) {
-        for (int c = 0; c < NP * TS / 16; ++c) reinterpret_cast<uint4*>(row)[c] = make_uint4(0, 0, 0, 0);
+        for (int c = n; c < np; ++c) row[c] = T(0);
+      } else if (r < np) {
+        for (int c = 0; c < np * TS / 16; ++c) reinterpret_cast<uint4*>(row)[c] = make_uint4(0, 0, 0, 0);
         row[r] = T(1);
       }
     }
@@ -74,12 +76,12 @@ __device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const in
         const int v = piv[k];
         if (v >= 0 && v < n) q[s] = v;
       }
-      if (k < NP) pv[k] = q[s];
+      if (k < np) pv[k] = q[s];
       q[s] = k;
     }
     __syncwarp();
 #pragma unroll 1
-    for (int j0 = NP - 4; j0 >= 0; j0 -= 4) {
+    for (int j0 = np - 4; j0 >= 0; j0 -= 4) {
       const int4 pj = *reinterpret_cast<const int4*>(pv + j0);
       const int pp[4] = {pj.x, pj.y, pj.z, pj.w};
 #pragma unroll
@@ -89,7 +91,7 @@ __device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const in
     }
 #pragma unroll
     for (int s = 0; s < MR; ++s)
-      if (lane + 32 * s < NP) perm[lane + 32 * s] = q[s];
+      if (lane + 32 * s < np) perm[lane + 32 * s] = q[s];
   }
 }
 
@@ -98,7 +100,9 @@ __device__ __forceinline__ void trs_stage(unsigned char* M, const T* A, const in
 // tile at positions 8 I + 2 fq and 8 I + 2 fq + 1 of every block I. The four lanes of a
 // right-hand side gather its 8 values of a block and each solves it in registers: one
 // exchange per block, where the right-hand sides along the lanes took one per position
-// (getrs n = 48, 12 right-hand sides, 32,768 matrices 387 -> 372 us). The reciprocals of the diagonal stand in the rows' padding.
+// (getrs n = 48, 12 right-hand sides, 32,768 matrices 387 -> 372 us). The reciprocals of
+// the diagonal stand in the rows' padding. Orders run in the next multiple of 8 (one
+// block): a block too many costs its loads, products and exchanges.
 template <int NP, int NT, bool LU, int WPC>
 __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> p) {
   using C = TrsCfg<double, NP>;
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f64_kernel(SolveArgs<double> 
       prefetch_l2(p.A + (m + step) * nn, nn * 8);
       prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 8);
     }
-    trs_stage<double, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, lane);
+    trs_stage<double, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, NP, lane);
     if (LU) __syncwarp();
     double* Bm = p.B + m * (long long)n * p.ldb + p.b0;
     double2 c[NB][NT];
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
   unsigned char* M = smem + warp * C::WARPB;
   const unsigned Mu = (unsigned)__cvta_generic_to_shared(M), Xu = Mu + C::OFF_X;
   const int* perm = reinterpret_cast<const int*>(M + C::OFF_PERM) + NP;
-  const int n = p.n;
+  const int n = p.n, np = (n + 3) & ~3;  // the steps run to np
   const long long nn = (long long)n * n, step = (long long)gridDim.x * wpc;
 
   for (long long m = (long long)blockIdx.x * wpc + warp; m < p.batch; m += step) {
@@ -275,7 +279,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
       prefetch_l2(p.A + (m + step) * nn, nn * 4);
       prefetch_l2(p.B + (m + step) * (long long)n * p.ldb, (long long)n * p.ldb * 4);
     }
-    trs_stage<float, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, lane);
+    trs_stage<float, NP, LU>(M, p.A + m * nn, LU ? p.piv + m * n : nullptr, n, np, lane);
     if (LU) __syncwarp();
     float* Bm = p.B + m * (long long)n * p.ldb + p.b0;
     E b[MR][NU];
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
     unsigned own[MR], xown[MR];
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
-      const int r = lane + 32 * s < NP ? lane + 32 * s : NP - 1;
+      const int r = lane + 32 * s < np ? lane + 32 * s : np - 1;
       own[s] = Mu + r * RS;
       xown[s] = Xu + r * XB;
       dg[s] = *reinterpret_cast<const float*>(M + r * RS + r * 4);
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
     // forward: L y = P b; a row's y is final after its own step, where it is published
 #pragma unroll
     for (int t = 0; t < MR; ++t) {
-      const int top = 32 * (t + 1) < NP ? 32 * (t + 1) : NP;
+      const int top = min(32 * (t + 1), np);
 #pragma unroll 1
       for (int k0 = 32 * t; k0 < top; k0 += 4) {
         Unit2<E> lv[MR];
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
     // backward: U x = y (LU) or L^T x = y (Cholesky)
 #pragma unroll
     for (int t = MR - 1; t >= 0; --t) {
-      const int top = 32 * (t + 1) < NP ? 32 * (t + 1) : NP;
+      const int top = min(32 * (t + 1), np);
 #pragma unroll 1
       for (int k0 = top - 4; k0 >= 32 * t; k0 -= 4) {
         float uv[MR][4];
@@ -382,7 +386,7 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
             const float4 v = *reinterpret_cast<const float4*>(M + (own[s] - Mu) + k0 * 4);
             uv[s][0] = v.x; uv[s][1] = v.y; uv[s][2] = v.z; uv[s][3] = v.w;
           } else {
-            const int r = lane + 32 * s < NP ? lane + 32 * s : NP - 1;
+            const int r = lane + 32 * s < np ? lane + 32 * s : np - 1;
 #pragma unroll
             for (int i = 0; i < 4; ++i) uv[s][i] = *reinterpret_cast<const float*>(M + (k0 + i) * RS + r * 4);
           }
@@ -430,6 +434,98 @@ __global__ void __launch_bounds__(WPC * 32, 1) trs_f32_kernel(SolveArgs<float> p
 #pragma unroll
       for (int c = 0; c < NRHS; ++c)
         if (c < p.nrhs) row[c] = NRHS == 1 ? b1[s] : x[c];
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------- orders up to 12
+// A lane per right-hand side and matrix: lg = log2 of the lanes per matrix (the right-hand
+// sides rounded up to a power of two), 32 >> lg matrices per warp, all of a lane's column
+// in registers, the factors of the unit as one run of elements in shared memory. No
+// exchange between lanes and no padding; the operations and their order are those of the
+// kernels above. With a warp per matrix and its padded tile, most lanes and most of the
+// steps of these orders do nothing. Copies of the factors bound it, and for one right-hand
+// side the shared memory of 32 matrices a warp. Against the warp per matrix and, before
+// that one's padding, its unpadded form: float32 potrs, 400,000 matrices, 8 right-hand
+// sides, n = 2 1486 and 318 us; n = 9, 12 right-hand sides 2007 and 1795, here 229; float64
+// getrs, one right-hand side, n = 4, 400,000 matrices 488 and 253; n = 9, 231,481 matrices
+// 304 and 262, here 52; n = 12, 130,208 matrices 178 and 182, here 57.
+constexpr int kSmallWpc = 4;
+__host__ __device__ constexpr int trs_small_stride(int n) { return (n * n) | 1; }  // elements: odd, for the banks
+__host__ __device__ constexpr int trs_small_elems(int n, int lg) { return (32 >> lg) * trs_small_stride(n); }
+
+template <class T, int NP, bool LU>
+__global__ void __launch_bounds__(kSmallWpc * 32) trs_small_kernel(SolveArgs<T> p, int lg) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
+  const int n = p.n, nn = n * n, stride = trs_small_stride(n), S = 32 >> lg;
+  T* F = reinterpret_cast<T*>(smem) + warp * trs_small_elems(n, lg);
+  const T* own = F + (lane >> lg) * stride;
+  const int col = lane & ((1 << lg) - 1);
+  const int dm = 32 / nn, de = 32 - dm * nn;  // 32 elements on
+  const int m_first = lane / nn, e_first = lane - m_first * nn;
+  const long long step = (long long)gridDim.x * wpc * S;
+  for (long long m0 = ((long long)blockIdx.x * wpc + warp) * S; m0 < p.batch; m0 += step) {
+    const int cnt = (int)(p.batch - m0 < S ? p.batch - m0 : S);
+    {
+      const T* src = p.A + m0 * nn;
+      int at = m_first * stride + e_first, e = e_first;
+#pragma unroll 4
+      for (int i = lane; i < cnt * nn; i += 32) {
+        cp_async<int(sizeof(T))>(F + at, src + i);
+        e += de;
+        const bool wrap = e >= nn;
+        e -= wrap ? nn : 0;
+        at += dm * stride + de + (wrap ? stride - nn : 0);
+      }
+      cp_async_commit();
+    }
+    const long long m = m0 + (lane >> lg);
+    const bool live = (lane >> lg) < cnt && col < p.nrhs;
+    T* b = p.B + (live ? m * n * p.ldb + p.b0 + col : 0);
+    T y[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) y[i] = (live && i < n) ? b[i * p.ldb] : T(0);
+    if constexpr (LU) {
+      // swaps in increasing k; a pivot outside [0, n) is ignored
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const int q = (live && k < n) ? p.piv[m * n + k] : k;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          if (j == k) continue;
+          const bool s = q == j && j < n;
+          const T t = y[k];
+          y[k] = s ? y[j] : t;
+          y[j] = s ? t : y[j];
+        }
+      }
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    if (live) {
+      T d[NP];
+#pragma unroll
+      for (int k = 0; k < NP; ++k) d[k] = k < n ? rcp_(own[k * n + k]) : T(0);
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        if (k >= n) break;
+        if constexpr (!LU) y[k] = div_by(y[k], own[k * n + k], d[k]);
+#pragma unroll
+        for (int i = k + 1; i < NP; ++i)
+          if (i < n) y[i] = fma_(-own[i * n + k], y[k], y[i]);
+      }
+#pragma unroll
+      for (int k = NP - 1; k >= 0; --k) {
+        if (k >= n) continue;
+        y[k] = y[k] * d[k];
+#pragma unroll
+        for (int i = k - 1; i >= 0; --i) y[i] = fma_(-(LU ? own[i * n + k] : own[k * n + i]), y[k], y[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (i < n) b[i * p.ldb] = y[i];
     }
     __syncwarp();
   }
