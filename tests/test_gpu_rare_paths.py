@@ -141,6 +141,29 @@ def test_solves_of_large_batches(oracle, n, batch, nrhs, dtype):
         assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
 
 
+@pytest.mark.parametrize("spd", [False, True])
+@pytest.mark.parametrize("n", [5, 17, 40, 64])
+def test_refinement_of_a_large_batch_of_mixed_tiers(n, spd):
+    """Several rounds of full blocks whose warps take different tiers, float64 ones that leave
+    the round at once among them: every copy of a system with its tier has the bits of the
+    first."""
+    r = np.random.default_rng(n + 7 * spd)
+    batch = 7001
+    A = (M.spd if spd else M.general)(r, 7, n, 1e3)
+    b = r.standard_normal((7, n))
+    at = torch.arange(batch, device="cuda")
+    x = dev(b)[at % 7]
+    tier = (at % 4).to(torch.int8)
+    outs = (x, *device.ir(dev(A)[at % 7], x, spd, tier=tier))
+    for t in outs:
+        bits = t.view(torch.int64) if t.dtype == torch.float64 else t
+        assert torch.equal(bits, bits[:28][at % 28])
+    X = x[:28].cpu().numpy()
+    num = np.linalg.norm(b[np.arange(28) % 7] - np.einsum("bij,bj->bi", A[np.arange(28) % 7], X), axis=1)
+    den = np.linalg.norm(A, axis=(1, 2))[np.arange(28) % 7] * np.linalg.norm(X, axis=1) + np.linalg.norm(b, axis=1)[np.arange(28) % 7]
+    assert (num / den).max() <= 8 * n * 2.0 ** -53
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
 def test_binary16_storage_equals_cpu(n):
     r = np.random.default_rng(n)

@@ -104,7 +104,17 @@ __global__ void __launch_bounds__(WPC * 32, 1) ir_kernel(IrArgs p) {
   const long long per_round = (long long)gridDim.x * wpc;
   const int q4 = lane % CGP, rho = lane / CGP;  // cooperative pass coordinates
 
-  for (long long t = (long long)blockIdx.x * wpc + warp; t < p.batch; t += per_round) {
+  // A block barrier before every round keeps the warps on the same code. Without it they
+  // drift apart over the rounds (a matrix takes two to four refinement steps) and their
+  // instructions no longer fit the cache: general matrices, float32 tier, n = 17, 129,757 of
+  // them 2796 us without and 1986 with it; n = 40, 156,250 6701 and 5069; n = 64, 61,035
+  // 2967 and 2596. The code for SPD matrices of orders up to 16 fits, and is faster without
+  // (n = 8, 600,000 matrices 3172 and 3537; the next one, n = 32, 244,140 3238 and 3237).
+  constexpr bool LOCKSTEP = !(SPD && NP == 16);
+  for (long long base = (long long)blockIdx.x * wpc; base < p.batch; base += per_round) {
+    if constexpr (LOCKSTEP) __syncthreads();
+    const long long t = base + warp;
+    if (t >= p.batch) continue;
     const long long m = p.idx ? (long long)p.idx[t] : t;
     const int tier = p.tier ? (int)p.tier[m] : p.default_tier;
     if (tier >= kTierF64) {  // solved directly by the fp64 pass
