@@ -164,6 +164,40 @@ def test_refinement_of_a_large_batch_of_mixed_tiers(n, spd):
     assert (num / den).max() <= 8 * n * 2.0 ** -53
 
 
+def test_metrics_from_several_threads():
+    """Calls of different orders side by side, each thread on its own stream: every one
+    succeeds (a kernel's shared-memory limit belongs to the function, so no call may lower
+    it under another's launch) and gives what it gives alone."""
+    import threading
+    r = np.random.default_rng(4)
+    work, errors = [], []
+    for n in (64, 40, 64, 40):  # one kernel, 6 and 8 matrices a block
+        A = dev(r.standard_normal((900, n, n)))
+        F = A.clone()
+        piv, _ = device.getrf(F)
+        work.append((A, F, piv, device.lu_backward_error(A, F, piv)))
+    torch.cuda.synchronize()
+    start = threading.Barrier(len(work))
+
+    def loop(A, F, piv, want):
+        try:
+            out, stream = torch.empty_like(want), torch.cuda.Stream()
+            args = (capi.ptr(A), capi.ptr(F), capi.ptr(piv), A.shape[-1], A.shape[0], capi.ptr(out), capi.stream_ptr(stream))
+            start.wait()
+            for _ in range(4000):
+                capi.check(capi.call("tsdx_cuda_lu_backward_error_f64", *args), "lu_backward_error")
+            stream.synchronize()
+            assert torch.equal(out, want)
+        except Exception as e:
+            errors.append(e)
+    threads = [threading.Thread(target=loop, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
 def test_binary16_storage_equals_cpu(n):
     r = np.random.default_rng(n)

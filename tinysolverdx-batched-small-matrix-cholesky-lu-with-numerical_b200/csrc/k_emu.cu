@@ -14,8 +14,8 @@ namespace {
 // one warp per matrix; at most 8 warps a CTA keep several CTAs of small orders per SM
 template <class Kern, class... Args>
 int launch(Kern kern, int warp_words, long long batch, cudaStream_t st, Args... args) {
-  const int wpc = warps_for(batch, std::max(1, std::min(8, 227 * 1024 / (warp_words * 4)))), smem = wpc * warp_words * 4;
-  if (int rc = prepare(kern, smem)) return rc;
+  const int wpc = warps_for(batch, std::max(1, std::min(8, kMostSmem / (warp_words * 4)))), smem = wpc * warp_words * 4;
+  if (int rc = prepare(kern, smem, kMostSmem)) return rc;
   const int grid = grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, st>>>(args...);
   const cudaError_t e = cudaGetLastError();

@@ -19,7 +19,7 @@ int launch_ir(const dev::IrArgs& a, cudaStream_t st) {
   constexpr int WPC = FIT < 1 ? 1 : (FIT > CAP ? CAP : FIT);
   constexpr int SMEM = WPC * C::WARPB;
   auto kern = dev::ir_kernel<NP, SPD, WPC>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const int wpc = warps_for(a.batch, WPC), smem = wpc * C::WARPB;
   const int grid = grid_for(kern, smem, (a.batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, st>>>(a);

@@ -12,7 +12,7 @@
 namespace {
 using namespace tsdx;
 // warps per CTA: one matrix each, as many as shared memory holds, at most 16
-int warps_for(int warp_bytes) { return std::max(1, std::min(16, 227 * 1024 / warp_bytes)); }
+int warps_for(int warp_bytes) { return std::max(1, std::min(16, host::kMostSmem / warp_bytes)); }
 
 int finish(const char* what) {
   const cudaError_t e = cudaGetLastError();
@@ -38,7 +38,7 @@ int factor_metric(const double* A, const double* F, const int* piv, int n, int64
   const int tw = n > 32 ? 2 : 1, bytes = dev::met_factor_bytes(n);
   auto kern = tw == 2 ? dev::factor_bwd_kernel<CHOL, 2> : dev::factor_bwd_kernel<CHOL, 1>;
   const int upc = host::warps_for(batch, std::min(16 / tw, warps_for(bytes))), smem = upc * bytes, threads = upc * tw * 32;
-  if (int rc = host::prepare(kern, smem)) return rc;
+  if (int rc = host::prepare(kern, smem, host::kMostSmem)) return rc;
   const int grid = host::grid_for(kern, smem, (batch + upc - 1) / upc, threads);
   kern<<<grid, threads, smem, static_cast<cudaStream_t>(st)>>>(A, F, piv, n, batch, out);
   return finish(CHOL ? "cholesky backward error kernel" : "lu backward error kernel");
@@ -52,7 +52,7 @@ API int tsdx_cuda_solve_backward_error_f64(const double* A, const double* x, con
   if (!A || !x || !b || !out) return TSDX_ERR_NULL;
   auto kern = dev::solve_bwd_kernel;
   const int wpc = host::warps_for(batch, warps_for(dev::met_solve_bytes(n))), smem = wpc * dev::met_solve_bytes(n);
-  if (int rc = host::prepare(kern, smem)) return rc;
+  if (int rc = host::prepare(kern, smem, host::kMostSmem)) return rc;
   const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);
   return finish("solve backward error kernel");

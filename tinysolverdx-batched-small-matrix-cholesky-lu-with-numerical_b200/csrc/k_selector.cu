@@ -65,7 +65,7 @@ API int tsdx_cuda_mlp_grad(const float* params, const float* norm, const float* 
   const long long blocks = train_blocks(batch);
   if (blocks > 0x7fffffffLL) return TSDX_ERR_BATCH;
   auto st = static_cast<cudaStream_t>(stream);
-  if (int rc = host::prepare(dev::mlp_train_kernel, kTrainSmem)) return rc;
+  if (int rc = host::prepare(dev::mlp_train_kernel, kTrainSmem, kTrainSmem)) return rc;
   float* part = static_cast<float*>(scratch);
   dev::mlp_train_kernel<<<(unsigned)blocks, dev::kTrainThreads, kTrainSmem, st>>>(params, norm, features, label,
                                                                                 class_weight, batch, part);

@@ -55,12 +55,16 @@ inline int warps_for(long long units, int wpc) {
   return (int)(per_sm < 1 ? 1 : per_sm < wpc ? per_sm : wpc);
 }
 
+// Allows a kernel the smem bytes of dynamic shared memory that a call uses. most is the most
+// that any of its calls uses, the same in every call: the limit belongs to the function on
+// a device, so a call that set its own smaller need would lower it between another
+// thread's prepare and launch.
+constexpr int kMostSmem = 227 * 1024;  // of a block, less its static shared memory
 template <class Kern>
-int prepare(Kern kern, int smem) {
-  // the attribute is per function and per device; setting it is idempotent (the 48 KB
-  // that need none hold a kernel's static shared memory as well)
+int prepare(Kern kern, int smem, int most) {
+  // (the 48 KB that need no leave hold a kernel's static shared memory as well)
   if (smem > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute"); return -5; }
   }
   return 0;
@@ -108,7 +112,7 @@ int launch_blk2(const SolveArgs<T>& a, cudaStream_t st) {
   constexpr int TPC = FIT < 1 ? 1 : (FIT > 8 ? 8 : FIT);
   constexpr int SMEM = TPC * C::TEAMB;
   auto kern = dev::blk2_kernel<T, NP, NRHS, TPC>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const long long ctas = (a.batch + TPC - 1) / TPC;
   const int grid = grid_for(kern, SMEM, ctas, TPC * 64);
   kern<<<grid, TPC * 64, SMEM, st>>>(a);
@@ -130,7 +134,7 @@ int launch_blk3(const SolveArgs<T>& a, cudaStream_t st) {
   // the panel warp also takes part of the trailing update (pivot steps counted as 3
   // chunk updates): +3.8 % at n = 64, -1.3 % at n = 61 on B200
   auto kern = dev::blk3_kernel<T, NP, NRHS, TPC, 3>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const long long ctas = (a.batch + TPC - 1) / TPC;
   const int grid = grid_for(kern, SMEM, ctas, TPC * 64);
   kern<<<grid, TPC * 64, SMEM, st>>>(a);
@@ -155,7 +159,7 @@ int launch_tc(const SolveArgs<double>& a, cudaStream_t st) {
   constexpr int WPC = FIT < 1 ? 1 : (FIT > 16 ? 16 : FIT);
   constexpr int SMEM = WPC * C::WARPB;
   auto kern = dev::tc_kernel<NP, NRHS, WPC>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const int wpc = warps_for(a.batch, WPC), smem = wpc * C::WARPB;
   const int grid = grid_for(kern, smem, (a.batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, st>>>(a);
@@ -186,7 +190,7 @@ int launch_blk(const SolveArgs<T>& a, cudaStream_t st) {
   constexpr int WPC = blk_wpc<T, NP, NRHS, GO>();
   constexpr int SMEM = WPC * C::WARPB;
   auto kern = dev::blk_kernel<T, NP, NRHS, WPC, CHOL, GO>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const long long units = (a.batch + C::S - 1) / C::S;
   const int wpc = warps_for(units, WPC), smem = wpc * C::WARPB;
   const int grid = grid_for(kern, smem, (units + wpc - 1) / wpc, wpc * 32);
@@ -210,7 +214,7 @@ int launch_trs(const SolveArgs<T>& a, cudaStream_t st) {
     if constexpr (sizeof(T) == 8) return dev::trs_f64_kernel<NP, W, LU, WPC>;
     else return dev::trs_f32_kernel<NP, W, LU, WPC>;
   }();
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const int wpc = warps_for(a.batch, WPC), smem = wpc * C::WARPB;
   const int grid = grid_for(kern, smem, (a.batch + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, st>>>(a);
@@ -252,11 +256,11 @@ template <class T, int NP, bool LU>
 int launch_trs_small(const SolveArgs<T>& a, cudaStream_t st) {
   auto kern = dev::trs_small_kernel<T, NP, LU>;
   constexpr int MOST = dev::kSmallWpc * dev::trs_small_elems(NP, 0) * int(sizeof(T));
-  if (int rc = prepare(kern, MOST)) return rc;
   int lg = 0;
   while ((1 << lg) < a.nrhs) ++lg;
   const long long units = (a.batch + (32 >> lg) - 1) / (32 >> lg);
   const int wpc = warps_for(units, dev::kSmallWpc), smem = wpc * dev::trs_small_elems(a.n, lg) * int(sizeof(T));
+  if (int rc = prepare(kern, smem, MOST)) return rc;
   const int grid = grid_for(kern, smem, (units + wpc - 1) / wpc, wpc * 32);
   kern<<<grid, wpc * 32, smem, st>>>(a, lg);
   launch_counter().fetch_add(1);

@@ -44,7 +44,7 @@ int launch_drain(const dev::StreamArgs<T>& a, cudaStream_t st) {
   constexpr int WPC = FIT < 1 ? 1 : (FIT >= 16 ? 16 : FIT >= 12 ? 12 : FIT);
   constexpr int SMEM = WPC * WARPB;
   auto kern = dev::stream_kernel<T, WARPB, WPC, CLO, CHI>;
-  if (int rc = prepare(kern, SMEM)) return rc;
+  if (int rc = prepare(kern, SMEM, SMEM)) return rc;
   const int grid = grid_for(kern, SMEM, 1LL << 30, WPC * 32);
   kern<<<grid, WPC * 32, SMEM, st>>>(a);
   return 0;
