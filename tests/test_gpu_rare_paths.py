@@ -198,6 +198,51 @@ def test_metrics_from_several_threads():
     assert not errors, errors
 
 
+@pytest.mark.parametrize("n", [20, 33, 64])
+def test_metrics_keep_double_double_sums(n):
+    """Sums whose remainder stands 105 bits below their largest term, after n - 8 roundings
+    of the high part in one direction: exact in double-double, which renormalises at each
+    term; lost in a low part that is a plain running sum."""
+    from oracle import exact_metrics as X
+    v = np.concatenate([[2.0 ** 53], np.full(n - 9, 0.75), np.full(5, 2.0 ** -52), [-2.0 ** 53, -0.75 * (n - 9)]])[:n]
+    assert len(v) == n - 1
+    A = np.zeros((1, n, n))
+    A[0, -1, :-1] = v
+    x, b = np.ones((1, n)), np.zeros((1, n))
+    got = device.solve_backward_error(dev(A), dev(x), dev(b)).cpu().numpy()
+    want = X.solve_backward_error(A, x, b)
+    assert want[0] > 0
+    np.testing.assert_allclose(got, want, rtol=1e-13, atol=0)
+    LU = A.copy()
+    LU[0, :-1, -1] = 1.0
+    P = np.zeros((1, n, n))
+    P[0, :-1, -1] = 1.0
+    piv = np.arange(n, dtype=np.int32)[None]
+    got = device.lu_backward_error(dev(P), dev(LU), dev(piv)).cpu().numpy()
+    np.testing.assert_allclose(got, X.lu_backward_error(P, LU, piv), rtol=1e-13, atol=0)
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 47, 64])
+def test_metrics_of_large_batches(oracle, n):
+    """Every warp and team of a block, and several rounds: each copy has the bits of the first,
+    and the first ones the values of exact arithmetic."""
+    from oracle import exact_metrics as X
+    batch = 5003
+    r = np.random.default_rng(n)
+    A, S, b = M.general(r, 5, n, 1e3), M.spd(r, 5, n, 1e3), r.standard_normal((5, n))
+    LU, piv, _ = oracle.lu(A, "scalar")
+    L, _ = oracle.cholesky(S, "simd")
+    x = oracle.lu_solve(LU, piv, b[..., None])[..., 0]
+    piv = piv.astype(np.int32)
+    at = torch.arange(batch, device="cuda") % 5
+    for got, want in ((device.lu_backward_error(dev(A)[at], dev(LU)[at], dev(piv)[at]), X.lu_backward_error(A[:2], LU[:2], piv[:2])),
+                      (device.chol_backward_error(dev(S)[at], dev(L)[at]), X.chol_backward_error(S[:2], L[:2])),
+                      (device.solve_backward_error(dev(A)[at], dev(x)[at], dev(b)[at]), X.solve_backward_error(A[:2], x[:2], b[:2]))):
+        bits = got.view(torch.int64)
+        assert torch.equal(bits, bits[:5][at])
+        np.testing.assert_allclose(got[:2].cpu().numpy(), want, rtol=1e-12, atol=0)
+
+
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64])
 def test_binary16_storage_equals_cpu(n):
     r = np.random.default_rng(n)

@@ -50,11 +50,12 @@ API int tsdx_cuda_solve_backward_error_f64(const double* A, const double* x, con
   if (int rc = check(n, batch)) return rc;
   if (batch == 0) return TSDX_OK;
   if (!A || !x || !b || !out) return TSDX_ERR_NULL;
-  auto kern = dev::solve_bwd_kernel;
-  const int wpc = host::warps_for(batch, warps_for(dev::met_solve_bytes(n))), smem = wpc * dev::met_solve_bytes(n);
+  const int tw = n > 32 ? 2 : 1, bytes = dev::met_solve_bytes(n);
+  auto kern = tw == 2 ? dev::solve_bwd_kernel<2> : dev::solve_bwd_kernel<1>;
+  const int upc = host::warps_for(batch, std::min(16 / tw, warps_for(bytes))), smem = upc * bytes, threads = upc * tw * 32;
   if (int rc = host::prepare(kern, smem, host::kMostSmem)) return rc;
-  const int grid = host::grid_for(kern, smem, (batch + wpc - 1) / wpc, wpc * 32);
-  kern<<<grid, wpc * 32, smem, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);
+  const int grid = host::grid_for(kern, smem, (batch + upc - 1) / upc, threads);
+  kern<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(A, x, b, n, batch, out);
   return finish("solve backward error kernel");
 }
 

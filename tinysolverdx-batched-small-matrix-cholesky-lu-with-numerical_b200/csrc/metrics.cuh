@@ -10,13 +10,13 @@
 // about 106 significand bits, more than the reference's x87 long double (64), so
 // the sums of products here are at least as accurate as the reference's. The
 // building blocks are the published error-free transformations: TwoSum (Knuth,
-// TAOCP vol. 2, 4.2.2), TwoProduct with a fused multiply-add, sums of products by
-// Dot2 (Ogita, Rump and Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput.
-// 26(6), 2005: as accurate as in twice the working precision, 10 operations a
-// product), and the double-double additions of Hida, Li and Bailey ("Algorithms for
-// quad-double precision floating point arithmetic", ARITH-15, 2001) across lanes.
+// TAOCP vol. 2, 4.2.2), TwoProduct with a fused multiply-add, and the double-double
+// additions of Hida, Li and Bailey ("Algorithms for quad-double precision floating point
+// arithmetic", ARITH-15, 2001), in the sums of products too: with the low part a plain
+// running sum instead (10 operations a product), the elements of A - L U of order 64 had
+// 3.5 times the error.
 //
-// What bounds them: the factor metrics are FP64 arithmetic (n^3 / 3 products at 10
+// What bounds them: the factor metrics are FP64 arithmetic (n^3 / 3 products at 19
 // operations), the solve metric reads A once. The matrix is staged in shared memory
 // (cp.async, coalesced) in rows of an odd number of 16-byte units, so that a lane per row
 // reads two columns at a time without bank conflicts.
@@ -50,25 +50,18 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
   s.lo = __dadd_rn(s.lo, t.lo);
   return fast_two_sum(s.hi, s.lo);
 }
-// A sum of products: hi is the rounded running sum, lo the errors of its additions and
-// products.
-struct Dot2 {
-  double hi, lo;
-  __device__ __forceinline__ void add(double p, double e) {  // p + e, |e| an error term of p
-    const DD t = two_sum(hi, p);
-    hi = t.hi;
-    lo = __dadd_rn(lo, __dadd_rn(t.lo, e));
-  }
-  __device__ __forceinline__ void fma(double x, double y) {
-    const double p = __dmul_rn(x, y);
-    add(p, __fma_rn(x, y, -p));
-  }
-  __device__ __forceinline__ DD value() const { return two_sum(hi, lo); }
-};
-// + d^2
-__device__ __forceinline__ void add_square(Dot2& a, DD d) {
-  const double p = __dmul_rn(d.hi, d.hi);
-  a.add(p, __fma_rn(__dmul_rn(2.0, d.hi), d.lo, __fma_rn(d.hi, d.hi, -p)));
+// a + x y, the product taken exactly (TwoProduct). dd_add without its last renormalisation,
+// which does not change the sum.
+__device__ __forceinline__ DD dd_fma(DD a, double x, double y) {
+  const double p = __dmul_rn(x, y);
+  const DD t = two_sum(a.lo, __fma_rn(x, y, -p));
+  DD s = two_sum(a.hi, p);
+  s = fast_two_sum(s.hi, __dadd_rn(s.lo, t.hi));
+  return {s.hi, __dadd_rn(s.lo, t.lo)};
+}
+__device__ __forceinline__ DD dd_sqr(DD a) {
+  const double p = __dmul_rn(a.hi, a.hi);
+  return fast_two_sum(p, __fma_rn(__dmul_rn(2.0, a.hi), a.lo, __fma_rn(a.hi, a.hi, -p)));
 }
 __device__ __forceinline__ DD dd_warp_sum(DD v) {
   for (int o = 16; o > 0; o >>= 1) {
@@ -84,7 +77,7 @@ __device__ __forceinline__ double dd_sqrt(DD a) { return sqrt(__dadd_rn(a.hi, a.
 // Shared-memory row of an order-n matrix: an odd number of 16-byte units.
 __host__ __device__ constexpr int met_row_bytes(int n) { return (((n + 1) / 2) | 1) * 16; }
 __host__ __device__ constexpr int met_factor_bytes(int n) { return n * met_row_bytes(n) + 64 * 4 + 32; }  // + pivots, partial sums
-__host__ __device__ constexpr int met_solve_bytes(int n) { return n * met_row_bytes(n) + 64 * 8; }   // + x
+__host__ __device__ constexpr int met_solve_bytes(int n) { return n * met_row_bytes(n) + 64 * 8 + 64; }   // + x, partial sums
 
 // Stages an n x n matrix; a last odd column is paired with zero. Two warps take every
 // other row.
@@ -112,59 +105,62 @@ __device__ __forceinline__ void met_stage(unsigned char* M, const double* A, int
     for (int r = lane + 32 * w; r < n; r += 32 * TW) *reinterpret_cast<double*>(M + r * rs + rowb) = 0.0;
 }
 
-// ||b - A x|| / (||A||_F ||x|| + ||b||); lane i owns rows i and i + 32.
-__global__ void __launch_bounds__(512) solve_bwd_kernel(const double* __restrict__ A, const double* __restrict__ x,
+// ||b - A x|| / (||A||_F ||x|| + ||b||). A row per lane, two warps (TW) above order 32;
+// sums over even and odd columns, so that four chains of additions are in flight (order
+// 64, 2,000 matrices: one warp, two rows a lane 52 us, this 44).
+template <int TW>
+__global__ void __launch_bounds__(512, 1) solve_bwd_kernel(const double* __restrict__ A, const double* __restrict__ x,
                                                         const double* __restrict__ b, int n, long long batch,
                                                         double* out) {
   extern __shared__ __align__(16) unsigned char met_smem[];
-  const int wpc = blockDim.x >> 5, warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int unit = warp / TW, w = warp % TW, units = (blockDim.x >> 5) / TW, i = lane + 32 * w;
   const int rs = met_row_bytes(n);
-  unsigned char* M = met_smem + warp * met_solve_bytes(n);
+  unsigned char* M = met_smem + unit * met_solve_bytes(n);
   double* xs = reinterpret_cast<double*>(M + n * rs);
-  const long long step = (long long)gridDim.x * wpc;
-  for (long long m = (long long)blockIdx.x * wpc + warp; m < batch; m += step) {
-    if (lane == 0 && m + step < batch) prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
-    met_stage<1>(M, A + m * n * n, n, rs, lane, 0);
-    Dot2 fx{0, 0}, fb{0, 0}, num{0, 0}, fa[2] = {{0, 0}, {0, 0}}, r[2] = {{0, 0}, {0, 0}};
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int i = lane + 32 * s;
-      const double xi = i < n ? x[m * n + i] : 0.0;
-      xs[i] = xi;  // zero from n on: the partner of a last odd column
-      r[s].hi = i < n ? b[m * n + i] : 0.0;
-      fx.fma(xi, xi);
-      fb.fma(r[s].hi, r[s].hi);
-    }
+  double* part = xs + 64;
+  auto barrier = [&]() {
+    if constexpr (TW == 1) __syncwarp();
+    else named_barrier(1 + unit, 32 * TW);
+  };
+  const long long step = (long long)gridDim.x * units;
+  for (long long m = (long long)blockIdx.x * units + unit; m < batch; m += step) {
+    if (i == 0 && m + step < batch) prefetch_l2(A + (m + step) * n * n, (long long)n * n * 8);
+    met_stage<TW>(M, A + m * n * n, n, rs, lane, w);
+    const double xi = i < n ? x[m * n + i] : 0.0, bi = i < n ? b[m * n + i] : 0.0;
+    xs[i] = xi;  // zero from n on: the partner of a last odd column
+    DD num{0, 0}, fa{0, 0}, fx = dd_fma({0, 0}, xi, xi), fb = dd_fma({0, 0}, bi, bi);
     cp_async_wait<0>();
-    __syncwarp();
-    const unsigned char* row0 = M + (lane < n ? lane : 0) * rs;
-    const unsigned char* row1 = M + (lane + 32 < n ? lane + 32 : 0) * rs;
+    barrier();
+    if (i < n) {
+      const unsigned char* row = M + i * rs;
+      DD r0{bi, 0}, r1{0, 0}, f0{0, 0}, f1{0, 0};
 #pragma unroll 2
-    for (int j = 0; j < n; j += 2) {
-      const double2 a0 = *reinterpret_cast<const double2*>(row0 + j * 8);
-      const double x0 = -xs[j], x1 = -xs[j + 1];
-      r[0].fma(a0.x, x0);
-      r[0].fma(a0.y, x1);
-      fa[0].fma(a0.x, a0.x);
-      fa[0].fma(a0.y, a0.y);
-      if (n > 32) {
-        const double2 a1 = *reinterpret_cast<const double2*>(row1 + j * 8);
-        r[1].fma(a1.x, x0);
-        r[1].fma(a1.y, x1);
-        fa[1].fma(a1.x, a1.x);
-        fa[1].fma(a1.y, a1.y);
+      for (int j = 0; j < n; j += 2) {
+        const double2 a = *reinterpret_cast<const double2*>(row + j * 8), v = *reinterpret_cast<const double2*>(xs + j);
+        r0 = dd_fma(r0, a.x, -v.x);
+        r1 = dd_fma(r1, a.y, -v.y);
+        f0 = dd_fma(f0, a.x, a.x);
+        f1 = dd_fma(f1, a.y, a.y);
+      }
+      num = dd_sqr(dd_add(r0, r1));
+      fa = dd_add(f0, f1);
+    }
+    DD v[4] = {dd_warp_sum(num), dd_warp_sum(fa), dd_warp_sum(fx), dd_warp_sum(fb)};
+    if (TW == 2 && i == 32) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        part[2 * q] = v[q].hi;
+        part[2 * q + 1] = v[q].lo;
       }
     }
-    DD f{0, 0};
+    barrier();  // the last reads of the matrix are done as well
+    if (i == 0) {
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      if (lane + 32 * s >= n) continue;
-      add_square(num, r[s].value());
-      f = dd_add(f, fa[s].value());
+      for (int q = 0; q < 4; ++q)
+        if (TW == 2) v[q] = dd_add(v[q], {part[2 * q], part[2 * q + 1]});
+      out[m] = dd_sqrt(v[0]) / (dd_sqrt(v[1]) * dd_sqrt(v[2]) + dd_sqrt(v[3]));
     }
-    const DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(f), sx = dd_warp_sum(fx.value()), sb = dd_warp_sum(fb.value());
-    if (lane == 0) out[m] = dd_sqrt(sn) / (dd_sqrt(sa) * dd_sqrt(sx) + dd_sqrt(sb));
-    __syncwarp();
   }
 }
 
@@ -173,9 +169,10 @@ __global__ void __launch_bounds__(512) solve_bwd_kernel(const double* __restrict
 // columns at a time. Products beyond min(i, j) enter with a zero multiplier; both rows
 // share a loop over the first 32 columns of the factor, where only the first needs it.
 // Orders above 32 take two warps (TW), every other pair of columns each: shared memory
-// holds six matrices of order 64, and six warps leave the FP64 pipe half idle (LU of order
-// 64, 16,384 matrices, with the solve metric: one warp and row at a time 2855 us, rows
-// sharing a loop 2627, two warps 1877).
+// holds six matrices of order 64, and six warps leave the FP64 pipe half idle (measured
+// with cheaper sums, LU of order 64 and its solve metric, 16,384 matrices: one warp and
+// row at a time 2855 us, rows sharing a loop 2627, two warps 1877; with these sums LU
+// alone 2670, where one warp with uncoalesced reads took 7000).
 template <bool CHOL, int TW>
 __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restrict__ A, const double* __restrict__ F,
                                                          const int* __restrict__ piv, int n, long long batch,
@@ -213,7 +210,7 @@ __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restric
     }
     cp_async_wait<0>();
     barrier();
-    Dot2 num{0, 0}, fa{0, 0};
+    DD num{0, 0}, fa{0, 0};
     const bool v16 = vec_of<double>(A, n) == 16, both = TW == 2;
     const unsigned char* row[2];
     const double* arow[2];
@@ -236,23 +233,16 @@ __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restric
 #pragma unroll 1
     for (int j = 2 * w; j < n; j += 2 * TW) {
       const bool two = j + 1 < n;
-      Dot2 d[2][2];
+      DD d[2][2];  // the sums of products; then A's elements less these
+      double2 av[2];
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int i = lane + 32 * s;
         if (s == 1 && !both) break;
-        const double x = an[s].x, y = an[s].y;
-        d[s][0] = {x, 0};
-        d[s][1] = {y, 0};
-        if (i < n) {
-          fa.fma(x, x);
-          if (two) fa.fma(y, y);
-        }
-        if constexpr (!CHOL) {  // the unit diagonal of L: - U(i, j), - U(i, j + 1)
-          const double2 u = *reinterpret_cast<const double2*>(row[s] + j * 8);
-          const DD t0 = two_sum(x, i <= j ? -u.x : -0.0), t1 = two_sum(y, i <= j + 1 ? -u.y : -0.0);
-          d[s][0] = {t0.hi, t0.lo};
-          d[s][1] = {t1.hi, t1.lo};
+        d[s][0] = d[s][1] = {0, 0};
+        av[s] = an[s];
+        if (lane + 32 * s < n) {
+          fa = dd_fma(fa, av[s].x, av[s].x);
+          if (two) fa = dd_fma(fa, av[s].y, av[s].y);
         }
       }
       if (j + 2 * TW < n) fetch(j + 2 * TW);
@@ -280,10 +270,10 @@ __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restric
             l.x = (CHOL ? k <= i : k < i) ? l.x : 0.0;
             l.y = (CHOL ? k < i : k + 1 < i) ? l.y : 0.0;
           }
-          d[s][0].fma(-l.x, u0.x);
-          d[s][1].fma(-l.x, u0.y);
-          if constexpr (!LAST) d[s][0].fma(-l.y, u1.x);
-          d[s][1].fma(-l.y, u1.y);
+          d[s][0] = dd_fma(d[s][0], l.x, u0.x);
+          d[s][1] = dd_fma(d[s][1], l.x, u0.y);
+          if constexpr (!LAST) d[s][0] = dd_fma(d[s][0], l.y, u1.x);
+          d[s][1] = dd_fma(d[s][1], l.y, u1.y);
         }
       };
       using Z = std::integral_constant<int, 0>;
@@ -304,12 +294,18 @@ __global__ void __launch_bounds__(512) factor_bwd_kernel(const double* __restric
       }
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        if (lane + 32 * s >= n) continue;
-        add_square(num, d[s][0].value());
-        if (two) add_square(num, d[s][1].value());
+        const int i = lane + 32 * s;
+        if (i >= n) continue;
+        if constexpr (!CHOL) {  // the unit diagonal of L
+          const double2 u = *reinterpret_cast<const double2*>(row[s] + j * 8);
+          d[s][0] = dd_add(d[s][0], {i <= j ? u.x : 0.0, 0.0});
+          d[s][1] = dd_add(d[s][1], {i <= j + 1 ? u.y : 0.0, 0.0});
+        }
+        num = dd_add(num, dd_sqr(dd_add({av[s].x, 0.0}, {-d[s][0].hi, -d[s][0].lo})));
+        if (two) num = dd_add(num, dd_sqr(dd_add({av[s].y, 0.0}, {-d[s][1].hi, -d[s][1].lo})));
       }
     }
-    DD sn = dd_warp_sum(num.value()), sa = dd_warp_sum(fa.value());
+    DD sn = dd_warp_sum(num), sa = dd_warp_sum(fa);
     if constexpr (TW == 2) {
       if (tid == 32) {
         part[0] = sn.hi;
