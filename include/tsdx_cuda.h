@@ -128,7 +128,8 @@ int tsdx_cuda_posv_ir_f64(const double* A, int n, int64_t batch, double* B, cons
  * The reference's per-operation-rounding formats (precision.hpp:41-97), which it runs
  * only on the CPU (batched.hpp:130-132), bit-identical to its CPU results. Storage is
  * float64 as in the runtime API (runtime.cpp:95-141); _f32: float32, _f16: binary16 bits
- * (values are rounded into the format on entry); fmt 0 = fp16, 1 = bf16.
+ * (values are rounded into the format on entry); fmt 0 = fp16, 1 = bf16, with _f16 fp16
+ * only (binary16 does not hold bf16's range: TSDX_ERR_NULL, as for any other fmt).
  *   factor: lu = 0 Cholesky (A <- L, info), lu = 1 LU (A <- L\U, piv, info)
  *   solve:  lu = 0 B <- (L L^T)^{-1} B, lu = 1 B <- (P L U)^{-1} B */
 int tsdx_cuda_emu_factor_host(int fmt, int lu, double* A, int n, int64_t batch, int* piv, int* info);

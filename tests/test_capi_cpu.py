@@ -102,3 +102,14 @@ def test_stream_solve_host_python_validation():
         stream.solve_host(A, B, piv, info[:1], n, r, k)
     e = torch.zeros(0, dtype=torch.int32)
     stream.solve_host(A, B, piv, info, e, e, torch.zeros(0, dtype=torch.int8))  # count 0: nothing to do
+
+
+def test_binary16_storage_is_for_fp16_alone():
+    """bf16's range does not fit binary16: the _f16 entries refuse it as they refuse a format
+    that does not exist, before they look for a device."""
+    lib = capi.lib()
+    a = np.zeros((1, 2, 2), np.uint16)
+    piv, info = np.zeros((1, 2), np.int32), np.zeros(1, np.int32)
+    for fmt in (1, 2, -1):
+        assert lib.tsdx_cuda_emu_factor_host_f16(fmt, 1, capi.ptr(a), 2, 1, capi.ptr(piv), capi.ptr(info)) == capi.TSDX_ERR_NULL
+        assert lib.tsdx_cuda_emu_solve_host_f16(fmt, 0, capi.ptr(a), None, 2, 1, capi.ptr(a), 2) == capi.TSDX_ERR_NULL

@@ -249,8 +249,9 @@ int run_host(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int
 }
 
 // ---- emulated formats (S: the storage type), through the same pipeline
-int emu_check(int fmt, int n, int64_t batch) {
-  if (fmt != 0 && fmt != 1) return TSDX_ERR_NULL;
+template <class S> int emu_check(int fmt, int n, int64_t batch) {
+  // binary16 storage holds every fp16 value, but not bf16's range
+  if (fmt != 0 && (fmt != 1 || sizeof(S) == 2)) return TSDX_ERR_NULL;
   if (n < 1 || n > 64) return TSDX_ERR_N;
   if (batch < 0) return TSDX_ERR_BATCH;
   int count = 0;
@@ -261,7 +262,7 @@ int emu_check(int fmt, int n, int64_t batch) {
   return TSDX_OK;
 }
 template <class S> int emu_factor_host(int fmt, int lu, S* A, int n, int64_t batch, int* piv, int* info) {
-  if (int rc = emu_check(fmt, n, batch)) return rc;
+  if (int rc = emu_check<S>(fmt, n, batch)) return rc;
   return run_host_with<S>(lu ? GETRF : POTRF, A, nullptr, n, batch, nullptr, 0, piv, info, false,
                           [&](S* dA, int* dpiv, int64_t cnt, S*, int* dinfo, cudaStream_t st) {
                             return run_emu_factor<S>(fmt, lu != 0, dA, n, cnt, dpiv, dinfo, st);
@@ -269,7 +270,7 @@ template <class S> int emu_factor_host(int fmt, int lu, S* A, int n, int64_t bat
 }
 template <class S>
 int emu_solve_host(int fmt, int lu, const S* F, const int* piv, int n, int64_t batch, S* B, int nrhs) {
-  if (int rc = emu_check(fmt, n, batch)) return rc;
+  if (int rc = emu_check<S>(fmt, n, batch)) return rc;
   if (nrhs < 0) return TSDX_ERR_NRHS;
   if (batch == 0 || nrhs == 0) return TSDX_OK;
   return run_host_with<S>(lu ? GETRS : POTRS, const_cast<S*>(F), piv, n, batch, B, nrhs, nullptr, nullptr, false,

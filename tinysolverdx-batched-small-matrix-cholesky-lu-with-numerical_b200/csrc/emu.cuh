@@ -9,8 +9,8 @@
 // float operation is an explicitly rounded intrinsic so nothing is contracted.
 //
 // One warp per matrix, the matrix in shared memory as float (every value of the formats
-// is a float). Storage in global memory is float64, float32 or binary16 bits; every
-// stored value is exactly representable, so the round trip is exact. What bounds it: the
+// is a float). Storage in global memory is float64, float32 or (fp16 alone) binary16 bits;
+// every stored value is exactly representable, so the round trip is exact. What bounds it: the
 // host copies; the kernel itself is arithmetic in shared memory (one thread per matrix
 // over float64 global memory, which this replaces, spent its time on uncoalesced reads).
 #pragma once
@@ -79,8 +79,9 @@ __device__ __forceinline__ void emu_store(const float* M, S* a, int n, int lane)
 }
 
 // Row by row, as the reference: row i takes its entries j < i in increasing j, each
-// updating the rest of the row. A pivot that is not positive stops there: the rows from
-// i on (and the pivot) keep their rounded input, the upper triangle is left as it is.
+// updating the rest of the row. A pivot that is not positive stops there: row i keeps its
+// entries j < i, the pivot and the rows after i their rounded input, and the upper
+// triangle is left as it is.
 template <int FMT, class S>
 __global__ void __launch_bounds__(256) emu_cholesky_kernel(S* A, int n, long long batch, int* info) {
   using E = EmuOps<FMT>;
