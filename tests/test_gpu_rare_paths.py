@@ -263,6 +263,13 @@ def test_binary16_storage_equals_cpu(n):
     assert same(tsdx.lu_solve(LU, piv, B[3:], backend="cuda"), tsdx.lu_solve(LU, piv, B[3:], backend="scalar"))
 
 
+def test_empty_batch_of_an_emulated_format_needs_no_pointers():
+    for sfx in ("", "_f32", "_f16"):
+        assert capi.call("tsdx_cuda_emu_factor_host" + sfx, 0, 1, None, 4, 0, None, None) == capi.TSDX_OK
+        assert capi.call("tsdx_cuda_emu_solve_host" + sfx, 0, 1, None, None, 4, 0, None, 3) == capi.TSDX_OK
+        assert capi.call("tsdx_cuda_emu_factor_host" + sfx, 0, 1, None, 4, 1, None, None) == capi.TSDX_ERR_NULL
+
+
 @pytest.mark.parametrize("batch", [1, 63, 64, 65, 600])
 def test_training_gradient_of_partial_blocks(batch):
     """Against float64: float32 sums of at most 600 samples over 64 units carry a few

@@ -263,6 +263,7 @@ template <class S> int emu_check(int fmt, int n, int64_t batch) {
 }
 template <class S> int emu_factor_host(int fmt, int lu, S* A, int n, int64_t batch, int* piv, int* info) {
   if (int rc = emu_check<S>(fmt, n, batch)) return rc;
+  if (batch == 0) return TSDX_OK;
   return run_host_with<S>(lu ? GETRF : POTRF, A, nullptr, n, batch, nullptr, 0, piv, info, false,
                           [&](S* dA, int* dpiv, int64_t cnt, S*, int* dinfo, cudaStream_t st) {
                             return run_emu_factor<S>(fmt, lu != 0, dA, n, cnt, dpiv, dinfo, st);
