@@ -270,6 +270,23 @@ def test_empty_batch_of_an_emulated_format_needs_no_pointers():
         assert capi.call("tsdx_cuda_emu_factor_host" + sfx, 0, 1, None, 4, 1, None, None) == capi.TSDX_ERR_NULL
 
 
+def test_wide_host_solves_keep_little_device_memory():
+    """400 MB of right-hand sides of small factors go through in chunks: what the calls leave
+    allocated is bounded by the chunks, not by the right-hand sides."""
+    n, batch, nrhs = 2, 32, 800_000
+    F = np.broadcast_to(np.array([[2.0, 0.0], [1.0, 4.0]]), (batch, n, n)).copy()
+    B = np.ones((batch, n, nrhs))
+    B[:, 1] = np.arange(batch)[:, None]
+    device.potrf(dev(np.eye(2)[None]))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    X = tsdx.cholesky_solve(F, B, precision="fp16", backend="cuda")
+    assert free - torch.cuda.mem_get_info()[0] < 3 * (200 << 20)
+    want = tsdx.cholesky_solve(F, B[..., :3].copy(), precision="fp16", backend="scalar")
+    assert same(np.ascontiguousarray(X[..., [0, nrhs // 2, nrhs - 1]]), want)
+
+
 @pytest.mark.parametrize("batch", [1, 63, 64, 65, 600])
 def test_training_gradient_of_partial_blocks(batch):
     """Against float64: float32 sums of at most 600 samples over 64 units carry a few

@@ -124,7 +124,7 @@ int run_device(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, i
 
 // ---- host-pointer implementation ----------------------------------------------
 constexpr int kSlots = 3;
-constexpr size_t kChunkBytes = size_t(96) << 20;  // A bytes per chunk, at most
+constexpr size_t kChunkBytes = size_t(96) << 20;  // bytes of A, and of B, per chunk, at most
 // A small batch is still cut into kMinChunks chunks (of at least kMinChunkBytes), so
 // that its copies overlap too: with two chunks, most of the transfer would run alone.
 constexpr int kMinChunks = 8;
@@ -187,8 +187,11 @@ int run_host_with(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B
     ctx.init = true;
   }
   const size_t mat = size_t(n) * n * sizeof(T), rhs = size_t(n) * nrhs * sizeof(T);
-  const size_t target = std::min(kChunkBytes, std::max(kMinChunkBytes, mat * size_t(batch) / kMinChunks));
-  const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(batch, int64_t(target / mat)));
+  // counted in the larger of a matrix and its right-hand sides: the slots keep what they
+  // have grown to
+  const size_t per = std::max(mat, rhs);
+  const size_t target = std::min(kChunkBytes, std::max(kMinChunkBytes, per * size_t(batch) / kMinChunks));
+  const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(batch, int64_t(target / per)));
   for (auto& s : ctx.slot) {
     if (int rc = grow(&s.a, &s.acap, mat * chunk)) return rc;
     if (has_b && nrhs > 0)
