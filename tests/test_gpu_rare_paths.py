@@ -63,6 +63,42 @@ def test_odd_pivots_bit_exact(oracle, n, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [3, 4, 8, 16, 24, 31, 32, 40, 45, 48, 56, 61, 64])
+def test_scaled_matrices_bit_exact(oracle, n, dtype):
+    """Powers of two put pivots and numerators on either side of the range of the shared
+    reciprocal division: whole matrices, single rows and columns, and D S D of an SPD
+    matrix; with -0 among the numerators, ties, and symmetric matrices that are not
+    dominated by their diagonal."""
+    r = np.random.default_rng(600 + n)
+    edges = (99, 100, 101, 119, 121) if dtype == np.float32 else (899, 900, 901, 600, 400, 500)
+    A, S = [], []
+    for e in edges:
+        for sign in (1, -1):
+            X = r.standard_normal((n, n))
+            Q = X @ X.T / n + 0.2 * np.eye(n)
+            Z = np.where(r.random((n, n)) < 0.3, -0.0, X)
+            d, col = np.ones(n), np.ones(n)
+            d[r.integers(n)] = col[r.integers(n)] = 2.0 ** (sign * e)
+            half = 2.0 ** r.integers(-(e // 2), e // 2 + 1, n)
+            A += [X * 2.0 ** (sign * e), X * d[:, None], X * col, Z, np.rint(2 * X) * 2.0 ** (sign * (e // 2))]
+            S += [Q * 2.0 ** (sign * e), Q * half[:, None] * half, np.where(np.abs(Q) < 0.3, -0.0, Q) + np.diag(np.full(n, n + 0.0)),
+                  X + X.T, Q * np.sqrt(d)[:, None] * np.sqrt(d)]
+    with np.errstate(over="ignore", under="ignore"):
+        A, S = np.stack(A).astype(dtype), np.stack(S).astype(dtype)
+    a = dev(A)
+    piv, info = device.getrf(a)
+    LUo, pivo, infoo = oracle.lu(A, "scalar")
+    assert np.array_equal(info.cpu().numpy(), infoo) and np.array_equal(piv.cpu().numpy(), pivo)
+    assert same(a.cpu().numpy(), LUo)
+    s = dev(S)
+    info = device.potrf(s).cpu().numpy()
+    Lo, infoo = oracle.cholesky(S, "simd")
+    assert np.array_equal(info, infoo)
+    ok = infoo == 0
+    assert ok.any() and same(s.cpu().numpy()[ok], Lo[ok])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 47, 49, 64])
 @pytest.mark.parametrize("nrhs", [2, 4, 5, 8, 16, 17])
 def test_solves_from_factor(oracle, n, nrhs, dtype):

@@ -379,6 +379,7 @@ __device__ __forceinline__ void lu_tc_matrix(unsigned char* M, const MatJob<doub
         *reinterpret_cast<T*>(M + row[s] * RS + C::OFF_RCP) = rcp;  // the last one stands: the step that retires the row
       };
       bool far = false;
+      const unsigned lim = D::limit(m);
       unsigned tie = 0;
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
@@ -386,15 +387,15 @@ __device__ __forceinline__ void lu_tc_matrix(unsigned char* M, const MatJob<doub
         const unsigned x = __ballot_sync(kFull, key[s] == m);
         tie |= (x & (x - 1)) | (b ? x : 0u);
         b |= x;
-        far |= D::outside(pan[s][i], D::kLo);
+        far |= D::outside(pan[s][i], lim);
       }
       far = __any_sync(kFull, far);
       __syncwarp();
       bool zero = false;
-      // rare, by the whole warp: a tie, or a column whose largest entry is zero, tiny,
-      // huge, infinite or NaN
-      const bool odd = (tie != 0) | (m - D::kLo > D::kHi - D::kLo);
-      if (odd) {
+      // rare, by the whole warp: a tie (of high words), or a column whose largest entry is
+      // tiny, huge, zero, infinite or NaN
+      const bool wide = m - D::kLo > D::kHi - D::kLo;
+      if ((tie != 0) | wide) {
         Candidates<T, MR> c;
 #pragma unroll
         for (int s = 0; s < MR; ++s) {
@@ -432,7 +433,7 @@ __device__ __forceinline__ void lu_tc_matrix(unsigned char* M, const MatJob<doub
           const T q = __dmul_rn(pan[s][i], ry);
           l[s] = __fma_rn(__fma_rn(-vpk, q, pan[s][i]), ry, q);
         }
-        if (odd || far) {
+        if (wide || far) {
 #pragma unroll
           for (int s = 0; s < MR; ++s) l[s] = act[s] ? div_slow(pan[s][i], vpk) : T(0);
         }

@@ -148,15 +148,22 @@ __device__ __forceinline__ double rcp_in_range(double p) {
 // needs no other check: no intermediate underflows and the remainder x - p q is exact,
 // because ulp(p) ulp(q) >= ulp(x)^2 / 2 is still a representable number. float32: p in
 // [2^-100, 2^100] and |x| >= max(2^-100, |p| 2^-120) (the quotient stays normal);
-// float64: p in [2^-600, 2^400] and |x| >= 2^-600. A +0 numerator needs no check
-// either; a -0 would lose its sign, so it counts as outside. Divisors are tested by the
-// high word m of |p|, once per step. The tests are combined with & and |: && and || became
-// branches (float64 LU on the tensor cores, a step of order 64 alone on its SM 502 -> 373
-// cycles; float32 posv n = 45, 50,000 matrices 1056 -> 972 us, a mixed stream of 262,144
-// 4323 -> 4147).
+// float64: p in [2^-900, 2^900] and |x| >= max(2^-900, |p| 2^-900). A +0 numerator needs no
+// check either; a -0 would lose its sign, so it counts as outside.
+// Divisors are tested by the high word m of |p|, once per step. The tests are combined with
+// & and |: && and || became branches (float64 LU on the tensor cores, a step of order 64
+// alone on its SM 502 -> 373 cycles; float32 posv n = 45, 50,000 matrices 1056 -> 972 us, a
+// mixed stream of 262,144 4323 -> 4147). Matrices scaled over 10^-250 .. 10^250 lie inside
+// (float64 getrf, order 16, 34,179 of them 87 us, where p in [2^-600, 2^400] sent a third
+// of them to the IEEE division and took 143; order 64, 4,096 203 and 559 us).
+//
+// kInf: from there on the high word belongs to an infinity or a NaN. A winner's high word
+// in [1, kInf) that no other candidate shares decides the pivot, whatever the range. A tie
+// needs the exact choice but no other division (integers of -1 .. 1, float32 LU of order 8:
+// 26 % less time than with the IEEE division at every tie).
 template <class T> struct DivRange;
 template <> struct DivRange<float> {
-  static constexpr unsigned kLo = (127u - 100u) << 23, kHi = (127u + 100u) << 23;
+  static constexpr unsigned kLo = (127u - 100u) << 23, kHi = (127u + 100u) << 23, kInf = 0x7f800000u;
   // the limit of |x| for a divisor m
   __device__ static __forceinline__ float limit(unsigned m) {
     return __int_as_float(__viaddmax_s32((int)m, -(120 << 23), (int)kLo));
@@ -164,8 +171,11 @@ template <> struct DivRange<float> {
   __device__ static __forceinline__ bool outside(float x, float lim) { return (fabsf(x) < lim) & (__float_as_int(x) != 0); }
 };
 template <> struct DivRange<double> {
-  static constexpr unsigned kLo = (1023u - 600u) << 20, kHi = (1023u + 400u) << 20;
-  __device__ static __forceinline__ unsigned limit(unsigned) { return kLo; }
+  static constexpr unsigned kLo = (1023u - 900u) << 20, kHi = (1023u + 900u) << 20, kInf = 0x7ff00000u;
+  // the limit of |x|'s high word
+  __device__ static __forceinline__ unsigned limit(unsigned m) {
+    return (unsigned)__viaddmax_s32((int)m, -(900 << 20), (int)kLo);
+  }
   __device__ static __forceinline__ bool outside(double x, unsigned lim) {
     return (((unsigned)__double2hiint(x) & 0x7fffffffu) < lim) & ((__double2hiint(x) | __double2loint(x)) != 0);
   }
@@ -348,10 +358,10 @@ __device__ __forceinline__ void lu_rows_group(unsigned Mu, RowRegs<T, NP, NRHS, 
     int wr;
     const bool one = one_row<G, MR>(b, g, wr);
     unsigned urow = Mu + wr * RS;
-    // rare, by the whole warp: a tie, or a column whose largest entry is zero, tiny, huge,
-    // infinite or NaN
-    bool odd = __any_sync(kFull, !one | (m - D::kLo > D::kHi - D::kLo)), zero = false;
-    if (odd) {
+    // rare, by the whole warp: a tie (of high words), or a column whose largest entry is
+    // zero, infinite or NaN
+    bool zero = false;
+    if (__any_sync(kFull, !one | (m - 1u >= D::kInf - 1u))) {
       Candidates<T, MR> c;
 #pragma unroll
       for (int s = 0; s < MR; ++s) {
@@ -394,7 +404,7 @@ __device__ __forceinline__ void lu_rows_group(unsigned Mu, RowRegs<T, NP, NRHS, 
     const T ry = rcp_in_range(piv);
     const auto lim = D::limit(m);
     T l[MR];
-    bool slow = odd;
+    bool slow = m - D::kLo > D::kHi - D::kLo;
 #pragma unroll
     for (int s = 0; s < MR; ++s) {
       const T q = x[s] * ry;
