@@ -62,6 +62,50 @@ def test_odd_pivots_bit_exact(oracle, n, dtype):
         assert same(LU[i], LUo[i]), i
 
 
+def step_check(a, b):
+    out = [torch.empty_like(a) for _ in range(4)]
+    capi.check(capi.call("tsdx_internal_step_check_" + ("f32" if a.dtype == torch.float32 else "f64"), capi.ptr(a), capi.ptr(b),
+                         *map(capi.ptr, out), a.numel(), capi.stream_ptr()))
+    q, q_ieee, y, y_ieee = (t.view(torch.int32 if a.dtype == torch.float32 else torch.int64) for t in out)
+    assert torch.equal(y, y_ieee) and torch.equal(q, q_ieee)
+
+
+@pytest.mark.parametrize("exponent", [-100, -99, -50, -1, 0, 1, 64, 99, 100])
+def test_step_division_float32(exponent):
+    """Every significand as the divisor, numerators from its size down to the smallest."""
+    g = torch.Generator(device="cuda").manual_seed(exponent + 200)
+    sig = torch.arange(1 << 23, device="cuda", dtype=torch.int32)
+    for sign in (0, -(1 << 31)):
+        b = (sig | ((127 + exponent) << 23) | sign).view(torch.float32)
+        for low in (0, 30, 130):
+            u = torch.rand(1 << 23, device="cuda", generator=g) * 2 - 1
+            a = (b * u) * torch.exp2(-torch.randint(0, low + 1, (1 << 23,), device="cuda", generator=g).float())
+            a[::1001] = 0.0
+            a[1::1001] = -0.0
+            a[2::1001] = b[2::1001]
+            step_check(a, b)
+
+
+@pytest.mark.parametrize("exponent", [-900, -899, -600, -1, 0, 1, 400, 899, 900])
+def test_step_division_float64(exponent):
+    """Random significands and those next to all ones and to one, numerators likewise."""
+    n = 1 << 24
+    g = torch.Generator(device="cuda").manual_seed(exponent + 2000)
+    ones = (1 << 52) - 1
+    for rep in range(4):
+        sig = torch.randint(0, ones + 1, (n,), device="cuda", generator=g, dtype=torch.int64)
+        near = torch.randint(0, 64, (n // 4,), device="cuda", generator=g, dtype=torch.int64)
+        sig[: n // 4] = ones - near * (rep % 2)
+        sig[n // 4: n // 2] = near
+        b = (sig | ((1023 + exponent) << 52)).view(torch.float64) * (1 - 2 * (rep // 2))
+        a = b * (torch.rand(n, device="cuda", generator=g, dtype=torch.float64) * 2 - 1)
+        a *= torch.exp2(-torch.randint(0, (1, 60, 950, 1000)[rep] + 1, (n,), device="cuda", generator=g).double())
+        a[::1001] = 0.0
+        a[1::1001] = -0.0
+        a[2::1001] = b[2::1001]
+        step_check(a, b)
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("n", [3, 4, 8, 16, 24, 31, 32, 40, 45, 48, 56, 61, 64])
 def test_scaled_matrices_bit_exact(oracle, n, dtype):

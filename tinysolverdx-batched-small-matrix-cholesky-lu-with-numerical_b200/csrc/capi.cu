@@ -336,6 +336,41 @@ API int tsdx_internal_div_check_f32(const float* a, const float* b, float* fast,
   return div_check<float>(a, b, fast, ieee, count, st);
 }
 
+// The pivot steps' reciprocal and guarded quotient (rcp_in_range and DivRange, rows.cuh) for
+// |a| <= |b|, beside the IEEE ones; a reciprocal outside the range is not compared.
+namespace {
+template <class T>
+__global__ void step_check_kernel(const T* a, const T* b, T* q, T* q_ieee, T* y, T* y_ieee, long long count) {
+  using namespace tsdx::dev;
+  using D = DivRange<T>;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  const T x = a[i], p = b[i], r = rcp_in_range(p), t = x * r;
+  const unsigned m = abs_hi(p);
+  const bool far = m - D::kLo > D::kHi - D::kLo;
+  q[i] = far | D::outside(x, D::limit(m)) ? div_slow(x, p) : fma_(fma_(-p, t, x), r, t);
+  q_ieee[i] = div_(x, p);
+  y_ieee[i] = rcp_(p);
+  y[i] = far ? y_ieee[i] : r;
+}
+template <class T>
+int step_check(const T* a, const T* b, T* q, T* q_ieee, T* y, T* y_ieee, int64_t count, void* st) {
+  if (count <= 0) return TSDX_OK;
+  step_check_kernel<T><<<(unsigned)((count + 255) / 256), 256, 0, ST(st)>>>(a, b, q, q_ieee, y, y_ieee, count);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { tsdx::host::set_cuda_error(e, "kernel launch"); return TSDX_ERR_CUDA; }
+  return TSDX_OK;
+}
+}  // namespace
+API int tsdx_internal_step_check_f64(const double* a, const double* b, double* q, double* q_ieee, double* y,
+                                     double* y_ieee, int64_t count, void* st) {
+  return step_check<double>(a, b, q, q_ieee, y, y_ieee, count, st);
+}
+API int tsdx_internal_step_check_f32(const float* a, const float* b, float* q, float* q_ieee, float* y, float* y_ieee,
+                                     int64_t count, void* st) {
+  return step_check<float>(a, b, q, q_ieee, y, y_ieee, count, st);
+}
+
 // ---- emulated fp16 / bf16 ---------------------------------------------------------
 #define TSDX_EMU_API(SFX, S)                                                                                        \
   API int tsdx_cuda_emu_factor_host##SFX(int fmt, int lu, S* A, int n, int64_t batch, int* piv, int* info) {        \

@@ -122,14 +122,14 @@ __device__ __forceinline__ bool plain_zero(double v) { return __double_as_longlo
 __device__ __forceinline__ unsigned abs_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned abs_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 
-// RN(1/p) without a branch, for p in DivRange: from the hardware's approximation, a
-// Newton step (a third-order one in float64) to within one ulp, and Markstein's final
-// step y + y (1 - p y), which rounds correctly from there unless p's significand is all
-// ones (P. Markstein, IBM J. Res. Develop. 34(1), 1990). That last case needs the step
-// before to round up: 1/p then lies just above the middle of two neighbours, and the
-// final step is right from the upper one. Equal to __frcp_rn on every float32 of the
-// range and to __drcp_rn on 1.2e9 float64 values of either sign, the all-ones ones
-// included.
+// RN(1/p) without a branch, for p in DivRange: from the hardware's approximation to
+// within one ulp (float32 as it comes; float64 after a third-order Newton step), and
+// Markstein's final step y + y (1 - p y), which rounds correctly from there unless p's
+// significand is all ones (P. Markstein, IBM J. Res. Develop. 34(1), 1990). That last case
+// needs the value before to be rounded up: 1/p then lies just above the middle of two
+// neighbours, and the final step is right from the upper one. Checked against __frcp_rn for
+// every float32 significand and against __drcp_rn for float64 ones at random and all ones,
+// at exponents over the range, by tests/test_gpu_rare_paths.py::test_step_division_*.
 __device__ __forceinline__ float rcp_in_range(float p) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(p));
