@@ -62,6 +62,77 @@ def test_odd_pivots_bit_exact(oracle, n, dtype):
         assert same(LU[i], LUo[i]), i
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [2, 4, 7, 8, 16, 21, 24, 29, 32, 40, 45, 48, 61, 64])
+@pytest.mark.parametrize("nrhs", [1, 3, 8])
+def test_odd_pivots_with_right_hand_sides(oracle, n, nrhs, dtype):
+    """The same pivots under gesv, in warps shared with healthy matrices: factors, pivots and
+    info as the oracle's, and the healthy ones' solutions as in a batch of their own."""
+    odd = odd_matrices(n, dtype, 300 + n)
+    r = np.random.default_rng(n * 5 + nrhs)
+    good = M.general(r, len(odd), n, 1e2).astype(dtype)
+    A = np.empty((2 * len(odd), n, n), dtype)
+    A[0::2], A[1::2] = odd, good
+    B = r.standard_normal((len(A), n, nrhs)).astype(dtype)
+    a, b = dev(A), dev(B)
+    piv, info = (t.cpu().numpy() for t in device.gesv(a, b))
+    LUo, pivo, infoo = oracle.lu(A, "scalar")
+    assert np.array_equal(info, infoo) and np.array_equal(piv, pivo) and same(a.cpu().numpy(), LUo)
+    a, x = dev(good), dev(B[1::2])
+    device.gesv(a, x)
+    assert same(b[1::2].cpu().numpy(), x.cpu().numpy())
+    X, B64 = x.cpu().numpy().astype(np.float64), B[1::2].astype(np.float64)
+    num = np.linalg.norm(B64 - good.astype(np.float64) @ X, axis=1)
+    den = np.linalg.norm(good.astype(np.float64), axis=(1, 2))[:, None] * np.linalg.norm(X, axis=1) + np.linalg.norm(B64, axis=1)
+    assert (num / den).max() <= 8 * n * np.finfo(dtype).eps / 2
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("sched", [0, 15])
+def test_odd_pivots_in_a_stream(oracle, sched, dtype):
+    """Every order, odd and healthy matrices and both kinds in the same units: factors, pivots
+    and info as the oracle's, the healthy ones' solutions as in the dense batch."""
+    st = load_pkg("stream")
+    r = np.random.default_rng(77 + sched)
+    count = 64 * 24
+    n = np.tile(np.arange(1, 65, dtype=np.int32), 24)
+    nrhs = r.choice([0, 1, 3, 8], count).astype(np.int32)
+    kind = r.integers(0, 2, count).astype(np.int8)
+    order = r.permutation(count)
+    n = n[order]
+    mats, healthy = [], []
+    for i in range(count):
+        m, ok = int(n[i]), not kind[i] or i % 3 == 0
+        if not kind[i]:
+            mats.append(M.spd(r, 1, m, 1e2)[0].astype(dtype))
+        elif ok or m < 2:
+            mats.append(M.general(r, 1, m, 1e2)[0].astype(dtype))
+        else:
+            mats.append(odd_matrices(m, dtype, int(i))[int(r.integers(14))])
+        healthy.append(ok or m < 2)
+    rhs = [r.standard_normal((int(m), int(k))).astype(dtype) for m, k in zip(n, nrhs)]
+    plan = st.StreamPlan(n, nrhs, kind, dtype=torch.float32 if dtype == np.float32 else torch.float64)
+    plan.sched = sched
+    plan.load(dev(np.concatenate([a.ravel() for a in mats])), dev(np.concatenate([b.ravel() for b in rhs])))
+    plan.launch()
+    A, B, piv, info = (t.cpu().numpy() for t in (plan.A, plan.B, plan.piv, plan.info))
+    aoff, boff, poff = (t.cpu().numpy() for t in (plan.aoff, plan.boff, plan.poff))
+    for i in range(count):
+        m, k = int(n[i]), int(nrhs[i])
+        F = A[aoff[i]:aoff[i] + m * m].reshape(1, m, m)
+        if kind[i]:
+            Fo, po, io = oracle.lu(mats[i][None], "scalar")
+            assert np.array_equal(piv[poff[i]:poff[i] + m], po[0]), i
+        else:
+            Fo, io = oracle.cholesky(mats[i][None], "simd")
+        assert info[i] == io[0] and same(F, Fo), i
+        if healthy[i] and k:
+            a, b = dev(mats[i][None]), dev(rhs[i][None])
+            device.gesv(a, b) if kind[i] else device.posv(a, b)
+            X, Y = B[boff[i]:boff[i] + m * k].reshape(m, k), b[0].cpu().numpy()
+            assert same(X, Y), i
+
+
 def step_check(a, b):
     out = [torch.empty_like(a) for _ in range(4)]
     capi.check(capi.call("tsdx_internal_step_check_" + ("f32" if a.dtype == torch.float32 else "f64"), capi.ptr(a), capi.ptr(b),
@@ -341,6 +412,28 @@ def test_binary16_storage_equals_cpu(n):
     assert same(tsdx.cholesky_solve(L, B[2:], backend="cuda"), tsdx.cholesky_solve(L, B[2:], backend="scalar"))
     LU, piv, _ = tsdx.lu(G[3:], backend="scalar")
     assert same(tsdx.lu_solve(LU, piv, B[3:], backend="cuda"), tsdx.lu_solve(LU, piv, B[3:], backend="scalar"))
+
+
+@pytest.mark.parametrize("n", [3, 17, 33, 64])
+@pytest.mark.parametrize("fmt", ["fp16", "bf16"])
+def test_emulated_formats_of_large_batches(n, fmt):
+    """More matrices than a wave of full blocks: five systems repeated, each copy with the bits
+    of the CPU's result."""
+    r = np.random.default_rng(n)
+    batch = 12_001 if n < 40 else 6_001
+    S = M.spd(r, 5, n, 10.0).astype(np.float32)
+    G = r.standard_normal((5, n, n)).astype(np.float32)
+    B = r.standard_normal((5, n, 2)).astype(np.float32)
+    at = np.arange(batch) % 5
+    for f, X in ((tsdx.cholesky, S), (tsdx.lu, G)):
+        got, want = f(X[at], precision=fmt, backend="cuda"), f(X, precision=fmt, backend="scalar")
+        assert same(got[0], want[0][at]) and all(np.array_equal(g, w[at]) for g, w in zip(got[1:], want[1:]))
+    L, _ = tsdx.cholesky(S, precision=fmt, backend="scalar")
+    LU, piv, _ = tsdx.lu(G, precision=fmt, backend="scalar")
+    assert same(tsdx.cholesky_solve(L[at], B[at], precision=fmt, backend="cuda"),
+                tsdx.cholesky_solve(L, B, precision=fmt, backend="scalar")[at])
+    assert same(tsdx.lu_solve(LU[at], piv[at], B[at], precision=fmt, backend="cuda"),
+                tsdx.lu_solve(LU, piv, B, precision=fmt, backend="scalar")[at])
 
 
 def test_empty_batch_of_an_emulated_format_needs_no_pointers():
