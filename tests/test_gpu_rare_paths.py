@@ -414,6 +414,30 @@ def test_binary16_storage_equals_cpu(n):
     assert same(tsdx.lu_solve(LU, piv, B[3:], backend="cuda"), tsdx.lu_solve(LU, piv, B[3:], backend="scalar"))
 
 
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 8, 9])
+@pytest.mark.parametrize("nrhs", [4, 5, 8, 11])
+def test_posv_of_a_large_batch_equals_a_small_one(n, nrhs):
+    """From 16,384 matrices on, float64 posv of orders 4 and 8 solves five or more right-hand
+    sides from the factor: factors, info and solutions as the one-pass kernel's, failing
+    pivots and non-finite entries included."""
+    r = np.random.default_rng(n * 19 + nrhs)
+    S = M.spd(r, 9, n, 1e3)
+    S[1, n // 2, n // 2] = -1.0
+    S[2] *= 1e200
+    S[3, -1, 0] = np.nan
+    S[4, 0, 0] = 0.0
+    B = r.standard_normal((9, n, nrhs))
+    B[5, 0, 0], B[6, -1, -1], B[7, 0] = np.inf, np.nan, -0.0
+    want = (dev(S), dev(B))
+    info = device.posv(*want)
+    at = torch.arange(16384 + 5, device="cuda") % 9
+    got = (dev(S)[at], dev(B)[at])
+    big = device.posv(*got)
+    assert torch.equal(big, info[at])
+    for g, w in zip(got, want):
+        assert same(g.cpu().numpy(), w[at].cpu().numpy())
+
+
 @pytest.mark.parametrize("n", [3, 17, 33, 64])
 @pytest.mark.parametrize("fmt", ["fp16", "bf16"])
 def test_emulated_formats_of_large_batches(n, fmt):

@@ -77,6 +77,19 @@ inline int check_common(int n, int64_t batch, int nrhs) {
 }
 template <class T> inline bool aligned(const T* p) { return reinterpret_cast<uintptr_t>(p) % alignof(T) == 0; }
 
+// The right-hand sides that the factorization takes along; the others are solved from the
+// factor. float64 Cholesky of order 4 or 8 takes none of five or more in a batch that fills
+// the chip: there the kernel with a lane per right-hand side (solve.cuh) costs less than
+// the factorization's columns (n = 4, 8 right-hand sides, 234,375 matrices 124 -> 63 us,
+// where the factorization before rows.cuh took 106; n = 8 267 -> 146 and 253; 16,384 of
+// n = 4 17.4 -> 15.4); below it the second launch costs more (4,000 matrices 11 us with one,
+// 13 with two; equal at 8,000 to 16,000). Orders that fill their tile, so that both ways
+// agree on right-hand sides that are not finite as well.
+constexpr int64_t kSplitBatch = 16384;
+template <class T> int fused_rhs(Kind kind, int n, int64_t batch, int nrhs) {
+  return kind == POSV && sizeof(T) == 8 && (n == 4 || n == 8) && nrhs > 4 && batch >= kSplitBatch ? 0 : 8;
+}
+
 // ---- device-pointer implementation --------------------------------------------
 template <class T>
 int run_device(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, int nrhs, int* piv, int* info,
@@ -102,10 +115,10 @@ int run_device(Kind kind, T* A, const int* piv_in, int n, int64_t batch, T* B, i
   a.wf = 1;
   if (kind == POTRF || kind == GETRF || kind == POSV || kind == GESV) {
     a.b0 = 0;
-    a.nrhs = std::min(nrhs, 8);
+    a.nrhs = std::min(nrhs, fused_rhs<T>(kind, n, batch, nrhs));
     const int rc = (kind == POTRF || kind == POSV) ? run_chol<T>(a, st) : run_lu<T>(a, st);
     if (rc) return rc;
-    for (int b0 = 8; b0 < nrhs; b0 += kTrsRhs) {  // remaining right-hand sides from the factor
+    for (int b0 = a.nrhs; b0 < nrhs; b0 += kTrsRhs) {  // remaining right-hand sides from the factor
       a.b0 = b0;
       a.nrhs = std::min(kTrsRhs, nrhs - b0);
       const int r2 = (kind == POSV) ? run_potrs<T>(a, st) : run_getrs<T>(a, st);
