@@ -484,6 +484,18 @@ def test_wide_host_solves_keep_little_device_memory():
     assert same(np.ascontiguousarray(X[..., [0, nrhs // 2, nrhs - 1]]), want)
 
 
+@pytest.mark.parametrize("n", [1, 5, 32, 33, 64])
+def test_features_of_zero_rows_have_no_negative_zero(n):
+    sel = load_pkg("selector")
+    r = np.random.default_rng(n)
+    A = r.standard_normal((3, n, n))
+    A[0] = 0.0
+    A[1] = -0.0
+    A[2, n // 2] = 0.0
+    X = sel.features(dev(A), 1).cpu().numpy()
+    assert not (np.signbit(X) & (X == 0.0)).any()
+
+
 @pytest.mark.parametrize("batch", [1, 63, 64, 65, 600])
 def test_training_gradient_of_partial_blocks(batch):
     """Against float64: float32 sums of at most 600 samples over 64 units carry a few

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(WPC * 32, 2) features_kernel(const double* __r
         X[8] = fmax(X[8], -ra);
         X[9] = fmax(X[9], -g);
         X[10] = fmax(X[10], -ca);
-        X[11] = fmax(X[11], (ra > 0) ? -(g / ra) : 0.0);
+        X[11] = fmax(X[11], (ra > 0) ? -(g / ra) : -0.0);  // the feature is its negative
       }
     }
     const double sum = fold16(S, lane, add), ext = fold16(X, lane, mx);  // lane i: value i / 2
