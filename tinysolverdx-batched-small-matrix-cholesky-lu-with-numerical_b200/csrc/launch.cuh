@@ -73,8 +73,11 @@ int prepare(Kern kern, int smem, int most) {
 // LU / Cholesky with rows in registers (rows.cuh): a persistent CTA per SM with as many
 // warps as shared memory holds, at most 16. Between 12 and 16 it stays at 12: warps are
 // dealt to four schedulers, so 13 to 15 cost the registers of 16 (128 a thread instead of
-// 168) without its parallelism (float32 LU, order 56, 65,536 matrices: 1547 us with 12,
-// 1568 with 14; Cholesky 1398 and 1476).
+// 168) without its parallelism (float32, 4 right-hand sides: LU of order 24, 262,144
+// matrices 869 us with 12, 978 with 15; order 56, 65,536 1686 and 1950 with 14; Cholesky of
+// order 40 597 and 714 with 13; without right-hand sides within 2 %). A batch that 12 warps
+// an SM do not quite hold pays a second round (float32 LU of order 52, 2,000 matrices 105
+// us, 1,700 60).
 template <class T, int NP, int NRHS, int GO = 0>
 constexpr int blk_wpc() {
   constexpr int FIT = (227 * 1024 - dev::kRowConst) / dev::BlkCfg<T, NP, NRHS, GO>::WARPB;
@@ -83,13 +86,16 @@ constexpr int blk_wpc() {
 
 // Lanes per matrix (0: the layout's own choice; the matrices that share a warp run its
 // steps together, so small orders spend fewer instructions each). Measured on B200 at
-// 65,536 to 262,144 matrices against the next choice, best warps each: order 8, 4 lanes
-// 117 us against 118 with 8 (float32 LU), 102 against 113 (float64 Cholesky); order 16, 8
-// lanes 180 against 247 with 16 (float32 Cholesky), 325 against 429 (float64); order 24,
-// float32 8 lanes 595 against 691 with 16, float64 16 lanes 650 against 681 with 8;
-// order 32, float32 16 lanes 1114 against 1132 with 32, float64 32 lanes 1105 against
-// 1226 with 16; order 40, float32 16 lanes 1214 against 1371 with 32, float64 32 lanes
-// (within 2 % of 16). Above that, one matrix per warp.
+// 65,536 to 262,144 matrices against the next choice, factorizations alone (LU, Cholesky;
+// us): order 8, 4 lanes float32 73 and 56, with 8 89 and 75, float64 101 and 75 against 116
+// and 95; order 16, 8 lanes float32 232 and 148, with 16 259 and 232, float64 374 and 222
+// against 376 and 329; order 24 float32, 8 lanes 586 and 384, with 16 640 and 556; order 32
+// float32, 16 lanes 493 and 415, with 32 634 and 556; order 40 float32, 16 lanes 609 and
+// 404, with 32 618 and 540. In float64 the next choice came out ahead there once panels
+// ran in a rolled loop: order 24 with 8 lanes 1148 and 745 against 1172 and 845 with the 16
+// taken here (with 4 right-hand sides 1316 and 1281 against 1685 and 1433), Cholesky of
+// order 32 with 16 lanes 681 against 833 with 32, of order 40 837 against 943. Above that,
+// one matrix per warp.
 template <class T, int NP>
 constexpr int blk_lanes() {
   constexpr bool F32 = sizeof(T) == 4;
@@ -102,9 +108,9 @@ constexpr int blk_lanes() {
   }
 }
 
-// Two warps per matrix (blk2.cuh) for float64 LU of padded order 48..56: measured on
-// B200 against one warp per matrix at 65,536-131,072 matrices with 4 right-hand
-// sides, 1.10x (order 48), 1.22x (56), 1.10x (64); slower at 40 and in float32.
+// Two warps per matrix (blk2.cuh) for float64 LU of padded order 48..56: 1.10x (order 48)
+// and 1.22x (56) the one-warp kernel on CUDA cores that rows.cuh replaced (65,536 to
+// 131,072 matrices, 4 right-hand sides); slower at 40 and in float32.
 template <class T, int NP, int NRHS>
 int launch_blk2(const SolveArgs<T>& a, cudaStream_t st) {
   using C = dev::Blk2Cfg<T, NP, NRHS>;
@@ -171,13 +177,13 @@ int launch_tc(const SolveArgs<double>& a, cudaStream_t st) {
 
 template <class T, int NP, int NRHS, bool CHOL>
 int launch_blk(const SolveArgs<T>& a, cudaStream_t st) {
-  // float64 LU from padded order 32 on: the tensor-core trailing update. Measured on
-  // B200 against the shared-memory kernels (65,536-262,144 matrices, 4 right-hand
-  // sides, M solves/s): n=25 77.1 vs 68.1, n=32 93.0 vs 65.3, n=40 38.0 vs 33.3,
-  // n=48 26.8 vs 23.1, n=56 18.2 vs 16.7, n=64 15.3 vs 12.9 (its later changes took
-  // n=64 to 16.9: the back substitution, the winner record and U12). Odd orders above 48
-  // stay on the shared-memory kernels (n=61 11.6 vs 12.3): their rows are not whole
-  // 16-byte units, so the matrix cannot arrive by bulk copies.
+  // float64 LU from padded order 32 on: the tensor-core trailing update. Measured on B200
+  // against the kernels on CUDA cores (4 right-hand sides, 131,072 matrices up to order 32,
+  // 65,536 above, us): n=25 1080 and 1304, n=32 1084 and 1304, n=40 1066 and 1320, n=48 1574
+  // and 2739, n=56 2332 and 3800, n=64 3229 and 4985. Odd orders above 48 run on
+  // blk2/blk3: the line was drawn when rows came by bulk copies, which their 8-byte rows
+  // did not allow. With the copies of today tc_kernel takes them too (TSDX_LU_KERNEL=tc) and
+  // is the faster one, n=49 2307 and 3953, n=55 2421 and 4114, n=61 3389 and 5620.
   if constexpr (!CHOL && sizeof(T) == 8 && NP >= 32) {
     const int fam = lu_kernel_family();
     if (fam == 3 || (fam == 0 && (NP <= 48 || a.n % 2 == 0)))

@@ -1,5 +1,5 @@
 // Error metrics on the GPU: the reference's long-double ground-truth metrics
-// (src/runtime.cpp:194-242) restated in double-double arithmetic, one warp per
+// (src/runtime.cpp:194-242) restated in double-double arithmetic, one or two warps per
 // matrix, so that error reports over whole batches need no host round trip.
 //
 //   chol_backward_error   ||A - L L^T||_F / ||A||_F                  (runtime.cpp:194-206)

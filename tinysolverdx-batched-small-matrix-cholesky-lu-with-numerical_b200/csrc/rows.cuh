@@ -209,8 +209,10 @@ struct RowCfg {
   // multipliers are known, so this costs no search, and no more stores and updates than
   // updating it step by step. Whole rows above order 16 spill or leave too few warps, and
   // their fully unrolled steps do not fit the instruction cache (float32 LU, order 32, 4
-  // right-hand sides, 262,144 matrices: whole rows 1576 us, panels of 16 1352 to 1403,
-  // of 8 1389; order 64, 65,536: panels of 32 2697, of 16 2277, of 8 2199).
+  // right-hand sides, 262,144 matrices: whole rows 1576 us, unrolled panels of 8 1389).
+  // Rolled panels of 8 against 16: Cholesky of order 48, 65,536 matrices, 4 right-hand sides
+  // 972 and 1082 us in float32, 2122 and 2377 in float64; LU in float32 order 32, 131,072
+  // 636 and 679, order 64 1877 and 1869 (without right-hand sides 1445 and 1273).
   static constexpr int PW = NP <= 16 ? NP : 8;
   static constexpr int LASTW = NCV - (NP - 1) / PW * PW;       // the last panel holds the right-hand sides
   static constexpr int RW = LASTW > PW ? LASTW : PW;

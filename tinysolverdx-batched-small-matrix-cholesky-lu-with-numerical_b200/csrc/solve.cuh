@@ -457,7 +457,7 @@ __host__ __device__ constexpr int trs_small_elems(int n, int lg) { return (32 >>
 
 template <class T, int NP, bool LU>
 __global__ void __launch_bounds__(kSmallWpc * 32) trs_small_kernel(SolveArgs<T> p, int lg) {
-  extern __shared__ __align__(16) unsigned char smem[];
+  extern __shared__ __align__(128) unsigned char smem[];
   const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, wpc = blockDim.x >> 5;
   const int n = p.n, nn = n * n, stride = trs_small_stride(n), S = 32 >> lg;
   T* F = reinterpret_cast<T*>(smem) + warp * trs_small_elems(n, lg);

@@ -21,7 +21,8 @@ from . import capi
 CHOLESKY, LU = 0, 1
 # sched bit c (order class c: n in 1..8, 9..16, 17..24, 25..32) set -> those matrices
 # run one per warp; clear -> they share a warp (8 at n <= 8, 4 at
-# n <= 16, 4 (float32) or 2 (float64) at n <= 24, 2 (float32) at n <= 32)
+# n <= 16, 4 (float32) or 2 (float64) at n <= 24, 2 (float32) at n <= 32; orders 33..40
+# share by two in float32, whatever the bits)
 SCHED_BITS = 4
 
 
